@@ -7,15 +7,15 @@ the device, timed with CUDA events on the engine's stream, best of `repeats`):
     batch_part_log2  build rows per partition 2^8 .. 2^13 -- the radix fan-out:
                      an instance with b build rows gets ceil(log2(b / 2^x))
                      partition bits (0 .. 11), reported as `radix_bits`
-    batch_load_pct   build rows per 100 buckets of a partition table (50 .. 90)
+    batch_load_pct   build rows per 100 buckets of a partition table, and per 100 slots of
+                     the table that R0 is looked up in (50 .. 90)
   plain path (HJ_BATCH_PLAIN, the engine's regular build / probe)
     radix_bits       MSD partition bits of the table build (0 .. 12, or -1 = automatic)
     probe_group      output rows per thread of the match writer (1, 4, 8, 32): a
                      probe key's matches spread over count / probe_group threads
 
-The batched join gives each probe key one thread: its tables live in shared
-memory and a bucket holds under one key on average, so wider groups only add
-idle lanes.  Results are cached as JSON keyed by the GPU name and the
+The batched join gives each probe key one thread: a lookup is one 32-byte
+bucket, so wider groups only add idle lanes.  Results are cached as JSON keyed by the GPU name and the
 workload's shape; `apply()` sets the chosen options on an engine.
 """
 from __future__ import annotations

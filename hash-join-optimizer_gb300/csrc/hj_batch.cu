@@ -10,18 +10,16 @@
 // payloadm-1 (fp_start / fp_add / fp_final below; the same on every path and
 // in the oracle).
 //
-// Batched path: because every join of an instance is on the same key, one
-// radix partitioning of the key serves the whole chain.  All relations of all
-// instances are partitioned together (one histogram, scan and scatter pass),
-// then each work item -- (instance, partition, chunk of R0 rows) -- builds the
-// partition of every build relation as a shared-memory table and runs its R0
-// rows through the whole chain in registers; no intermediate is written.  The
-// kernels are persistent: grids sized to the resident capacity pull work
-// items from device-side queues (atomic counters), so instances of very
-// different sizes share the SMs evenly, and the whole batch runs without host
-// synchronisation, captured and launched as one CUDA graph.  A partition too
-// large for shared memory (heavy duplicate keys) flags its instance, which is
-// then recomputed on the plain path.
+// Batched path: because every join of an instance is on the same key, the
+// build relations (R1, R2, ...) are joined among themselves first -- radix
+// partitioned together, one histogram, scan and scatter pass over all
+// instances, then one block per partition -- into one hash table per
+// instance, and R0 is streamed once against it; no intermediate is written.
+// The kernels are persistent: grids sized to the resident capacity take work
+// items in turn, so instances of very different sizes share the SMs evenly,
+// and the whole batch runs without host synchronisation, captured and launched
+// as one CUDA graph.  A partition too large for shared memory (heavy duplicate
+// keys) flags its instance, which is then recomputed on the plain path.
 //
 // Plain path: the instances one at a time through the engine's regular
 // radix-partitioned table build and two-pass probe (hj_build.cu, hj_probe.cu),
@@ -96,30 +94,36 @@ __global__ void k_batch_generate(uint64_t seed, uint32_t inst, uint32_t rel, uin
     }
 }
 
-// ---- batched path: one multi-way partitioned pass ---------------------------
-// Every relation of an instance joins on the same key, so one partitioning of
-// the key serves the whole chain: partition l of R0 meets only partition l of
-// R1, R2, ...  Instance i gets p_i partition bits (about `part_rows` build
-// rows per partition summed over its build relations); a row belongs to
-// partition top_p_i(hash(key)).
-//   1. row counts per (relation, partition), all relations of all instances
-//      (8192-row items round robin; counts kept per block until its
-//      relation changes)                                     k_bpart_hist
+// ---- batched path -----------------------------------------------------------
+// Every join of an instance is on the same key, so (R0 x R1) x R2 ... equals
+// R0 x (R1 x R2 x ...), and the build relations are small beside R0 (a tenth
+// in the synthetic workload).  They are partitioned and joined among
+// themselves first, and R0 is then streamed once against the result:
+//   1. row counts of the build relations per (relation, partition)  k_bpart_hist
 //   2. exclusive scan -> partition offsets in one partitioned buffer
-//   3. rows into partition order                             k_bpart_scatter
-//      (block-local counting sort in shared memory, payloads staged by
-//      cp.async meanwhile, one global range reservation per (block,
-//      partition), runs written out coalesced as (key, payload) pairs)
-//   4. join work list: (instance partition, chunk of its R0 rows)
-//                                                            k_bjoin_plan
-//   5. per work item: the partition of every build relation becomes a
-//      shared-memory table, and each R0 row walks the chain through them in
-//      registers -- no intermediate results are written    k_bjoin
-// A partition whose build rows exceed the shared-memory capacity (heavy
-// duplicates) flags its instance, which is then recomputed on the plain path.
+//   3. build rows into partition order                              k_bpart_scatter
+//   4. per instance partition: R2, R3, ... become shared-memory
+//      tables, R1's rows are looked up in them, and the rows whose
+//      key is in all go to the partition's piece of table F, their
+//      partners' payloads beside the slot                           k_bt_build
+//   5. R0 rows looked up in F                                       k_bt_probe
+//   6. R0 rows of instances with duplicate keys in R2, R3, ...      k_bt_enum
+// Instance i gets p_i partition bits (about `part_rows` build rows per
+// partition summed over its build relations); a row belongs to partition
+// top_p_i(hash(key)).  A partition whose build rows exceed the shared-memory
+// capacity (heavy duplicates) flags its instance, which is then recomputed on
+// the plain path.
+//
+// F is read in place of a partitioned R0: random 32-byte reads of tables up to
+// 64 MB run at 292e9/s on a GB300 (one L2 sector per SM and cycle; 84e9/s at
+// 256 MB, past the L2), and at 273e9 rows/s together with the stream of R0,
+// where a partition of R0 beside the build relations (28 bytes a row in three
+// passes) took 17 ps a row.  64 instances of 1k .. 4M build rows (364M R0
+// rows): 5.5 ms with R0 partitioned, 3.5 ms so.  Tables built in place by
+// atomics, without the partition, took 30 ps a build row to insert and 50 to
+// reduce, against 7 to partition and 13 to build here.
 constexpr int      kPT         = 512;   // threads of the partition and join blocks
 constexpr uint32_t kPartItem   = 8192;  // rows per partition-pass work item
-constexpr uint32_t kJoinChunk  = 8192;  // least R0 rows per join work item (else 16 per build row)
 constexpr uint32_t kMaxPartBits = 11;
 constexpr uint32_t kMaxRel     = 8;     // relations per instance
 
@@ -127,18 +131,52 @@ struct RelInst {  // one relation of one instance
     const int32_t* keys;
     const int32_t* pay;
     uint64_t       rows;
-    uint64_t       item_base;  // first partition-pass item
-    uint64_t       part_base;  // global partition id of its partition 0
+    uint64_t       item_base;  // first work item (build relations: of the partition passes, then R0s: of the probe)
+    uint64_t       part_base;  // global partition id of partition 0 (R0s: of R1's, which their keys are looked up in)
     uint32_t       pbits;
     uint32_t       inst;
+    uint32_t       irows;  // R0s: rows per work item
+    uint32_t       nrel;
+};
+
+// One work item of the probe, whole, so that a block waits for one load.
+struct Item {
+    const int32_t *k, *p;
+    uint64_t       part_base;
+    uint32_t       n, inst, pbits, nt;  // rows; instance; its partition bits and tables beside F
 };
 
 struct InstInfo {
-    uint64_t part_base;  // global partition id of (R0, partition 0); relation j, partition l: + j * 2^pbits + l
-    uint64_t ip_base;    // first instance-partition entry of the join plan (2^pbits entries)
+    uint64_t part_base;  // global partition id of (R1, partition 0); relation j, partition l: + (j - 1) * 2^pbits + l
+    uint64_t ip_base;    // first instance partition (2^pbits of them)
     uint32_t nrel;
     uint32_t pbits;
 };
+
+// Per-instance results and flags, cleared together.
+struct InstOut {
+    unsigned long long rows, sum;
+    uint32_t           ovf;   // a partition too large for shared memory, or a row equal to kFree
+    uint32_t           dups;  // R2, R3, ... hold a key of R1 more than once: partners are enumerated
+};
+
+// A table in buckets of four (key, payload) slots, 32 bytes (one L2 sector,
+// read by one 256-bit load).  A row goes to the first free slot from its home
+// bucket on (linear probing over the piece's buckets); equal keys take a slot
+// each.  A full bucket that rows went past has its last two slots in
+// descending order, else ascending, so a lookup goes on only from those (5% of
+// the buckets at half load; 14% are full).
+// A piece is the part of a table that one instance partition's rows are in:
+// its first bucket, and its buckets | kDup when partners are enumerated from
+// the pieces of R2, R3, ....  Pieces without rows are bucket 0, which is free.
+struct Piece {
+    uint32_t first, nbk;
+};
+constexpr uint32_t kDup = 1u << 31;
+
+// A free slot.  A build row that is this very pair cannot be stored: its
+// instance is left to the plain path.
+constexpr uint64_t kFree = 0x8181818181818181ull;
 
 // Top 32 bits of fib_hash(k) in 32-bit arithmetic: with k sign-extended to 64
 // bits, hi32(k * C) = umulhi(k, C_lo) + k * C_hi - (k < 0 ? C_lo : 0) (mod 2^32).
@@ -203,13 +241,42 @@ __device__ __forceinline__ void smem_scan(uint32_t* a, uint32_t n, bool inclusiv
     __syncthreads();
 }
 
-// 0. the relation of every partition-pass item, so that the histogram and
-// scatter blocks find an item's relation with one load instead of a binary
-// search of dependent loads each
-__global__ void k_item_rel(const RelInst* __restrict__ R, uint32_t nr, uint64_t items, uint32_t* __restrict__ rmap) {
+// Where the pieces go: buckets are handed out from a counter (the memory is
+// sized for the rows of all build relations).
+struct Tables {
+    uint64_t* tab;
+    uint32_t* side;      // `stride` words per slot: the payloads of an F slot's partners
+    uint32_t* next;      // buckets handed out, from 1 on
+    uint32_t  stride;
+    uint32_t  slot_q16;  // buckets per row, in 65536ths
+};
+
+// 0. the relation of every partition-pass item, the probe's items and the
+// instance of every instance partition, so that a block finds its work with one
+// load instead of a binary search of dependent loads
+__global__ void k_item_rel(const RelInst* __restrict__ R, uint32_t nr, uint64_t bitems, uint64_t items,
+                           uint32_t* __restrict__ rmap, Item* __restrict__ imap, const InstInfo* __restrict__ I,
+                           uint32_t n, uint64_t nip, uint32_t* __restrict__ pmap, Tables T) {
+    if (blockIdx.x == 0 && threadIdx.x < 4) {  // bucket 0 stays free
+        T.tab[threadIdx.x] = kFree;
+        if (threadIdx.x == 0) *T.next = 1;
+    }
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < items; t += stride)
-        rmap[t] = owner(nr, t, [&](uint32_t i) { return R[i].item_base; });
+    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < items + nip; t += stride) {
+        if (t >= items) {
+            pmap[t - items] = owner(n, t - items, [&](uint32_t i) { return I[i].ip_base; });
+            continue;
+        }
+        const uint32_t ri = owner(nr, t, [&](uint32_t i) { return R[i].item_base; });
+        if (t < bitems) {
+            rmap[t] = ri;
+            continue;
+        }
+        const RelInst& r  = R[ri];
+        const uint64_t r0 = (t - r.item_base) * r.irows;
+        imap[t - bitems]  = Item{r.keys + r0, r.pay + r0, r.part_base, uint32_t(min(r.rows - r0, uint64_t(r.irows))),
+                                r.inst, r.pbits, r.nrel - 2};
+    }
 }
 
 // 1. per (relation, partition) row counts
@@ -362,97 +429,110 @@ __global__ void __launch_bounds__(kPT, 2)
     }
 }
 
-// R0 rows of one join work item: at least 16 per build row, so the table build
-// is amortised (a partition of a probe side 10x its build side is then one
-// item, its tables built once).
-__device__ __forceinline__ uint64_t join_chunk(uint64_t build_rows) {
-    const uint64_t c = 16 * build_rows;
-    return c > kJoinChunk ? c : uint64_t(kJoinChunk);
+struct Slots {
+    uint64_t s[4];
+};
+__device__ __forceinline__ Slots load_bucket(const uint64_t* tab, uint64_t b) {
+    Slots r;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(r.s[0]), "=l"(r.s[1]), "=l"(r.s[2]), "=l"(r.s[3])
+                 : "l"(tab + 4 * b));
+    return r;
 }
+// Home bucket of a key in a piece of nbk buckets: the first steps of
+// MurmurHash3's 32-bit finaliser (Appleby), then the high product.  The
+// partition's multiplicative hash will not do: keys in arithmetic progression
+// can fall into few of its buckets, and linear probing then runs through them
+// (64 chains of 1k .. 16k build rows: 148 us of probing, with this hash 41 us).
+__device__ __forceinline__ uint32_t home_of(int32_t k, uint32_t nbk) {
+    uint32_t h = uint32_t(k);
+    h = (h ^ (h >> 16)) * 0x85ebca6bu;
+    h = (h ^ (h >> 13)) * 0xc2b2ae35u;
+    return __umulhi(h, nbk);
+}
+__device__ __forceinline__ uint64_t slot_of(int32_t k, int32_t p) {
+    return uint64_t(uint32_t(k)) | (uint64_t(uint32_t(p)) << 32);
+}
+__device__ __forceinline__ int32_t slot_key(uint64_t s) { return int32_t(uint32_t(s)); }
+__device__ __forceinline__ int32_t slot_pay(uint64_t s) { return int32_t(uint32_t(s >> 32)); }
+__device__ __forceinline__ bool goes_on(const Slots& s) { return s.s[2] >= s.s[3] && s.s[3] != kFree; }
+__device__ __forceinline__ uint32_t next_bucket(uint32_t b, uint32_t nbk) { return b + 1 == nbk ? 0u : b + 1; }
+
+// Walks the rows of key k in a table, in slot order.
+struct Walk {
+    const uint64_t* tab;
+    uint32_t        nbk, b, left;
+    int32_t         k;
+    Slots           s;
+    int             i;
+    Walk() = default;
+    __device__ __forceinline__ Walk(const uint64_t* tab_, uint32_t nbk_, int32_t k_)
+        : tab(tab_), nbk(nbk_), b(home_of(k_, nbk_)), left(nbk_), k(k_), i(0) {
+        s = load_bucket(tab, b);
+    }
+    // the next such row: its payload and slot in the piece; false at the end
+    __device__ __forceinline__ bool next(int32_t& pay, uint64_t& slot) {
+        for (;;) {
+            for (; i < 4; ++i) {
+                const uint64_t v = i == 0 ? s.s[0] : i == 1 ? s.s[1] : i == 2 ? s.s[2] : s.s[3];
+                if (slot_key(v) == k && v != kFree) {
+                    pay  = slot_pay(v);
+                    slot = uint64_t(b) * 4 + i++;
+                    return true;
+                }
+            }
+            if (!goes_on(s) || --left == 0) return false;
+            b = next_bucket(b, nbk);
+            s = load_bucket(tab, b);
+            i = 0;
+        }
+    }
+};
+
 
 __device__ __forceinline__ uint64_t part_rows(const uint64_t* off, uint64_t pid) { return off[pid + 1] - off[pid]; }
 
-// 4. join work items per instance partition: chunks of its R0 rows (none when
-// any relation's partition is empty: the chain then has no result there)
-__global__ void k_bjoin_plan(const InstInfo* __restrict__ I, uint32_t n, uint64_t nip, const uint64_t* __restrict__ off,
-                             uint32_t* __restrict__ jcnt) {
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < nip; e += stride) {
-        const InstInfo& s   = I[owner(n, e, [&](uint32_t i) { return I[i].ip_base; })];
-        const uint64_t  l   = e - s.ip_base;
-        const uint64_t  np2 = 1ull << s.pbits;
-        const uint64_t  n0  = part_rows(off, s.part_base + l);
-        uint64_t        nb  = 0;
-        bool            any_empty = n0 == 0;
-        for (uint32_t j = 1; j < s.nrel; ++j) {
-            const uint64_t c = part_rows(off, s.part_base + j * np2 + l);
-            nb += c;
-            any_empty |= c == 0;
-        }
-        const uint64_t cs = join_chunk(nb);
-        jcnt[e]           = any_empty ? 0u : uint32_t((n0 + cs - 1) / cs);
-    }
-}
-
-// 4b. the (instance partition, instance) of every join work item, written by
-// each instance partition for its items (one load per item in the join)
-__global__ void k_bjoin_map(const InstInfo* __restrict__ I, uint32_t n, uint64_t nip, const uint64_t* __restrict__ joff,
-                            uint2* __restrict__ jmap) {
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t e = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < nip; e += stride) {
-        const uint64_t a = joff[e], b = joff[e + 1];
-        if (a == b) continue;
-        const uint32_t ii = owner(n, e, [&](uint32_t i) { return I[i].ip_base; });
-        for (uint64_t t = a; t < b; ++t) jmap[t] = make_uint2(uint32_t(e), ii);
-    }
-}
-
-// 5. join.  Shared memory: the build rows of the item's partition in every
-// build relation (keys, payloads; at most `cap` rows together), then per
-// table its bucket bounds.  Table j (relation j + 1) has 2^bits_j buckets
-// after a gap word; after one inclusive scan over all tables' counts and the
-// scatter, bucket b of table j holds tuples [S[sb_j + b + 1], S[sb_j + b + 2]).
-// Each R0 row looks its key up in every table (a cheap compare loop that
-// notes the first match and the count), stops at the first table without it,
-// and forms fingerprints only for complete matches; duplicate keys are
-// enumerated by an odometer over the match lists.  In chains of three or more
-// relations the rows that pass table 0 are queued per warp and looked up in
-// the later tables 32 at a time.
-__global__ void __launch_bounds__(kPT, 2)
-    k_bjoin(const InstInfo* __restrict__ I, const uint2* __restrict__ jmap, uint64_t nip,
-            const uint64_t* __restrict__ joff, unsigned long long* q, const uint64_t* __restrict__ off,
-            const int2* __restrict__ kp, uint32_t cap, uint32_t scap, uint32_t max_bits, uint32_t load_q8,
-            unsigned long long* __restrict__ rows, unsigned long long* __restrict__ sums, uint32_t* __restrict__ ovf) {
+// 4. One block per instance partition.  Shared memory: rows of R2, R3, ...
+// (keys, payloads; at most `cap` rows together), then per table its bucket
+// bounds -- table j (relation j + 2) has 2^bits_j buckets after a gap word;
+// after one inclusive scan over all tables' counts and the scatter, bucket b
+// of table j holds tuples [S[ts_j + b + 1], S[ts_j + b + 2]) -- and the row
+// counters of the piece that is being written.
+// R1's rows are looked up twice: counted, so that the piece is as large as its
+// rows need (tables of long chains shrink with every relation), then placed.
+// Bound by the latency of its phases: two blocks an SM, each at another one.
+constexpr int kBuildT = 512;
+__global__ void __launch_bounds__(kBuildT, 2)
+    k_bt_build(const InstInfo* __restrict__ I, const uint32_t* __restrict__ pmap, uint64_t nip,
+               const uint64_t* __restrict__ off, const int2* __restrict__ kp, uint32_t cap, uint32_t scap,
+               uint32_t fcap, uint32_t max_bits, uint32_t load_q8,
+               Tables T, Piece* __restrict__ pieces, InstOut* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem[];
     int32_t*  skey = reinterpret_cast<int32_t*>(smem);
     int32_t*  spay = skey + cap;
     uint32_t* S    = reinterpret_cast<uint32_t*>(spay + cap);
-    __shared__ unsigned long long sh;
-    __shared__ unsigned long long red[33];
-    __shared__ uint32_t           wsum[32];
-    // table geometry of the current item: bits, rows, first S word, source offset
-    __shared__ uint32_t g_tb[kMaxRel], g_tn[kMaxRel], g_ts[kMaxRel], g_words, g_nb, g_skip;
+    __shared__ uint32_t wsum[32];
+    __shared__ uint32_t g_tb[kMaxRel], g_tn[kMaxRel], g_ts[kMaxRel], g_to[kMaxRel + 1], g_words, g_skip, g_cnt, g_flags,
+        g_first;
     __shared__ uint64_t g_src[kMaxRel];
-    // per warp: rows that matched table 0 once, waiting for the later tables
-    constexpr uint32_t  kRing = 64;
-    __shared__ int32_t  ring_key[kPT / 32][kRing];
-    __shared__ uint64_t ring_fp[kPT / 32][kRing];
-    const uint32_t      lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t items = joff[nip];
-    for (uint64_t t = next_item(q, &sh); t < items; t = next_item(q, &sh)) {
-        const uint2     em  = jmap[t];
-        const uint32_t  e   = em.x, ii = em.y;
+    for (uint64_t e = blockIdx.x; e < nip; e += gridDim.x) {
+        const uint32_t  ii  = pmap[e];
         const InstInfo& s   = I[ii];
-        const uint32_t  pb  = s.pbits;
-        const uint32_t  nt  = s.nrel - 1;  // tables
-        const uint64_t  np2 = 1ull << pb;
-        const uint64_t  l   = e - s.ip_base;
+        const uint32_t  pb  = s.pbits, nt = s.nrel - 2;
+        const uint64_t  np2 = 1ull << pb, l = e - s.ip_base;
+        const uint64_t  pid = s.part_base + l;
+        __syncthreads();  // the last partition is done with shared memory
         if (threadIdx.x == 0) {
-            uint32_t nb = 0;
+            uint64_t all   = part_rows(off, pid);
+            bool     empty = all == 0;
+            uint32_t nb    = 0;
             for (uint32_t j = 0; j < nt; ++j) {
-                const uint64_t pid  = s.part_base + (j + 1) * np2 + l;
-                g_src[j]            = off[pid];
-                g_tn[j]             = uint32_t(part_rows(off, pid));
+                const uint64_t q = pid + (j + 1) * np2, rows = part_rows(off, q);
+                all += rows;
+                empty |= rows == 0;
+                g_src[j] = off[q];
+                g_tn[j]  = uint32_t(rows);
+                g_to[j]  = nb;
                 nb += g_tn[j];
                 const uint32_t want = uint32_t((uint64_t(g_tn[j]) * 256 + load_q8 - 1) / load_q8);
                 g_tb[j]             = min(max_bits, max(1u, want > 1 ? 32u - __clz(want - 1) : 1u));
@@ -474,182 +554,431 @@ __global__ void __launch_bounds__(kPT, 2)
                 w += (1u << g_tb[j]) + 2;
             }
             g_words = words;
-            g_nb    = nb;
             // a partition too large for shared memory: the plain path redoes the instance
-            g_skip  = nb > cap || words > scap;
-            if (g_skip) atomicOr(ovf + ii, 1u);
+            const bool big = all > cap || words > scap;
+            if (big && !empty) out[ii].ovf = 1;
+            g_skip  = big || empty;
+            g_cnt   = 0;
+            g_flags = 0;
+            if (empty || big) pieces[pid] = Piece{0, 1};
         }
         __syncthreads();
         if (g_skip) continue;
-        const uint32_t words = g_words;
+        const uint32_t words = g_words, n1 = uint32_t(part_rows(off, pid));
+        const int2*    r1    = kp + off[pid];
+        // row counters of the piece being written, two to a word (a piece has less than 2^16 rows):
+        // behind the tables, or in their place when there are none
+        uint32_t*      fcnt  = nt ? S + scap : reinterpret_cast<uint32_t*>(smem);
+        const uint32_t nbmax = nt ? fcap : 2 * (2 * cap + scap) + fcap;
+        auto           count = [&](uint32_t b) { return (fcnt[b >> 1] >> (16 * (b & 1))) & 0xffffu; };
         auto bucket = [&](uint32_t j, int32_t k) { return (fib_hi(k) << pb) >> (32 - g_tb[j]); };
-        // build the tables
-        for (uint32_t w = threadIdx.x; w < words; w += kPT) S[w] = 0;
+        // tables of R2, R3, ...
+        for (uint32_t w = threadIdx.x; w < words; w += kBuildT) S[w] = 0;
         __syncthreads();
         // four rows per thread in flight per step, loads before the atomics
         constexpr uint32_t kBU = 4;
         for (uint32_t j = 0; j < nt; ++j) {
             const uint32_t tn = g_tn[j];
-            const int32_t* kj = reinterpret_cast<const int32_t*>(kp + g_src[j]);  // keys: even words
-            for (uint32_t r = threadIdx.x; r < tn; r += kBU * kPT) {
-                int32_t kk[kBU];
+            const int2*    qj = kp + g_src[j];
+            for (uint32_t r = threadIdx.x; r < tn; r += kBU * kBuildT) {
+                int2 kv[kBU];
 #pragma unroll
-                for (uint32_t u = 0; u < kBU; ++u) kk[u] = r + u * kPT < tn ? __ldg(kj + 2 * (r + u * kPT)) : 0;
+                for (uint32_t u = 0; u < kBU; ++u) kv[u] = r + u * kBuildT < tn ? __ldg(qj + r + u * kBuildT) : make_int2(0, 0);
 #pragma unroll
                 for (uint32_t u = 0; u < kBU; ++u)
-                    if (r + u * kPT < tn) atomicAdd(&S[g_ts[j] + bucket(j, kk[u]) + 1], 1u);
+                    if (r + u * kBuildT < tn) atomicAdd(&S[g_ts[j] + bucket(j, kv[u].x) + 1], 1u);
             }
         }
         __syncthreads();
-        smem_scan(S, words, true, wsum);
+        if (nt) smem_scan(S, words, true, wsum);
         for (uint32_t j = 0; j < nt; ++j) {
             const uint32_t tn = g_tn[j];
-            const int2* qj = kp + g_src[j];
-            for (uint32_t r = threadIdx.x; r < tn; r += kBU * kPT) {
-                int32_t kk[kBU], pv[kBU];
+            const int2*    qj = kp + g_src[j];
+            for (uint32_t r = threadIdx.x; r < tn; r += kBU * kBuildT) {
+                int2 kv[kBU];
 #pragma unroll
-                for (uint32_t u = 0; u < kBU; ++u) {
-                    const int2 v = r + u * kPT < tn ? __ldg(qj + r + u * kPT) : make_int2(0, 0);
-                    kk[u]        = v.x;
-                    pv[u]        = v.y;
-                }
+                for (uint32_t u = 0; u < kBU; ++u) kv[u] = r + u * kBuildT < tn ? __ldg(qj + r + u * kBuildT) : make_int2(0, 0);
 #pragma unroll
                 for (uint32_t u = 0; u < kBU; ++u)
-                    if (r + u * kPT < tn) {
-                        const uint32_t pos = atomicSub(&S[g_ts[j] + bucket(j, kk[u]) + 1], 1u) - 1;
-                        skey[pos]          = kk[u];
-                        spay[pos]          = pv[u];
+                    if (r + u * kBuildT < tn) {
+                        const uint32_t pos = atomicSub(&S[g_ts[j] + bucket(j, kv[u].x) + 1], 1u) - 1;
+                        skey[pos]          = kv[u].x;
+                        spay[pos]          = kv[u].y;
                     }
             }
         }
         __syncthreads();
-        // probe the item's R0 rows
-        const uint64_t p0 = off[s.part_base + l];
-        const uint64_t cs = join_chunk(g_nb);
-        const uint64_t x0 = p0 + (t - joff[e]) * cs;
-        const uint32_t m  = uint32_t(min(p0 + part_rows(off, s.part_base + l), x0 + cs) - x0);
-        const int2*    pq = kp + x0;
-        unsigned long long my_rows = 0, my_sum = 0;
-        // matches of key k in bucket word b: their count, and the first in `first`
-        auto scan_bucket = [&](uint32_t b, int32_t k, uint32_t& first) {
-            const uint32_t be = S[b + 2];
-            uint32_t       cnt = 0, j1 = 0;
-            for (uint32_t y = S[b + 1]; y < be; ++y)
+        // rows of table j with key k: their number (0, 1, or 2 for more) and one of them
+        auto lookup = [&](uint32_t j, int32_t k, uint32_t& one) {
+            const uint32_t w = g_ts[j] + bucket(j, k), be = S[w + 2];
+            uint32_t       c = 0;
+            for (uint32_t y = S[w + 1]; y < be && c < 2; ++y)
                 if (skey[y] == k) {
-                    j1 = cnt ? j1 : y;
-                    ++cnt;
+                    one = y;
+                    ++c;
                 }
-            first = j1;
-            return cnt;
+            return c;
         };
-        auto lookup = [&](uint32_t j, int32_t k, uint32_t& first) {
-            return scan_bucket(g_ts[j] + bucket(j, k), k, first);
-        };
-        // table 0, which every row meets, with its geometry in registers
-        const uint32_t ts0 = g_ts[0], sh0 = 32 - g_tb[0];
-        auto lookup0 = [&](int32_t k, uint32_t& first) {
-            return scan_bucket(ts0 + ((fib_hi(k) << pb) >> sh0), k, first);
-        };
-        // every combination of one match per table j0 .. nt-1 for key k, the
-        // tables before j0 folded into fp (an odometer over the match lists)
-        auto enumerate = [&](uint32_t j0, int32_t k, uint64_t fp) {
-            uint32_t first[kMaxRel], pos[kMaxRel];
-            uint64_t fpl[kMaxRel + 1];
-            fpl[j0] = fp;
-            for (uint32_t j = j0; j < nt; ++j) {
-                if (!lookup(j, k, first[j])) return;
-                pos[j]     = first[j];
-                fpl[j + 1] = fp_add(fpl[j], spay[pos[j]]);
+        // R1 rows that are in every table: how many, and whether any has several partners
+        uint32_t mine = nt == 0 && threadIdx.x == 0 ? n1 : 0u, dup = 0;
+        static_assert((2u << 13) / kBuildT <= 32, "a bit for each of a thread's rows");
+        uint32_t found = nt ? 0u : ~0u;  // this thread's rows that are
+        for (uint32_t r = threadIdx.x, i = 0; nt && r < n1; r += kBuildT, ++i) {
+            const int32_t k   = __ldg(r1 + r).x;
+            bool          all = true;
+            for (uint32_t j = 0; j < nt && all; ++j) {
+                uint32_t       y;
+                const uint32_t c = lookup(j, k, y);
+                all              = c > 0;
+                dup |= c > 1;
             }
-            for (;;) {
-                ++my_rows;
-                my_sum += fp_final(fpl[nt]);
-                int j = int(nt) - 1;
-                for (; j >= int(j0); --j) {
-                    const uint32_t be = S[g_ts[j] + bucket(uint32_t(j), k) + 2];
-                    uint32_t       y  = pos[j] + 1;
-                    while (y < be && skey[y] != k) ++y;
-                    if (y < be) {
-                        pos[j] = y;
-                        break;
-                    }
-                    pos[j] = first[j];
-                }
-                if (j < int(j0)) break;
-                for (uint32_t z = uint32_t(j); z < nt; ++z) fpl[z + 1] = fp_add(fpl[z], spay[pos[z]]);
-            }
-        };
-        // the next row's key and payload are loaded while this row is looked up
-        int2 q_next = threadIdx.x < m ? __ldg(pq + threadIdx.x) : make_int2(0, 0);
-        if (nt == 1) {
-            for (uint32_t x = threadIdx.x; x < m; x += kPT) {
-                const int32_t k = q_next.x, pv = q_next.y;
-                if (x + kPT < m) q_next = __ldg(pq + x + kPT);
-                uint32_t       f;
-                const uint32_t c = lookup0(k, f);
-                if (c == 1) {
-                    ++my_rows;
-                    my_sum += fp_final(fp_add(fp_start(k, pv), spay[f]));
-                } else if (c > 1) {
-                    enumerate(0, k, fp_start(k, pv));
-                }
-            }
-        } else {
-            // Table 0 is looked up for every row.  Rows with one match there
-            // queue up in the warp's ring (key and fold state) and the later
-            // tables are looked up 32 queued rows at a time, so that lanes
-            // whose row missed table 0 do not idle through them.
-            int32_t*       qk   = ring_key[warp];
-            uint64_t*      qf   = ring_fp[warp];
-            uint32_t       qh = 0, qt = 0;  // ring head and tail (warp-uniform)
-            auto drain = [&](uint32_t cnt) {
-                __syncwarp();
-                if (lane < cnt) {
-                    const uint32_t slot = (qh + lane) % kRing;
-                    const int32_t  k    = qk[slot];
-                    uint64_t       fp   = qf[slot];
-                    uint32_t       j = 1, c = 1;
-                    for (; j < nt; ++j) {
-                        uint32_t f;
-                        c = lookup(j, k, f);
-                        if (c != 1) break;
-                        fp = fp_add(fp, spay[f]);
-                    }
-                    if (j == nt) {
-                        ++my_rows;
-                        my_sum += fp_final(fp);
-                    } else if (c > 1) {
-                        enumerate(j, k, fp);
-                    }
-                }
-                qh += cnt;
-                __syncwarp();
-            };
-            for (uint32_t x = threadIdx.x; x - lane < m; x += kPT) {  // warp-uniform bound
-                const int32_t k = q_next.x, pv = q_next.y;
-                if (x + kPT < m) q_next = __ldg(pq + x + kPT);
-                uint32_t f = 0, c = 0;
-                if (x < m) c = lookup0(k, f);
-                if (c > 1) enumerate(0, k, fp_start(k, pv));
-                const unsigned hm = __ballot_sync(0xffffffffu, c == 1);
-                if (c == 1) {
-                    const uint32_t slot = (qt + __popc(hm & ((1u << lane) - 1u))) % kRing;
-                    qk[slot]            = k;
-                    qf[slot]            = fp_add(fp_start(k, pv), spay[f]);
-                }
-                qt += __popc(hm);
-                if (qt - qh >= 32) drain(32);
-            }
-            drain(qt - qh);
+            mine += all;
+            found |= uint32_t(all) << i;
         }
-        unsigned long long tr, tsum;
-        block_exclusive_scan<unsigned long long>(my_rows, red, &tr);
-        block_exclusive_scan<unsigned long long>(my_sum, red, &tsum);
-        if (threadIdx.x == 0 && tr) {
-            atomicAdd(rows + ii, tr);
-            atomicAdd(sums + ii, tsum);
+        mine = warp_sum(mine);
+        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&g_cnt, mine);
+        if (dup) g_flags = 1;
+        __syncthreads();
+        // a piece of n rows from the table memory, emptied; counters cleared
+        auto open = [&](uint32_t n, Piece* p, uint32_t d) {
+            const uint32_t nbk = min(nbmax, uint32_t((uint64_t(n) * T.slot_q16) >> 16) + 1);
+            if (threadIdx.x == 0) {
+                g_first = atomicAdd(T.next, nbk);
+                *p      = Piece{g_first, nbk | d};
+            }
+            for (uint32_t b = threadIdx.x; b < (nbk + 1) / 2; b += kBuildT) fcnt[b] = 0;
+            __syncthreads();
+            ulonglong2* to = reinterpret_cast<ulonglong2*>(T.tab + 4 * uint64_t(g_first));
+            for (uint32_t b = threadIdx.x; b < 2 * nbk; b += kBuildT) to[b] = make_ulonglong2(kFree, kFree);
+            __syncthreads();
+            return nbk;
+        };
+        // a row's slot in the open piece (its rows fit: a quarter of the slots or more stays free)
+        auto place = [&](uint32_t nbk, int32_t k, int32_t p) {
+            uint32_t b = home_of(k, nbk), r;
+            while ((r = (atomicAdd(fcnt + (b >> 1), 1u << (16 * (b & 1))) >> (16 * (b & 1))) & 0xffffu) >= 4)
+                b = next_bucket(b, nbk);
+            const uint64_t slot = uint64_t(g_first + b) * 4 + r, v = slot_of(k, p);
+            T.tab[slot] = v;
+            if (v == kFree) out[ii].ovf = 1;
+            return slot;
+        };
+        // the order of each full bucket's last slots (and, in F, of their partners)
+        auto close = [&](uint32_t nbk, uint32_t words) {
+            __syncthreads();
+            for (uint32_t b = threadIdx.x; b < nbk; b += kBuildT) {
+                const uint32_t n = count(b);
+                if (n < 4) continue;
+                const uint64_t c = uint64_t(g_first + b) * 4 + 2;
+                const uint64_t x = T.tab[c], y = T.tab[c + 1];
+                if ((n > 4) == (x >= y)) continue;
+                T.tab[c]     = y;
+                T.tab[c + 1] = x;
+                for (uint32_t j = 0; j < words; ++j) {
+                    const uint32_t w                  = T.side[c * T.stride + j];
+                    T.side[c * T.stride + j]          = T.side[(c + 1) * T.stride + j];
+                    T.side[(c + 1) * T.stride + j]    = w;
+                }
+            }
+        };
+        const uint32_t fl  = g_flags ? kDup : 0u;
+        const uint32_t nbk = open(g_cnt, pieces + pid, fl);
+        for (uint32_t r = threadIdx.x; r < n1; r += kBuildT, found = nt ? found >> 1 : ~0u) {
+            if (!(found & 1u)) continue;
+            const int2     kv   = __ldg(r1 + r);
+            const uint64_t slot = place(nbk, kv.x, kv.y);
+            for (uint32_t j = 0; j < nt; ++j) {
+                uint32_t y = 0;
+                lookup(j, kv.x, y);
+                T.side[slot * T.stride + j] = uint32_t(spay[y]);
+            }
+        }
+        close(nbk, nt);
+        // duplicates: R2, R3, ... as pieces too
+        if (fl) {
+            if (threadIdx.x == 0) out[ii].dups = 1;
+            for (uint32_t j = 0; j < nt; ++j) {
+                __syncthreads();
+                const uint32_t tn = g_tn[j], nb = open(tn, pieces + pid + (j + 1) * np2, 0);
+                for (uint32_t r = threadIdx.x; r < tn; r += kBuildT) place(nb, skey[g_to[j] + r], spay[g_to[j] + r]);
+                close(nb, 0);
+            }
         }
     }
+}
+
+constexpr int kBT = 256;  // threads of the probe
+constexpr int kU  = 2;    // rows per thread in flight
+
+// Sums of the instance that a warp is at, added to its result when it comes to another.
+struct Sums {
+    unsigned long long rows = 0, sum = 0;
+    uint32_t           cur  = ~0u;
+    // every lane of the warp calls it
+    __device__ __forceinline__ void at(uint32_t inst, InstOut* out) {
+        if (inst == cur) return;
+        if (cur != ~0u) {
+            const unsigned long long tr = warp_sum(rows), ts = warp_sum(sum);
+            if ((threadIdx.x & 31) == 0 && tr) {
+                atomicAdd(&out[cur].rows, tr);
+                atomicAdd(&out[cur].sum, ts);
+            }
+        }
+        rows = sum = 0;
+        cur        = inst;
+    }
+};
+
+// 5. R0 rows against F.  kU rows a thread: keys and payloads of the next rows
+// are on their way while the buckets of these are looked at.  Bound by its
+// instructions and the L1's lines (about 155 a row of 32, 56% issue active, the
+// L1 77% busy: 142e9 rows/s on 1M-row tables), so the bucket reads allocate no
+// L1 lines, two rows a thread fit 64 registers without spills, and what only
+// some rows need is put off until a whole warp needs it: matches wait in the warp's queue until 32 of them are folded
+// together, and rows that have to go on to a next bucket (one in twenty at half
+// load, some in every warp) until 32 of them look together.  The instance's
+// pieces are kept in shared memory (reads of them through L1 would cost as
+// much as the buckets).  Each match of a key in F is a result row, unless R2,
+// R3, ... hold duplicates (k_bt_enum).
+constexpr uint32_t kQueue = 96;  // a step leaves at most 31 rows and adds at most 32 * kU
+static_assert(31 + 32 * kU <= int(kQueue), "a step's rows fit the queues");
+struct Queues {
+    int4     hit[kQueue];  // key, payloads of R0 and R1, F slot
+    int2     kp[kQueue];   // rows that go on, and the bucket they come from
+    uint32_t b[kQueue];
+};
+__global__ void __launch_bounds__(kBT, 4)
+    k_bt_probe(const Item* __restrict__ imap, uint64_t items, const uint64_t* __restrict__ tabs,
+               const uint32_t* __restrict__ side, uint32_t stride, const Piece* __restrict__ pieces,
+               InstOut* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    Piece* dir = reinterpret_cast<Piece*>(smem);  // the instance's pieces
+    __shared__ __align__(16) Queues queues[kBT / 32];
+    const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+    Queues&        Q    = queues[threadIdx.x >> 5];
+    uint32_t       qn = 0, hn = 0;  // entries of the two (the same in every lane)
+    Sums           acc;
+    uint32_t       pb = 0, nt = 0;
+    bool           skip = true;
+    auto home = [&](int32_t k) {
+        const Piece x = dir[part_of(k, pb)];
+        return x.first + home_of(k, x.nbk);
+    };
+    // Matches folded into the sums, 32 at a time, until fewer than `keep` wait.
+    auto fold = [&](uint32_t keep) {
+        while (hn >= keep && hn) {
+            __syncwarp();
+            const uint32_t n = hn < 32 ? hn : 32;
+            hn -= n;
+            if (lane < n) {
+                const int4 h  = Q.hit[hn + lane];
+                uint64_t   fp = fp_add(fp_start(h.x, h.y), h.z);
+                if (nt) {
+                    const uint32_t* w = side + uint64_t(uint32_t(h.w)) * stride;
+                    for (uint32_t j = 0; j < nt; ++j) fp = fp_add(fp, int32_t(__ldg(w + j)));
+                }
+                ++acc.rows;
+                acc.sum += fp_final(fp);
+            }
+            __syncwarp();
+        }
+    };
+    // Key k in its loaded bucket: its matches and the row itself to the queues.
+    auto look = [&](bool on, int32_t k, int32_t p, uint32_t b, const Slots& q) {
+        uint32_t m = 0;
+        if (slot_key(q.s[0]) == k) m = 1;
+        if (slot_key(q.s[1]) == k) m |= 2;
+        if (slot_key(q.s[2]) == k) m |= 4;
+        if (slot_key(q.s[3]) == k) m |= 8;
+        if (k == slot_key(kFree)) {  // a free slot is no match
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (q.s[i] == kFree) m &= ~(1u << i);
+        }
+        if (!on) m = 0;
+        for (unsigned bal; (bal = __ballot_sync(0xffffffffu, m != 0)) != 0;) {  // once, unless a key has several rows
+            if (m) {
+                const int32_t p1 = (m & 1) ? slot_pay(q.s[0]) : (m & 2) ? slot_pay(q.s[1]) : (m & 4) ? slot_pay(q.s[2])
+                                                                                              : slot_pay(q.s[3]);
+                Q.hit[hn + __popc(bal & lt)] = make_int4(k, p, p1, int32_t(b * 4 + __ffs(m) - 1));
+                m &= m - 1;
+            }
+            hn += __popc(bal);
+            if (hn > kQueue - 32) fold(32);
+        }
+        const bool     on2 = on && goes_on(q);
+        const unsigned bal = __ballot_sync(0xffffffffu, on2);
+        if (on2) {
+            const uint32_t at = qn + __popc(bal & lt);
+            Q.kp[at]          = make_int2(k, p);
+            Q.b[at]           = b;
+        }
+        qn += __popc(bal);
+    };
+    // The rows that go on, at their next buckets, until fewer than `keep` wait.
+    auto go_on = [&](uint32_t keep) {
+        while (qn >= keep && qn) {
+            __syncwarp();
+            const uint32_t n  = qn < 32 ? qn : 32;
+            const bool     on = lane < n;
+            qn -= n;
+            int2           kp = make_int2(0, 0);
+            uint32_t       b  = 0;
+            if (on) {
+                kp            = Q.kp[qn + lane];
+                b             = Q.b[qn + lane] + 1;
+                const Piece x = dir[part_of(kp.x, pb)];
+                if (b == x.first + x.nbk) b = x.first;
+            }
+            const Slots q = load_bucket(tabs, b);
+            __syncwarp();
+            look(on, kp.x, kp.y, b, q);
+            fold(32);
+        }
+    };
+    for (uint64_t t = blockIdx.x; t < items; t += gridDim.x) {
+        const Item it = imap[t];
+        if (it.inst != acc.cur) {
+            go_on(0);
+            fold(0);
+            acc.at(it.inst, out);
+            skip = out[it.inst].ovf || out[it.inst].dups;
+            pb   = it.pbits;
+            nt   = it.nt;
+            __syncthreads();
+            for (uint32_t x = threadIdx.x; x < (1u << pb); x += kBT) dir[x] = pieces[it.part_base + x];
+            __syncthreads();
+        }
+        if (skip) continue;
+        const int32_t *kk = it.k + threadIdx.x, *pp = it.p + threadIdx.x;
+        int            left = int(it.n) - int(threadIdx.x);  // rows from this thread's next one on
+        int32_t        nk[kU], np[kU];
+        auto           fetch = [&]() {
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                nk[u] = np[u] = 0;
+                if (left > u * kBT) {
+                    nk[u] = __ldcs(kk + u * kBT);
+                    np[u] = __ldcs(pp + u * kBT);
+                }
+            }
+            kk += kU * kBT;
+            pp += kU * kBT;
+        };
+        fetch();
+        for (int steps = int((it.n + kU * kBT - 1) / (kU * kBT)); steps > 0; --steps) {
+            int32_t  k[kU], p[kU];
+            uint32_t b[kU];
+            bool     on[kU];
+            Slots    q[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                k[u]  = nk[u];
+                p[u]  = np[u];
+                on[u] = left > u * kBT;
+                b[u]  = home(k[u]);
+                q[u]  = load_bucket(tabs, b[u]);
+            }
+            left -= kU * kBT;
+            fetch();
+#pragma unroll
+            for (int u = 0; u < kU; ++u) look(on[u], k[u], p[u], b[u], q[u]);
+            go_on(32);
+            fold(32);
+        }
+    }
+    go_on(0);
+    fold(0);
+    acc.at(~0u, out);
+}
+
+// 6. The same for instances whose R2, R3, ... hold a key of R1 more than once:
+// each F row of the key with every combination of one partner per table (an
+// odometer).  Up to kKeep partners a table are kept in the thread; a table
+// with more is walked for every combination of the tables before it.
+__global__ void __launch_bounds__(kBT)
+    k_bt_enum(const Item* __restrict__ imap, uint64_t items, const uint64_t* __restrict__ tabs,
+              const uint32_t* __restrict__ side, uint32_t stride, const Piece* __restrict__ pieces,
+              InstOut* __restrict__ out) {
+    constexpr int kKeep = 8;
+    Sums          acc;
+    for (uint64_t t = blockIdx.x; t < items; t += gridDim.x) {
+        const Item it = imap[t];
+        if (out[it.inst].ovf || !out[it.inst].dups) continue;
+        const uint32_t nt = it.nt, pb = it.pbits;
+        // walk over key k's rows of relation j + 1
+        auto walk = [&](uint32_t j, int32_t k) {
+            const Piece x = pieces[it.part_base + (uint64_t(j) << pb) + part_of(k, pb)];
+            return Walk(tabs + 4 * uint64_t(x.first), x.nbk & ~kDup, k);
+        };
+        acc.at(it.inst, out);
+        for (uint32_t x = threadIdx.x; x < it.n; x += kBT) {
+            const int32_t  k = __ldcs(it.k + x);
+            const uint64_t fp0 = fp_start(k, __ldcs(it.p + x));
+            int32_t        kept[kMaxRel - 2][kKeep], pay[kMaxRel - 2];  // pay: the combination's partners
+            uint32_t       cnt[kMaxRel - 2], at[kMaxRel - 2];
+            Walk           at_big[kMaxRel - 2];
+            uint64_t       fpl[kMaxRel - 1], slot;
+            int32_t        p;
+            Walk           f    = walk(0, k);
+            bool           some = f.next(p, slot);  // a key in F is in every table
+            if (!some) continue;
+            const Piece x1 = pieces[it.part_base + part_of(k, pb)];
+            if (!(x1.nbk & kDup)) {  // this partition has one partner per table
+                for (; some; some = f.next(p, slot)) {
+                    const uint32_t* w  = side + (uint64_t(x1.first) * 4 + slot) * stride;
+                    uint64_t        fp = fp_add(fp0, p);
+                    for (uint32_t j = 0; j < nt; ++j) fp = fp_add(fp, int32_t(w[j]));
+                    ++acc.rows;
+                    acc.sum += fp_final(fp);
+                }
+                continue;
+            }
+            for (uint32_t j = 0; j < nt; ++j) {
+                Walk           w = walk(j + 1, k);
+                uint32_t       c = 0;
+                int32_t        pj;
+                while (w.next(pj, slot)) {
+                    if (c < kKeep) kept[j][c] = pj;
+                    ++c;
+                }
+                cnt[j] = c;
+                at[j]  = 0;
+                pay[j] = kept[j][0];
+                if (c > kKeep) {
+                    at_big[j] = walk(j + 1, k);
+                    at_big[j].next(pj, slot);
+                }
+            }
+            // the next partner of table j; back at the first one, false
+            auto step = [&](uint32_t j) {
+                if (cnt[j] <= kKeep) {
+                    const bool more = ++at[j] < cnt[j];
+                    if (!more) at[j] = 0;
+                    pay[j] = kept[j][at[j]];
+                    return more;
+                }
+                uint64_t sl;
+                if (at_big[j].next(pay[j], sl)) return true;
+                at_big[j] = walk(j + 1, k);
+                at_big[j].next(pay[j], sl);
+                return false;
+            };
+            for (; some; some = f.next(p, slot)) {
+                fpl[0] = fp_add(fp0, p);
+                for (uint32_t z = 0;;) {
+                    for (; z < nt; ++z) fpl[z + 1] = fp_add(fpl[z], pay[z]);
+                    ++acc.rows;
+                    acc.sum += fp_final(fpl[nt]);
+                    int j = int(nt) - 1;
+                    while (j >= 0 && !step(uint32_t(j))) --j;
+                    if (j < 0) break;
+                    z = uint32_t(j);
+                }
+            }
+        }
+    }
+    acc.at(~0u, out);
 }
 
 // ---- plain path helper --------------------------------------------------------
@@ -689,10 +1018,10 @@ uint32_t ceil_log2u(uint64_t x) {
 // memory (the grid of a persistent launch); raises the kernel's dynamic
 // shared-memory limit first.  Not capturable: called before a capture.
 template <class K>
-int resident_grid(K kernel, size_t smem) {
+int resident_grid(K kernel, int threads, size_t smem) {
     HJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
-    HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPT, smem));
+    HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
     if (per_sm < 1) throw Error(HJ_ERR_INVALID, "batch: a kernel does not fit on an SM");
     return per_sm * num_sms();
 }
@@ -713,7 +1042,224 @@ void launch_batch_generate(uint64_t seed, uint32_t instance, uint32_t relation, 
     HJ_LAUNCH_CHECK();
 }
 
-std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const BatchOptions& o,
+void BatchGraph::clear() {
+    if (exec) cudaGraphExecDestroy(exec);
+    exec = nullptr;
+}
+
+namespace {
+
+// What the options give for partitions of ~T build rows (all build relations
+// together): tables of up to 2T rows in shared memory, bucket bounds for
+// 2^max_bits buckets; and in HBM the same load, kept where linear probing stays
+// short, with a counter per bucket of a piece (a piece of `cap` rows always
+// fits its counters).
+struct Geometry {
+    uint64_t T;
+    uint32_t cap, max_bits, scap, load_q8, fcap;
+    double   buckets_per_row;
+    size_t   build_smem;
+};
+
+Geometry geometry(const BatchOptions& o) {
+    Geometry g;
+    g.T        = 1ull << o.part_rows_log2;
+    g.cap      = uint32_t(2 * g.T);
+    g.max_bits = std::max<uint32_t>(1, ceil_log2u(uint64_t(std::ceil(double(g.T) / o.load))));
+    g.scap     = (1u << g.max_bits) + 2 * kMaxRel;
+    g.load_q8  = std::max<uint32_t>(1, uint32_t(std::lround(o.load * 256.0)));
+    const size_t tables = size_t(g.cap) * 8 + size_t(g.scap) * 4;
+    if (tables > 200 * 1024) throw Error(HJ_ERR_INVALID, "batch: partition tables exceed shared memory");
+    g.buckets_per_row = 0.25 / std::min(0.8, std::max(0.25, o.load));
+    g.fcap = uint32_t(std::min<uint64_t>(uint64_t(double(g.cap) * g.buckets_per_row) + 1, (220 * 1024 - tables) / 2));
+    g.build_smem = tables + size_t(g.fcap) * 2 + 4;
+    return g;
+}
+
+// Build rows of an instance, all build relations together; 0 when one of them has none (no result rows).
+uint64_t build_rows_of(const BatchInstance& b) {
+    uint64_t nb = 0;
+    for (size_t j = 1; j < b.rels.size(); ++j) {
+        if (!b.rels[j].rows) return 0;
+        nb += b.rels[j].rows;
+    }
+    return nb;
+}
+
+// Instances [i0, i1) of the batch; the ones in `plain` (left to the plain path) as if without rows.
+void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1, const std::vector<uint8_t>& plain,
+                const BatchOptions& o, const Geometry& G, BatchGraph& graph, uint64_t* rows, uint64_t* sums,
+                std::vector<uint32_t>& bad, cudaStream_t st) {
+    const uint32_t n = i1 - i0;
+    auto           rel_of = [&](uint32_t i, uint32_t j) {
+        BatchRelation r = all[i0 + i].rels[j];
+        if (plain[i0 + i]) r.rows = 0;
+        return r;
+    };
+    const uint64_t T   = G.T;
+    const uint32_t cap = G.cap, scap = G.scap, fcap = G.fcap, max_bits = G.max_bits, load_q8 = G.load_q8;
+    const double   buckets_per_row = G.buckets_per_row;
+    const size_t   build_smem      = G.build_smem;
+    std::vector<RelInst>  hr;
+    std::vector<InstInfo> hi(n);
+    uint64_t pbase = 0, ipbase = 0, items = 0, build_rows = 0;
+    uint32_t pmax = 0, stride = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t nrel = uint32_t(all[i0 + i].rels.size());
+        uint64_t       nb   = 0;
+        for (uint32_t j = 1; j < nrel; ++j) nb += rel_of(i, j).rows;
+        const uint32_t p = nb > T ? std::min(kMaxPartBits, ceil_log2u((nb + T - 1) / T)) : 0;
+        InstInfo&      s = hi[i];
+        pmax             = std::max(pmax, p);
+        s.part_base      = pbase;
+        s.ip_base        = ipbase;
+        s.nrel           = nrel;
+        s.pbits          = p;
+        stride           = std::max(stride, s.nrel - 2);
+        for (uint32_t j = 1; j < s.nrel; ++j) {
+            const BatchRelation br = rel_of(i, j);
+            hr.push_back({br.keys, br.payload, br.rows, items, pbase + (uint64_t(j - 1) << p), p, i, 0, 0});
+            items += (br.rows + kPartItem - 1) / kPartItem;
+        }
+        build_rows += nb;
+        pbase += uint64_t(s.nrel - 1) << p;
+        ipbase += 1ull << p;
+    }
+    // persistent grids (occupancy queries are not capturable: take them first)
+    const size_t hist_smem = (size_t(1) << pmax) * 4;
+    const size_t scat_smem = size_t(kPartItem) * 10 + (size_t(1) << pmax) * 16;
+    const size_t prb_smem  = (size_t(1) << pmax) * sizeof(Piece);
+    const int    g_hist    = resident_grid(k_bpart_hist, kPT, hist_smem);
+    const int    g_scat    = resident_grid(k_bpart_scatter, kPT, scat_smem);
+    const int    g_bld     = resident_grid(k_bt_build, kBuildT, build_smem);
+    const int    g_prb     = resident_grid(k_bt_probe, kBT, prb_smem);
+    const int    g_enm     = resident_grid(k_bt_enum, kBT, 0);
+    auto grid_for = [](int g, uint64_t work) { return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, work))); };
+
+    // R0s: an item is what one block has of its instance's rows when the grid
+    // shares them twice over, so that blocks stay with an instance, within
+    // 16 .. 64 steps of a block
+    const uint64_t bitems = items;  // items of the build relations, then of the R0s
+    constexpr uint64_t kStepRows = uint64_t(kBT) * kU;
+    for (uint32_t i = 0; i < n; ++i) {
+        const BatchRelation  br    = rel_of(i, 0);
+        const uint64_t       steps = br.rows / (2 * uint64_t(g_prb) * kStepRows);
+        const uint64_t       irows = std::min<uint64_t>(std::max<uint64_t>(steps, 16), 64) * kStepRows;
+        hr.push_back({br.keys, br.payload, br.rows, items, hi[i].part_base, hi[i].pbits, i, uint32_t(irows), hi[i].nrel});
+        items += (br.rows + irows - 1) / irows;
+    }
+    const uint32_t nr   = uint32_t(hr.size());
+    const uint64_t nbkt = uint64_t(double(build_rows) * buckets_per_row) + pbase + 2;
+
+    std::vector<InstOut> ho(n);
+    std::vector<void*>   owned;
+    struct Release {
+        std::vector<void*>& v;
+        cudaStream_t        st;
+        ~Release() {
+            // the host arrays above are read and written by copies on the stream
+            if (std::uncaught_exceptions()) cudaStreamSynchronize(st);
+            for (void* p : v) dfree(p, st);
+        }
+    } release{owned, st};
+    auto take = [&](size_t bytes) {
+        void* p = dalloc(bytes + 16, st);
+        owned.push_back(p);
+        return p;
+    };
+    // results, counters and queues, cleared by one fill
+    const size_t zero_bytes = n * sizeof(InstOut) + 4 * 8 + 2 * (pbase + 1) * 4;
+    auto*        d_out      = static_cast<InstOut*>(take(zero_bytes));
+    auto*        d_q        = reinterpret_cast<unsigned long long*>(d_out + n);
+    auto*        cnt        = reinterpret_cast<uint32_t*>(d_q + 4);
+    auto*        fill       = cnt + pbase + 1;
+    // relations and instances, copied together
+    std::vector<uint8_t> hd(nr * sizeof(RelInst) + n * sizeof(InstInfo));
+    std::memcpy(hd.data(), hr.data(), nr * sizeof(RelInst));
+    std::memcpy(hd.data() + nr * sizeof(RelInst), hi.data(), n * sizeof(InstInfo));
+    auto* d_R    = static_cast<RelInst*>(take(hd.size()));
+    auto* d_I    = reinterpret_cast<InstInfo*>(d_R + nr);
+    auto* off    = static_cast<uint64_t*>(take((pbase + 2) * 8));
+    auto* pieces = static_cast<Piece*>(take((pbase + 1) * sizeof(Piece)));
+    auto* tmp    = static_cast<uint64_t*>(take((scan_tmp_words(pbase) + 1) * 8));
+    auto* pkp    = static_cast<int2*>(take(build_rows * 8));  // (key, payload) in partition order
+    auto* rmap   = static_cast<uint32_t*>(take(bitems * 4));
+    auto* imap   = static_cast<Item*>(take((items - bitems) * sizeof(Item)));
+    auto* pmap   = static_cast<uint32_t*>(take(ipbase * 4));
+    auto* tabs   = static_cast<uint64_t*>(take(nbkt * 32));
+    auto* side   = static_cast<uint32_t*>(take(nbkt * 4 * stride * 4));
+    HJ_CUDA(cudaMemcpyAsync(d_R, hd.data(), hd.size(), cudaMemcpyHostToDevice, st));
+
+    Tables tb{tabs, side, reinterpret_cast<uint32_t*>(d_q + 2), stride, uint32_t(std::lround(buckets_per_row * 65536.0))};
+
+    auto enqueue = [&]() {
+        HJ_CUDA(cudaMemsetAsync(d_out, 0, zero_bytes, st));
+        if (!build_rows || items == bitems) return;  // no result rows
+        k_item_rel<<<unsigned(std::min<uint64_t>(div_up(items + ipbase, 256), uint64_t(num_sms()) * 8)), 256, 0, st>>>(
+            d_R, nr, bitems, items, rmap, imap, d_I, n, ipbase, pmap, tb);
+        HJ_LAUNCH_CHECK();
+        k_bpart_hist<<<grid_for(g_hist, bitems), kPT, hist_smem, st>>>(d_R, rmap, bitems, cnt);
+        HJ_LAUNCH_CHECK();
+        scan_exclusive_u32_to_u64_into(cnt, off, pbase, tmp, st);
+        k_bpart_scatter<<<grid_for(g_scat, bitems), kPT, scat_smem, st>>>(d_R, rmap, bitems, d_q + 1, off, fill, pmax,
+                                                                          pkp);
+        HJ_LAUNCH_CHECK();
+        k_bt_build<<<grid_for(g_bld, ipbase), kBuildT, build_smem, st>>>(d_I, pmap, ipbase, off, pkp, cap, scap, fcap,
+                                                                         max_bits, load_q8, tb, pieces, d_out);
+        HJ_LAUNCH_CHECK();
+        k_bt_probe<<<grid_for(g_prb, items - bitems), kBT, prb_smem, st>>>(imap, items - bitems, tabs, side, stride,
+                                                                           pieces, d_out);
+        HJ_LAUNCH_CHECK();
+        if (stride) {
+            k_bt_enum<<<grid_for(g_enm, items - bitems), kBT, 0, st>>>(imap, items - bitems, tabs, side, stride,
+                                                                       pieces, d_out);
+            HJ_LAUNCH_CHECK();
+        }
+    };
+    if (o.graph) {
+        cudaGraph_t g = nullptr;
+        HJ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        try {
+            enqueue();
+        } catch (...) {
+            cudaStreamEndCapture(st, &g);
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            throw;
+        }
+        HJ_CUDA(cudaStreamEndCapture(st, &g));
+        // the last call's executable graph takes this call's parameters when
+        // its kernels are the same (10 us), else it is made anew (60 us)
+        cudaError_t e = cudaSuccess;
+        if (graph.exec) {
+            cudaGraphExecUpdateResultInfo info;
+            if (cudaGraphExecUpdate(graph.exec, g, &info) != cudaSuccess) {
+                cudaGetLastError();
+                graph.clear();
+            }
+        }
+        if (!graph.exec) e = cudaGraphInstantiate(&graph.exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            graph.exec = nullptr;
+            throw Error(HJ_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
+        }
+        HJ_CUDA(cudaGraphLaunch(graph.exec, st));
+    } else {
+        enqueue();
+    }
+    readback(ho.data(), d_out, n * sizeof(InstOut), o.host_write, st);
+    HJ_CUDA(cudaStreamSynchronize(st));
+    for (uint32_t i = 0; i < n; ++i) {
+        rows[i0 + i] = ho[i].rows;
+        sums[i0 + i] = ho[i].sum;
+        if (ho[i].ovf) bad.push_back(i0 + i);
+    }
+}
+
+}  // namespace
+
+std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const BatchOptions& o, BatchGraph& graph,
                                     std::vector<uint64_t>& rows, std::vector<uint64_t>& sums, cudaStream_t st) {
     const uint32_t n = uint32_t(B.size());
     rows.assign(n, 0);
@@ -730,150 +1276,31 @@ std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const B
             if (r.rows && (!r.keys || !r.payload)) throw Error(HJ_ERR_INVALID, "a batch relation lacks its columns");
         }
     }
-    // shared-memory geometry: partitions of ~T build rows (all build relations
-    // together), tables of up to 2T rows, bucket bounds for 2^max_bits buckets
-    const uint64_t T        = 1ull << o.part_rows_log2;
-    const uint32_t cap      = uint32_t(2 * T);
-    const uint32_t max_bits = std::max<uint32_t>(1, ceil_log2u(uint64_t(std::ceil(double(T) / o.load))));
-    const uint32_t scap     = (1u << max_bits) + 2 * kMaxRel;
-    const uint32_t load_q8  = std::max<uint32_t>(1, uint32_t(std::lround(o.load * 256.0)));
-    const size_t   join_smem = size_t(cap) * 8 + size_t(scap) * 4;
-    if (join_smem > 200 * 1024) throw Error(HJ_ERR_INVALID, "batch: partition tables exceed shared memory");
-
-    std::vector<RelInst>  hr;
-    std::vector<InstInfo> hi(n);
-    uint64_t pbase = 0, ipbase = 0, items = 0, total_rows = 0, r0_rows = 0;
-    uint32_t pmax = 0;
-    for (uint32_t i = 0; i < n; ++i) {
-        uint64_t nb = 0;
-        for (size_t j = 1; j < B[i].rels.size(); ++j) nb += B[i].rels[j].rows;
-        const uint32_t p = nb > T ? std::min(kMaxPartBits, ceil_log2u((nb + T - 1) / T)) : 0;
-        pmax             = std::max(pmax, p);
-        InstInfo& s      = hi[i];
-        s.part_base      = pbase;
-        s.ip_base        = ipbase;
-        s.nrel           = uint32_t(B[i].rels.size());
-        s.pbits          = p;
-        for (uint32_t j = 0; j < s.nrel; ++j) {
-            const BatchRelation& br = B[i].rels[j];
-            hr.push_back({br.keys, br.payload, br.rows, items, pbase + (uint64_t(j) << p), p, i});
-            items += (br.rows + kPartItem - 1) / kPartItem;
-            total_rows += br.rows;
-        }
-        r0_rows += B[i].rels[0].rows;
-        pbase += uint64_t(s.nrel) << p;
-        ipbase += 1ull << p;
-    }
-    const uint32_t nr = uint32_t(hr.size());
-
-    std::vector<void*> owned;
-    struct Release {
-        std::vector<void*>& v;
-        cudaStream_t        st;
-        ~Release() {
-            for (void* p : v) dfree(p, st);
-        }
-    } release{owned, st};
-    auto take = [&](size_t bytes) {
-        void* p = dalloc(bytes + 16, st);
-        owned.push_back(p);
-        return p;
-    };
-    auto* d_rows = static_cast<unsigned long long*>(take(n * 8));
-    auto* d_sums = static_cast<unsigned long long*>(take(n * 8));
-    auto* d_ovf  = static_cast<uint32_t*>(take(n * 4));
-    auto* d_q    = static_cast<unsigned long long*>(take(4 * 8));
-    auto* d_R    = static_cast<RelInst*>(take(nr * sizeof(RelInst)));
-    auto* d_I    = static_cast<InstInfo*>(take(n * sizeof(InstInfo)));
-    auto* cnt    = static_cast<uint32_t*>(take((pbase + 1) * 4));
-    auto* fill   = static_cast<uint32_t*>(take((pbase + 1) * 4));
-    auto* off    = static_cast<uint64_t*>(take((pbase + 2) * 8));
-    auto* jcnt   = static_cast<uint32_t*>(take((ipbase + 1) * 4));
-    auto* joff   = static_cast<uint64_t*>(take((ipbase + 2) * 8));
-    auto* tmp    = static_cast<uint64_t*>(take((std::max(scan_tmp_words(pbase), scan_tmp_words(ipbase)) + 1) * 8));
-    auto* pkp    = static_cast<int2*>(take(total_rows * 8));  // (key, payload) in partition order
-    auto* rmap   = static_cast<uint32_t*>(take(items * 4));
-    // join items: at most one per instance partition plus one per kJoinChunk R0 rows
-    auto* jmap   = static_cast<uint2*>(take((ipbase + r0_rows / kJoinChunk + 1) * 8));
-    HJ_CUDA(cudaMemcpyAsync(d_R, hr.data(), nr * sizeof(RelInst), cudaMemcpyHostToDevice, st));
-    HJ_CUDA(cudaMemcpyAsync(d_I, hi.data(), n * sizeof(InstInfo), cudaMemcpyHostToDevice, st));
-    HJ_CUDA(cudaStreamSynchronize(st));  // the host arrays stay alive until here
-
-    // persistent grids (occupancy queries are not capturable: take them first)
-    const size_t hist_smem = (size_t(1) << pmax) * 4;
-    const size_t scat_smem = size_t(kPartItem) * 10 + (size_t(1) << pmax) * 16;
-    const int    g_hist    = resident_grid(k_bpart_hist, hist_smem);
-    const int    g_scat    = resident_grid(k_bpart_scatter, scat_smem);
-    const int    g_join    = resident_grid(k_bjoin, join_smem);
-    auto grid_for = [](int g, uint64_t work) { return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, work))); };
-
-    auto enqueue = [&]() {
-        HJ_CUDA(cudaMemsetAsync(d_rows, 0, n * 8, st));
-        HJ_CUDA(cudaMemsetAsync(d_sums, 0, n * 8, st));
-        HJ_CUDA(cudaMemsetAsync(d_ovf, 0, n * 4, st));
-        HJ_CUDA(cudaMemsetAsync(d_q, 0, 4 * 8, st));
-        HJ_CUDA(cudaMemsetAsync(cnt, 0, (pbase + 1) * 4, st));
-        HJ_CUDA(cudaMemsetAsync(fill, 0, (pbase + 1) * 4, st));
-        if (items) {
-            k_item_rel<<<unsigned(std::min<uint64_t>(div_up(items, 256), uint64_t(num_sms()) * 8)), 256, 0, st>>>(
-                d_R, nr, items, rmap);
-            HJ_LAUNCH_CHECK();
-            k_bpart_hist<<<grid_for(g_hist, items), kPT, hist_smem, st>>>(d_R, rmap, items, cnt);
-            HJ_LAUNCH_CHECK();
-        }
-        scan_exclusive_u32_to_u64_into(cnt, off, pbase, tmp, st);
-        if (items) {
-            k_bpart_scatter<<<grid_for(g_scat, items), kPT, scat_smem, st>>>(d_R, rmap, items, d_q + 1, off, fill,
-                                                                             pmax, pkp);
-            HJ_LAUNCH_CHECK();
-        }
-        k_bjoin_plan<<<unsigned(std::min<uint64_t>(div_up(ipbase, 256), uint64_t(num_sms()) * 8)), 256, 0, st>>>(
-            d_I, n, ipbase, off, jcnt);
-        HJ_LAUNCH_CHECK();
-        scan_exclusive_u32_to_u64_into(jcnt, joff, ipbase, tmp, st);
-        k_bjoin_map<<<unsigned(std::min<uint64_t>(div_up(ipbase, 256), uint64_t(num_sms()) * 8)), 256, 0, st>>>(
-            d_I, n, ipbase, joff, jmap);
-        HJ_LAUNCH_CHECK();
-        // the item count lives on the device: launch the resident grid
-        k_bjoin<<<unsigned(g_join), kPT, join_smem, st>>>(d_I, jmap, ipbase, joff, d_q + 2, off, pkp, cap,
-                                                          scap, max_bits, load_q8, d_rows, d_sums, d_ovf);
-        HJ_LAUNCH_CHECK();
-    };
-    if (o.graph) {
-        cudaGraph_t g = nullptr;
-        HJ_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        try {
-            enqueue();
-        } catch (...) {
-            cudaStreamEndCapture(st, &g);
-            if (g) cudaGraphDestroy(g);
-            cudaGetLastError();
-            throw;
-        }
-        HJ_CUDA(cudaStreamEndCapture(st, &g));
-        cudaGraphExec_t   ge = nullptr;
-        const cudaError_t e  = cudaGraphInstantiate(&ge, g, 0);
-        if (e != cudaSuccess) {
-            cudaGraphDestroy(g);
-            throw Error(HJ_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-        }
-        const cudaError_t le = cudaGraphLaunch(ge, st);
-        const cudaError_t se = cudaStreamSynchronize(st);
-        cudaGraphExecDestroy(ge);
-        cudaGraphDestroy(g);
-        HJ_CUDA(le);
-        HJ_CUDA(se);
-    } else {
-        enqueue();
-    }
-    std::vector<uint32_t> ovf(n);
-    HJ_CUDA(cudaMemcpyAsync(rows.data(), d_rows, n * 8, cudaMemcpyDeviceToHost, st));
-    HJ_CUDA(cudaMemcpyAsync(sums.data(), d_sums, n * 8, cudaMemcpyDeviceToHost, st));
-    HJ_CUDA(cudaMemcpyAsync(ovf.data(), d_ovf, n * 4, cudaMemcpyDeviceToHost, st));
-    HJ_CUDA(cudaStreamSynchronize(st));
+    const Geometry        G = geometry(o);
+    std::vector<uint8_t>  plain(n, 0);
     std::vector<uint32_t> bad;
-    for (uint32_t i = 0; i < n; ++i)
-        if (ovf[i]) bad.push_back(i);
+    // Waves of instances whose tables stay within kWaveBytes, so that a large
+    // batch takes no more memory than the inputs' own size and a slot's number
+    // fits 32 bits.  An instance with more build rows than its partitions can
+    // hold goes to the plain path at once.
+    constexpr uint64_t kWaveBytes = 24ull << 30;
+    for (uint32_t i0 = 0; i0 < n;) {
+        uint64_t bytes = 0;
+        uint32_t i1    = i0;
+        for (; i1 < n; ++i1) {
+            const uint64_t nb = build_rows_of(B[i1]);
+            if (nb > (uint64_t(G.cap) << kMaxPartBits)) {
+                plain[i1] = 1;
+                bad.push_back(i1);
+                continue;
+            }
+            const uint64_t need = uint64_t(double(nb) * (G.buckets_per_row * (32 + 16 * (kMaxRel - 2)) + 8));
+            if (i1 > i0 && bytes + need > kWaveBytes) break;
+            bytes += need;
+        }
+        batch_wave(B, i0, i1, plain, o, G, graph, rows.data(), sums.data(), bad, st);
+        i0 = i1;
+    }
     return bad;
 }
 

@@ -378,6 +378,7 @@ struct hj_context {
     std::shared_ptr<hj::Store> store;  // resident tables (shared with cloned serving slots)
     int64_t             table_cache = 0;     // reuse tables built over resident base columns
     int64_t             fuse_filters = 0;    // evaluate a probe side's scan predicate inside the probe
+    hj::BatchGraph      batch_exec;          // the last batch's executable graph
 };
 
 struct hj_result {
@@ -1133,6 +1134,7 @@ void hj_context_destroy(hj_context* c) {
     if (c->staging) cudaFreeHost(c->staging);
     if (c->pinned) cudaFreeHost(c->pinned);
     c->pool.reset();
+    c->batch_exec.clear();
     if (c->st) cudaStreamDestroy(c->st);
     delete c;
 }
@@ -1540,8 +1542,9 @@ int hj_batch_execute(hj_context* c, const hj_batch_instance* inst, uint32_t n, i
         o.load       = double(c->batch_load_pct) / 100.0;
         o.graph      = c->batch_graph != 0;
         o.part_rows_log2 = int(c->batch_part_log2);
+        o.host_write     = c->ats_capable;
         std::vector<uint64_t> r, s;
-        const std::vector<uint32_t> redo = hj::batch_execute(B, o, r, s, c->st);
+        const std::vector<uint32_t> redo = hj::batch_execute(B, o, c->batch_exec, r, s, c->st);
         std::copy(r.begin(), r.end(), rows);
         std::copy(s.begin(), s.end(), checksums);
         for (uint32_t i : redo) plain(i);

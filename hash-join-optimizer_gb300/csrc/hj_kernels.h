@@ -188,14 +188,21 @@ struct BatchInstance {
     std::vector<BatchRelation> rels;
 };
 struct BatchOptions {
-    double load       = 0.5;   // build rows per bucket of a partition table (2^ceil(log2(rows / load)) buckets)
+    double load       = 0.5;   // build rows per bucket of a partition table (2^ceil(log2(rows / load)) buckets),
+                               // and per slot of the table that R0 is looked up in (within 0.25 .. 0.8)
     int    part_rows_log2 = 12;  // partitions of ~2^x build rows (x in 8..13); radix bits follow per instance
     bool   graph      = true;  // capture the whole batch in one CUDA graph
+    bool   host_write = false;  // the GPU writes pageable host memory (results come back without a copy engine)
+};
+// The executable graph of a context's last batch, updated in place by the next.
+struct BatchGraph {
+    cudaGraphExec_t exec = nullptr;
+    void            clear();
 };
 // Row count and checksum (sum of row fingerprints) per instance.  Returns the
 // instances with a partition too large for a shared-memory table (their rows /
 // sums are not valid; the caller recomputes them with plain_instance).
-std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& b, const BatchOptions& o,
+std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& b, const BatchOptions& o, BatchGraph& graph,
                                     std::vector<uint64_t>& rows, std::vector<uint64_t>& sums, cudaStream_t st);
 // One instance through the regular table build and two-pass probe.
 void plain_instance(const BatchInstance& b, const ProbeParams& prm, int dir_bits, int radix_bits, int dir_cap_bits,

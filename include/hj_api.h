@@ -277,11 +277,11 @@ int hj_table_probe_noalloc(hj_context* ctx, const hj_hash_table* t, const int32_
  * HBM without NULLs.  Per instance the call returns the result row count and a
  * checksum: the sum mod 2^64 over the result rows of a 64-bit fingerprint
  * folded over (key, payload of R0, ..., payload of Rm-1).
- *   mode HJ_BATCH_PERSISTENT: all relations of all instances radix-partitioned
- *     together on the key (partitions of ~2^batch_part_log2 build rows), then
- *     per (instance, partition) the build relations become shared-memory
- *     tables and R0's rows run through the whole chain -- persistent kernels
- *     over device-side work queues, the whole batch launched as one CUDA graph
+ *   mode HJ_BATCH_PERSISTENT: the build relations (all but R0) of all instances
+ *     radix-partitioned together on the key (partitions of ~2^batch_part_log2
+ *     build rows) and joined among themselves in shared memory, per (instance,
+ *     partition), into one hash table per instance; R0's rows are then looked
+ *     up in it -- persistent kernels, the whole batch launched as one CUDA graph
  *     (options batch_part_log2, batch_load_pct, batch_graph).  Instances with
  *     a partition too large for shared memory (heavy duplicate keys) are
  *     recomputed with the plain path; *recomputed (may be NULL) counts them.
