@@ -178,14 +178,6 @@ constexpr uint32_t kDup = 1u << 31;
 // instance is left to the plain path.
 constexpr uint64_t kFree = 0x8181818181818181ull;
 
-// Top 32 bits of fib_hash(k) in 32-bit arithmetic: with k sign-extended to 64
-// bits, hi32(k * C) = umulhi(k, C_lo) + k * C_hi - (k < 0 ? C_lo : 0) (mod 2^32).
-// Partition and bucket bits (at most 11 + 14) all come from these 32 bits.
-__device__ __forceinline__ uint32_t fib_hi(int32_t k) {
-    constexpr uint32_t CL = uint32_t(kFib), CH = uint32_t(kFib >> 32);
-    const uint32_t     kl = uint32_t(k);
-    return __umulhi(kl, CL) + kl * CH - (k < 0 ? CL : 0u);
-}
 __device__ __forceinline__ uint32_t part_of(int32_t k, uint32_t pbits) {
     return pbits ? fib_hi(k) >> (32 - pbits) : 0u;
 }

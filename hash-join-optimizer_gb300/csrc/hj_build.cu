@@ -617,16 +617,259 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// Small builds in one launch: every block owns one partition of the directory
+// and reads ALL keys, keeping those of its partition; the number of valid keys
+// in lower partitions, counted on the way, is where its tuples start, so no
+// histogram, offsets or scatter pass precedes it and nothing is cleared.  A
+// partition of at most kDirectMax tuples is listed in shared memory and counted
+// and placed from there; a larger one (a heavy key) reads the keys twice again.
+// Every block reads the keys from L2, so the cost grows with keys x partitions.
+constexpr int      kDT        = 1024;        // threads
+constexpr uint32_t kDirectMax = 20480;       // listed tuples of a partition
+constexpr int      kDU        = 8;           // keys per thread in flight
+
+__host__ __device__ constexpr size_t direct_smem(uint32_t L) {
+    return (size_t(1) << L) * 4 + (((size_t(1) << L) + 1) / 2) * 4 + (((size_t(1) << L) + 31) / 32) * 4 + 2 * size_t(kDirectMax) * 4;
+}
+
+__global__ void __launch_bounds__(kDT, 1)
+    k_build_direct(KeyCol kc, Geo g, uint64_t* __restrict__ dir, int32_t* okey,
+                   uint32_t* __restrict__ orow, uint32_t* __restrict__ mixed, uint64_t* __restrict__ summary) {
+    extern __shared__ uint32_t sh[];
+    __shared__ uint32_t wsum[kDT / 32], s_n, s_low;
+    const uint32_t nl = 1u << g.L, lmask = nl - 1, part = blockIdx.x;
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1;
+    const uint32_t nbw = (nl + 1) / 2, nmw = (nl + 31) / 32;
+    uint32_t* cnt = sh;             // nl: counts, then cursors
+    uint32_t* blm = sh + nl;        // nbw words: two 16-bit Bloom tags each
+    uint32_t* mix = sh + nl + nbw;  // nmw words of mixed bits
+    int32_t*  sk  = reinterpret_cast<int32_t*>(mix + nmw);  // kDirectMax listed keys
+    uint32_t* sr  = reinterpret_cast<uint32_t*>(sk + kDirectMax);  // and rows
+    const uint64_t gb = uint64_t(part) << g.L;
+    for (uint32_t i = threadIdx.x; i < nl + nbw + nmw; i += kDT) sh[i] = 0;
+    if (threadIdx.x == 0) s_n = s_low = 0;
+    __syncthreads();
+    const uint32_t n = uint32_t(kc.n);
+    // kDU keys of this thread from i0 on, and which of them are the partition's; lower partitions' are counted
+    uint32_t low  = 0;
+    auto     mine = [&](uint32_t i0, int32_t (&key)[kDU]) {
+        uint32_t ok = 0, in = 0;
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) ok |= uint32_t(load_key(kc, uint64_t(i0) + uint64_t(u) * kDT, key[u])) << u;
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) {
+            const uint32_t p    = g.R ? fib_hi(key[u]) >> (32 - g.R) : 0u;
+            const bool     some = (ok >> u) & 1u;
+            low += some && p < part;
+            in |= uint32_t(some && p == part) << u;
+        }
+        return in;
+    };
+    auto bucket = [&](int32_t k) { return uint32_t(bucket_of(fib_hash(k), g.b)) & lmask; };
+    // the Bloom tag of key k; a heavy key's is there already: a read, not an atomic on one word
+    auto tag = [&](int32_t k) {
+        const uint64_t h     = fib_hash(k);
+        const uint32_t local = uint32_t(bucket_of(h, g.b)) & lmask;
+        const uint32_t t     = bloom_mask(h) << (16 * (local & 1));
+        if ((*reinterpret_cast<volatile uint32_t*>(blm + (local >> 1)) & t) != t) atomicOr(blm + (local >> 1), t);
+    };
+    // Of a warp's keys `in`, the ones equal to its first (in an unlisted
+    // partition mostly the heavy key, counted by one atomic a warp): k0 and which they are.
+    auto heavy = [&](uint32_t in, const int32_t (&k)[kDU], int32_t& k0) {
+        const unsigned some = __ballot_sync(0xffffffffu, in != 0);
+        int32_t        f    = 0;
+#pragma unroll
+        for (int u = kDU - 1; u >= 0; --u)
+            if ((in >> u) & 1u) f = k[u];
+        k0 = __shfl_sync(0xffffffffu, f, some ? __ffs(some) - 1 : 0);
+        uint32_t eq = 0;
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) eq |= uint32_t(((in >> u) & 1u) && k[u] == k0) << u;
+        return eq;
+    };
+    for (uint32_t i0 = threadIdx.x; i0 - lane < n; i0 += kDT * kDU) {  // warp-uniform bound
+        int32_t        key[kDU];
+        const uint32_t in  = mine(i0, key);
+        // list slots step by step, so that neighbouring lanes store to neighbouring slots
+        uint32_t bal[kDU], tot = 0;
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) {
+            bal[u] = __ballot_sync(0xffffffffu, (in >> u) & 1u);
+            tot += __popc(bal[u]);
+        }
+        if (tot == 0) continue;
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(&s_n, tot);
+        q = __shfl_sync(0xffffffffu, q, 0);
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) {
+            const uint32_t at = q + __popc(bal[u] & lt);
+            if (((in >> u) & 1u) && at < kDirectMax) {
+                sk[at] = key[u];
+                sr[at] = i0 + uint32_t(u) * kDT;
+            }
+            q += __popc(bal[u]);
+        }
+    }
+    low = warp_sum(low);
+    if (lane == 0 && low) atomicAdd(&s_low, low);
+    __syncthreads();
+    const uint32_t s = s_low, m = s_n;  // the partition's first slot and tuples
+    const bool     listed = m <= kDirectMax;
+    if (listed) {
+        for (uint32_t q = threadIdx.x; q - lane < m; q += kDT) {
+            const bool     ok  = q < m;
+            const unsigned act = __ballot_sync(0xffffffffu, ok);
+            if (ok) {
+                bucket_add(cnt, bucket(sk[q]), act);
+                tag(sk[q]);
+            }
+        }
+    } else {
+        for (uint32_t i0 = threadIdx.x; i0 - lane < n; i0 += kDT * kDU) {
+            int32_t        k[kDU];
+            const uint32_t in = mine(i0, k);
+            int32_t        k0;
+            const uint32_t eq  = heavy(in, k, k0);
+            const uint32_t tot = warp_sum(uint32_t(__popc(eq)));
+            if (lane == 0 && tot) {
+                atomicAdd(cnt + bucket(k0), tot);
+                tag(k0);
+            }
+#pragma unroll
+            for (int u = 0; u < kDU; ++u)
+                if (((in & ~eq) >> u) & 1u) {
+                    atomicAdd(cnt + bucket(k[u]), 1u);
+                    tag(k[u]);
+                }
+        }
+    }
+    __syncthreads();
+    // exclusive scan of the counts: warp w scans segments of 32 counts
+    const uint32_t nseg = (nl + 31) / 32, per_w = (nseg + kDT / 32 - 1) / (kDT / 32);
+    uint32_t       wrun = 0;
+    for (uint32_t q = warp * per_w; q < min(nseg, (warp + 1) * per_w); ++q) {
+        const uint32_t i = 32 * q + lane;
+        wrun += warp_sum(i < nl ? cnt[i] : 0u);
+    }
+    if (lane == 0) wsum[warp] = wrun;
+    __syncthreads();
+    uint32_t base = s;
+    for (uint32_t w = 0; w < warp; ++w) base += wsum[w];
+    for (uint32_t q = warp * per_w; q < min(nseg, (warp + 1) * per_w); ++q) {
+        const uint32_t i   = 32 * q + lane;
+        const uint32_t c   = i < nl ? cnt[i] : 0u;
+        const uint32_t inc = warp_inclusive_scan(c);
+        if (i < nl) {
+            const uint32_t start = base + inc - c;
+            cnt[i]               = start;
+            dir[gb + i]          = (uint64_t(start) << 16) | ((blm[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+        }
+        base += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (gb + nl == (1ull << g.b) && threadIdx.x == 0) dir[gb + nl] = uint64_t(s + m) << 16;
+    __syncthreads();
+    if (listed) {
+        for (uint32_t q = threadIdx.x; q - lane < m; q += kDT) {
+            const bool     ok  = q < m;
+            const unsigned act = __ballot_sync(0xffffffffu, ok);
+            if (ok) {
+                const int32_t  k  = sk[q];
+                const uint32_t to = bucket_add(cnt, bucket(k), act);
+                okey[to]          = k;
+                orow[to]          = sr[q];
+            }
+        }
+    } else {
+        for (uint32_t i0 = threadIdx.x; i0 - lane < n; i0 += kDT * kDU) {
+            int32_t        k[kDU];
+            const uint32_t in = mine(i0, k);
+            int32_t        k0;
+            const uint32_t eq = heavy(in, k, k0);
+            uint32_t       bal[kDU], tot = 0, to = 0;
+#pragma unroll
+            for (int u = 0; u < kDU; ++u) {
+                bal[u] = __ballot_sync(0xffffffffu, (eq >> u) & 1u);
+                tot += __popc(bal[u]);
+            }
+            if (lane == 0 && tot) to = atomicAdd(cnt + bucket(k0), tot);
+            to = __shfl_sync(0xffffffffu, to, 0);
+#pragma unroll
+            for (int u = 0; u < kDU; ++u) {
+                if ((in >> u) & 1u) {
+                    const uint32_t at = (eq >> u) & 1u ? to + __popc(bal[u] & lt) : atomicAdd(cnt + bucket(k[u]), 1u);
+                    okey[at]          = k[u];
+                    orow[at]          = i0 + uint32_t(u) * kDT;
+                }
+                to += __popc(bal[u]);
+            }
+        }
+    }
+    __syncthreads();
+    // cnt[i] is now the end of bucket i.  A bucket is mixed when a tuple's key differs from its first tuple's.
+    const int32_t* ks = okey + s;  // (this block's own stores)
+    for (uint32_t q0 = threadIdx.x; q0 < m; q0 += kDT * kDU) {
+        int32_t  k[kDU], first[kDU];
+        uint32_t local[kDU];
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) k[u] = q0 + u * kDT < m ? ks[q0 + u * kDT] : 0;
+#pragma unroll
+        for (int u = 0; u < kDU; ++u) {
+            local[u] = bucket(k[u]);
+            first[u] = q0 + u * kDT < m ? ks[(local[u] == 0 ? s : cnt[local[u] - 1]) - s] : k[u];
+        }
+#pragma unroll
+        for (int u = 0; u < kDU; ++u)
+            if (first[u] != k[u]) atomicOr(mix + (local[u] >> 5), 1u << (local[u] & 31));
+    }
+    __syncthreads();
+    // the partition's buckets are whole mixed words (2^L >= 32), or all of the directory's
+    for (uint32_t i = threadIdx.x; i < nmw; i += kDT) mixed[(gb >> 5) + i] = mix[i];
+    for (uint32_t i = threadIdx.x; i < nl; i += kDT) {
+        const uint32_t b0  = i == 0 ? s : cnt[i - 1];
+        const uint32_t len = cnt[i] - b0;
+        summary[gb + i]    = len == 0 ? 0ull
+                                      : make_summary(ks[b0 - s], (blm[i >> 1] >> (16 * (i & 1))) & 0xffffu, len,
+                                                     (mix[i >> 5] >> (i & 31)) & 1u);
+    }
+}
+
 template <class K>
 void prefer_shared(K kernel) {
     HJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  int(cudaSharedmemCarveoutMaxShared)));
 }
 
+constexpr uint64_t kDirectKeys = 1u << 16;  // most keys of a one-launch build
+constexpr uint64_t kDirectPart = 2048;      // tuples of one of its partitions, about
+constexpr uint32_t kDirectBits = 13;        // bucket bits of one, at most
+
+void alloc_table(Table& t, uint32_t b, uint64_t nv, cudaStream_t st) {
+    const uint64_t nb = 1ull << b;
+    t.dir_bits        = b;
+    t.n_tuples        = nv;
+    t.dir             = dalloc_n<uint64_t>(nb + 1, st);
+    t.keys            = dalloc_n<int32_t>(nv, st);
+    t.rows            = dalloc_n<uint32_t>(nv, st);
+    t.mixed           = dalloc_n<uint32_t>((nb + 31) / 32, st);
+    t.summary         = dalloc_n<uint64_t>(nb, st);
+}
+
 uint32_t ceil_log2(uint64_t n) {
     uint32_t b = 0;
     while ((1ull << b) < n) ++b;
     return b;
+}
+
+template <class K>
+void max_dynamic_smem(K kernel, size_t bytes) {
+    HJ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+}
+
+// Shared memory of k_bucket_local for 2^L buckets.
+size_t local_smem(uint32_t L) {
+    const size_t nl = size_t(1) << L;
+    return (nl + (nl + 1) / 2 + (nl + 31) / 32 + 2 * size_t(kFuseMax)) * sizeof(uint32_t);
 }
 
 int grid_for(uint64_t work, int threads, int per_sm = 4) {
@@ -639,6 +882,34 @@ int grid_for(uint64_t work, int threads, int per_sm = 4) {
 void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint64_t* scratch_host,
                  cudaStream_t st, int64_t n_valid, int dir_cap_bits) {
     t = Table{};
+    // Small builds whose tuples are counted already: one launch.  A partition
+    // of about 2048 tuples a block, its buckets at most 2^kDirectBits, whole
+    // words of mixed bits.  hj_table_build with and without it, us: 1,000 keys
+    // 22 / 63, 16,000 28 / 76, 60,000 42 / 79 (device time 26 / 39), with Zipf
+    // keys 50 / 91, with one key only 94 / 103.  At 131,072 keys distinct ones
+    // still gain (60 / 80) but a heavy key's single block loses (170 / 104), so
+    // the line is at 2^16.
+    if (n_valid > 0 && uint64_t(n_valid) <= kDirectKeys && kc.n <= kDirectKeys && radix_bits < 0) {
+        const uint32_t b = dir_bits >= 0 ? uint32_t(dir_bits)
+                                         : std::min(uint32_t(std::max(0, dir_cap_bits)), ceil_log2(uint64_t(n_valid)));
+        uint32_t R = uint64_t(n_valid) > kDirectPart ? ceil_log2((uint64_t(n_valid) + kDirectPart - 1) / kDirectPart) : 0;
+        R          = std::max(R, b > kDirectBits ? b - kDirectBits : 0u);
+        if (b >= 5) R = std::min(R, b - 5);
+        else        R = 0;
+        if (b - R <= kDirectBits && (1u << R) <= uint32_t(num_sms()) && (uint64_t(n_valid) >> R) <= 2 * kDirectMax) {
+            const Geo g{b, R, b - R};
+            alloc_table(t, b, uint64_t(n_valid), st);
+            static OncePerDevice once;
+            once([&] {
+                HJ_CUDA(cudaFuncSetAttribute(k_build_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             int(direct_smem(kDirectBits))));
+                prefer_shared(k_build_direct);
+            });
+            k_build_direct<<<1u << R, kDT, direct_smem(g.L), st>>>(kc, g, t.dir, t.keys, t.rows, t.mixed, t.summary);
+            HJ_LAUNCH_CHECK();
+            return;
+        }
+    }
     const uint64_t n_upper = n_valid >= 0 ? uint64_t(n_valid) : kc.n;
     const uint32_t cap     = uint32_t(std::max(0, dir_cap_bits));
     const uint32_t b_upper = dir_bits >= 0 ? uint32_t(dir_bits)
@@ -650,12 +921,22 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
     R                      = std::min(R, b_upper);
     if (R > kMaxRadix) throw Error(HJ_ERR_INVALID, "build side too large for the radix partition");
 
-    prefer_shared(k_part_hist);
-    prefer_shared(k_part_scatter<1024>);
-    prefer_shared(k_part_scatter<kThreads>);
-    prefer_shared(k_bucket_count);
-    prefer_shared(k_bucket_scatter);
-    prefer_shared(k_bucket_local);
+    // dynamic shared memory up to the most that any geometry takes
+    static OncePerDevice once;
+    once([&] {
+        prefer_shared(k_part_hist);
+        prefer_shared(k_part_scatter<1024>);
+        prefer_shared(k_part_scatter<kThreads>);
+        prefer_shared(k_bucket_count);
+        prefer_shared(k_bucket_scatter);
+        prefer_shared(k_bucket_local);
+        max_dynamic_smem(k_part_hist, sizeof(uint32_t) << kMaxRadix);
+        max_dynamic_smem(k_part_scatter<1024>, 200 * 1024);
+        max_dynamic_smem(k_part_scatter<kThreads>, (8u << kMaxRadix) + size_t(kTile) * 10);
+        max_dynamic_smem(k_bucket_count, 8u << kLocalBits);
+        max_dynamic_smem(k_bucket_local, local_smem(kLocalBits));
+        max_dynamic_smem(k_bucket_scatter, 4u << kLocalBits);
+    });
     unsigned long long* d_nvalid = dalloc_n<unsigned long long>(1, st);
     uint32_t*           part_cnt = nullptr;
     auto run_hist = [&](uint32_t r) {
@@ -664,9 +945,6 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
         HJ_CUDA(cudaMemsetAsync(part_cnt, 0, P * sizeof(uint32_t), st));
         HJ_CUDA(cudaMemsetAsync(d_nvalid, 0, sizeof(unsigned long long), st));
         const size_t smem = P * sizeof(uint32_t);
-        if (smem > 48 * 1024)
-            HJ_CUDA(cudaFuncSetAttribute(k_part_hist, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem)));
         k_part_hist<<<grid_for(kc.n, kThreads), kThreads, smem, st>>>(kc, r, part_cnt, d_nvalid);
         HJ_LAUNCH_CHECK();
         if (n_valid < 0) {
@@ -709,25 +987,16 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
         auto smem_for = [&](size_t tile) { return (2 * size_t(P) + 2 * tile) * sizeof(uint32_t) + tile * sizeof(uint16_t); };
         const size_t big = smem_for(size_t(1024) * kItems);
         if (big <= 200 * 1024) {
-            HJ_CUDA(cudaFuncSetAttribute(k_part_scatter<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(big)));
             k_part_scatter<1024><<<div_up(kc.n, 1024 * kItems), 1024, big, st>>>(kc, R, part_cursor, tkey, trow);
         } else {
             const size_t smem = smem_for(kTile);
-            HJ_CUDA(cudaFuncSetAttribute(k_part_scatter<kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem)));
             k_part_scatter<kThreads><<<div_up(kc.n, kTile), kThreads, smem, st>>>(kc, R, part_cursor, tkey, trow);
         }
         HJ_LAUNCH_CHECK();
     }
 
     const uint64_t nb     = 1ull << b;
-    t.dir_bits            = b;
-    t.n_tuples            = nv;
-    t.dir                 = dalloc_n<uint64_t>(nb + 1, st);
-    t.keys                = dalloc_n<int32_t>(nv, st);
-    t.rows                = dalloc_n<uint32_t>(nv, st);
-    t.mixed               = dalloc_n<uint32_t>((nb + 31) / 32, st);
-    t.summary             = dalloc_n<uint64_t>(nb, st);
+    alloc_table(t, b, nv, st);
     uint32_t* gcnt        = dalloc_n<uint32_t>(nb, st);
     uint32_t* gbloom      = dalloc_n<uint32_t>(nb, st);
     HJ_CUDA(cudaMemsetAsync(t.mixed, 0, ((nb + 31) / 32) * sizeof(uint32_t), st));
@@ -736,17 +1005,13 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
 
     {
         const size_t smem = 2 * (size_t(1) << g.L) * sizeof(uint32_t);
-        HJ_CUDA(cudaFuncSetAttribute(k_bucket_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(smem)));
         k_bucket_count<<<chunks_upper, kThreads, smem, st>>>(g, chunk_off, chunk_part, part_off, tkey, gcnt, gbloom);
         HJ_LAUNCH_CHECK();
     }
     k_bucket_dir<<<P, 1024, 0, st>>>(g, part_off, gcnt, gbloom, t.dir);
     HJ_LAUNCH_CHECK();
     {
-        const size_t nl   = size_t(1) << g.L;
-        const size_t smem = (nl + (nl + 1) / 2 + (nl + 31) / 32 + 2 * size_t(kFuseMax)) * sizeof(uint32_t);
-        HJ_CUDA(cudaFuncSetAttribute(k_bucket_local, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        const size_t smem = local_smem(g.L);
         k_bucket_local<<<std::min<uint32_t>(P, uint32_t(num_sms())), kLT, smem, st>>>(g, part_off, tkey, trow, t.dir,
                                                                                 t.keys, t.rows, t.mixed,
                                                                                 t.summary);
@@ -754,8 +1019,6 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
     }
     {
         const size_t smem = (size_t(1) << g.L) * sizeof(uint32_t);
-        HJ_CUDA(cudaFuncSetAttribute(k_bucket_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     int(smem)));
         k_bucket_scatter<<<chunks_upper, kThreads, smem, st>>>(g, chunk_off, chunk_part, part_off, tkey, trow, gcnt,
                                                               t.keys, t.rows);
         HJ_LAUNCH_CHECK();

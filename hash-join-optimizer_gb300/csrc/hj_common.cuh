@@ -21,6 +21,28 @@ constexpr uint64_t kFib        = 11400714819323198485ull;  // 2^64 / golden rati
 // multiples of it.
 int num_sms();
 
+// Runs a kernel's one-time settings (attributes) once on each device, and
+// again after another context was created (the device may have been reset in
+// between).  A thread that finds them being made makes them too, which does no
+// harm.
+extern std::atomic<uint64_t> g_contexts_created;
+class OncePerDevice {
+public:
+    template <class F>
+    void operator()(F&& f) {
+        int            dev   = 0;
+        const uint64_t epoch = g_contexts_created.load(std::memory_order_acquire) + 1;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDev) dev = kDev;
+        if (dev < kDev && done_[dev].load(std::memory_order_acquire) == epoch) return;
+        f();
+        if (dev < kDev) done_[dev].store(epoch, std::memory_order_release);
+    }
+
+private:
+    static constexpr int  kDev = 64;
+    std::atomic<uint64_t> done_[kDev] = {};
+};
+
 // Engine error carrying an HJ_* status; converted to a return code at the C ABI.
 struct Error : std::runtime_error {
     int status;
@@ -49,6 +71,15 @@ extern std::atomic<uint64_t> g_kernel_launches;
 // UnchainedHash::hash_key (include/unchained.h:56-66 of the reference).
 __host__ __device__ __forceinline__ uint64_t fib_hash(int32_t key) {
     return uint64_t(int64_t(key)) * kFib;
+}
+
+// Top 32 bits of fib_hash(k) in 32-bit arithmetic: with k sign-extended to 64
+// bits, hi32(k * C) = umulhi(k, C_lo) + k * C_hi - (k < 0 ? C_lo : 0) (mod 2^32).
+// Partition bits (and the batch's bucket bits below them) come from these.
+__device__ __forceinline__ uint32_t fib_hi(int32_t k) {
+    constexpr uint32_t CL = uint32_t(kFib), CH = uint32_t(kFib >> 32);
+    const uint32_t     kl = uint32_t(k);
+    return __umulhi(kl, CL) + kl * CH - (k < 0 ? CL : 0u);
 }
 
 // Bucket (directory slot) of a hash: its top `bits` bits (0 bits -> slot 0).

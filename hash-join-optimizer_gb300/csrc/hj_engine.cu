@@ -39,6 +39,7 @@
 namespace hj {
 
 std::atomic<uint64_t> g_kernel_launches{0};
+std::atomic<uint64_t> g_contexts_created{0};
 
 int num_sms() {
     constexpr int           kMaxDev = 64;
@@ -1091,6 +1092,7 @@ hj_context* hj_context_create(int device) {
         return nullptr;
     }
     auto* c = new hj_context();
+    hj::g_contexts_created.fetch_add(1);
     try {
         if (device < 0) HJ_CUDA(cudaGetDevice(&device));
         if (device >= n) throw hj::Error(HJ_ERR_NO_DEVICE, "device index out of range");
