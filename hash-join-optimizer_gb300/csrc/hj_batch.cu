@@ -1335,10 +1335,20 @@ void plain_instance(const BatchInstance& b, const ProbeParams& prm, int dir_bits
         uint64_t   total = 0;
         uint32_t * pr = nullptr, *bw = nullptr;
         try {
-            total = probe_count(t, pk, prm, &pp, st);
-            pr    = static_cast<uint32_t*>(take(total * 4));
-            bw    = static_cast<uint32_t*>(take(total * 4));
-            const RidOut ro[2] = {{0, nullptr, pr}, {1, nullptr, bw}};
+            pr = static_cast<uint32_t*>(take(np * 4));  // one match a row, or more: below
+            bw = static_cast<uint32_t*>(take(np * 4));
+            RidOut ro[2] = {{0, nullptr, pr}, {1, nullptr, bw}};
+            total        = probe_count(t, pk, prm, ro, 2, &pp, st);
+            if (total > np) {
+                for (RidOut& o : ro) {
+                    uint32_t* more = static_cast<uint32_t*>(take(total * 4));
+                    if (const uint64_t d = probe_direct(pp))
+                        HJ_CUDA(cudaMemcpyAsync(more, o.dst, d * 4, cudaMemcpyDeviceToDevice, st));
+                    o.dst = more;
+                }
+                pr = ro[0].dst;
+                bw = ro[1].dst;
+            }
             if (total) probe_write(t, pk, pp, ro, 2, st);
         } catch (...) {
             if (pp) probe_free(pp, st);

@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kLT, 1)
             const uint32_t len = cnt[i] - b0;
             summary[gb + i]    = len == 0 ? 0ull
                                           : make_summary(sk[b0 - s], (blm[i >> 1] >> (16 * (i & 1))) & 0xffffu, len,
-                                                         (mix[i >> 5] >> (i & 31)) & 1u);
+                                                         (mix[i >> 5] >> (i & 31)) & 1u, sr[b0 - s]);
         }
         __syncthreads();
     }
@@ -569,8 +569,8 @@ __global__ void __launch_bounds__(kLT, 1)
 // come from k_bucket_local): one block per partition.
 __global__ void __launch_bounds__(256)
     k_bucket_summary(Geo g, const uint32_t* __restrict__ part_off, const uint64_t* __restrict__ dir,
-                     const int32_t* __restrict__ key, const uint32_t* __restrict__ mixed,
-                     uint64_t* __restrict__ summary) {
+                     const int32_t* __restrict__ key, const uint32_t* __restrict__ row,
+                     const uint32_t* __restrict__ mixed, uint64_t* __restrict__ summary) {
     const uint32_t part = blockIdx.x;
     if (fused_part(part_off, part)) return;
     const uint32_t nl = 1u << g.L;
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(256)
         const uint32_t len = uint32_t(__ldg(dir + p + 1) >> 16) - b0;
         summary[p] = len == 0 ? 0ull
                               : make_summary(__ldg(key + b0), uint32_t(d0) & 0xffffu, len,
-                                             (__ldg(mixed + (p >> 5)) >> (p & 31)) & 1u);
+                                             (__ldg(mixed + (p >> 5)) >> (p & 31)) & 1u, len == 1 ? __ldg(row + b0) : 0u);
     }
 }
 
@@ -634,7 +634,7 @@ __host__ __device__ constexpr size_t direct_smem(uint32_t L) {
 
 __global__ void __launch_bounds__(kDT, 1)
     k_build_direct(KeyCol kc, Geo g, uint64_t* __restrict__ dir, int32_t* okey,
-                   uint32_t* __restrict__ orow, uint32_t* __restrict__ mixed, uint64_t* __restrict__ summary) {
+                   uint32_t* orow, uint32_t* __restrict__ mixed, uint64_t* __restrict__ summary) {
     extern __shared__ uint32_t sh[];
     __shared__ uint32_t wsum[kDT / 32], s_n, s_low;
     const uint32_t nl = 1u << g.L, lmask = nl - 1, part = blockIdx.x;
@@ -830,7 +830,7 @@ __global__ void __launch_bounds__(kDT, 1)
         const uint32_t len = cnt[i] - b0;
         summary[gb + i]    = len == 0 ? 0ull
                                       : make_summary(ks[b0 - s], (blm[i >> 1] >> (16 * (i & 1))) & 0xffffu, len,
-                                                     (mix[i >> 5] >> (i & 31)) & 1u);
+                                                     (mix[i >> 5] >> (i & 31)) & 1u, len == 1 ? orow[b0] : 0u);
     }
 }
 
@@ -1025,7 +1025,7 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
     }
     k_bucket_mixed<<<chunks_upper, kThreads, 0, st>>>(g, chunk_off, chunk_part, part_off, t.dir, t.keys, t.mixed);
     HJ_LAUNCH_CHECK();
-    k_bucket_summary<<<P, 256, 0, st>>>(g, part_off, t.dir, t.keys, t.mixed, t.summary);
+    k_bucket_summary<<<P, 256, 0, st>>>(g, part_off, t.dir, t.keys, t.rows, t.mixed, t.summary);
     HJ_LAUNCH_CHECK();
 
     for (void* p : {(void*)d_nvalid, (void*)part_cnt, (void*)part_off, (void*)part_cursor,

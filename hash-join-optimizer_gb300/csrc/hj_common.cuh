@@ -99,20 +99,30 @@ __host__ __device__ __forceinline__ uint32_t bloom_mask(uint64_t h) {
 // directory itself keeps UnchainedHash's layout).  One 8-byte load gives the
 // probe everything a bucket of one key needs:
 //   bits  0..31  first key of the bucket's tuples (0 when empty)
-//   bits 32..47  the bucket's 16-bit Bloom tag (the directory word's low bits)
-//   bits 48..62  tuples in the bucket, saturated at kSumLenMax
 //   bit  63      the bucket holds more than one distinct key ("mixed")
-// An empty bucket's summary is 0.
-constexpr uint32_t kSumLenMax = 0x7fffu;
+//   bit  62      a bucket of one tuple ("single"): bits 32..61 are its build row
+//   else
+//   bits 32..47  the bucket's 16-bit Bloom tag (the directory word's low bits)
+//   bits 48..61  tuples in the bucket, saturated at kSumLenMax
+// An empty bucket's summary is 0.  One tuple whose row does not fit 30 bits is
+// an ordinary bucket of length 1.
+constexpr uint32_t kSumLenMax = 0x3fffu;
+constexpr uint64_t kSumSingle = 1ull << 62;
 
-__host__ __device__ __forceinline__ uint64_t make_summary(int32_t head, uint32_t bloom, uint32_t len, bool mixed) {
+__host__ __device__ __forceinline__ uint64_t make_summary(int32_t head, uint32_t bloom, uint32_t len, bool mixed,
+                                                          uint32_t first_row) {
+    if (len == 1 && (first_row >> 30) == 0) return uint64_t(uint32_t(head)) | (uint64_t(first_row) << 32) | kSumSingle;
     const uint64_t l = len < kSumLenMax ? len : kSumLenMax;
     return uint64_t(uint32_t(head)) | (uint64_t(bloom & 0xffffu) << 32) | (l << 48) | (uint64_t(mixed) << 63);
 }
 __host__ __device__ __forceinline__ int32_t  sum_head(uint64_t w) { return int32_t(uint32_t(w)); }
-__host__ __device__ __forceinline__ uint32_t sum_bloom(uint64_t w) { return uint32_t(w >> 32) & 0xffffu; }
-__host__ __device__ __forceinline__ uint32_t sum_len(uint64_t w) { return uint32_t(w >> 48) & kSumLenMax; }
 __host__ __device__ __forceinline__ bool     sum_mixed(uint64_t w) { return (w >> 63) != 0; }
+__host__ __device__ __forceinline__ bool     sum_single(uint64_t w) { return (w >> 62) == 1; }
+__host__ __device__ __forceinline__ uint32_t sum_row(uint64_t w) { return uint32_t(w >> 32) & 0x3fffffffu; }  // single
+__host__ __device__ __forceinline__ uint32_t sum_bloom(uint64_t w) { return uint32_t(w >> 32) & 0xffffu; }     // others
+__host__ __device__ __forceinline__ uint32_t sum_len(uint64_t w) {
+    return sum_single(w) ? 1u : uint32_t(w >> 48) & kSumLenMax;
+}
 
 __device__ __forceinline__ bool bit_valid(const uint32_t* bm, uint64_t i) {
     return bm == nullptr || ((__ldg(bm + (i >> 5)) >> (i & 31)) & 1u);

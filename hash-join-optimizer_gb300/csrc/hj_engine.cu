@@ -372,6 +372,7 @@ struct hj_context {
     int64_t             batch_graph    = 1;    // batched joins: launch as one CUDA graph
     int64_t             batch_part_log2 = 12;  // batched joins: ~2^x build rows per partition
     uint64_t*           pinned      = nullptr;  // small readbacks
+    uint64_t*           counters    = nullptr;  // probe counters on the device, zero between probes
     uint8_t*            staging     = nullptr;  // pinned transfer ring
     size_t              staging_bytes = 0;
     cudaEvent_t         slot_ev[2]  = {nullptr, nullptr};
@@ -866,25 +867,35 @@ struct Exec {
         table_tuples += t.n_tuples;
         if (t.n_tuples) dir_words += (uint64_t(1) << t.dir_bits) + 1;
         phase("probe");
-        ProbeParams prm;
-        prm.light_max = int(c->light_max);
-        prm.group     = int(c->probe_group);
-        prm.pinned    = c->pinned;
+        ProbeParams prm = context_probe_params(c);
         prm.after_count = [this] { phase("probe_sync"); };
         ProbePlan* pp = nullptr;
         uint64_t total = 0;
         try {
-            total = probe_count(t, pkc, prm, &pp, c->st);
+            // streams for one match a probe row, which the count pass fills as
+            // far as that is so; a larger result gets larger ones
+            std::vector<RidOut> ro;
+            std::vector<Buf>    dst;
+            for (auto [side, s] : need) {
+                Inter& side_in = side == 1 ? B : P;
+                dst.push_back(make_buf(std::max<uint64_t>(pkc.n, 1) * 4, c->st));
+                ro.push_back(RidOut{side, side_in.srcs[s].rid ? side_in.srcs[s].rid->as<uint32_t>() : nullptr,
+                                    dst.back()->as<uint32_t>()});
+            }
+            total = probe_count(t, pkc, prm, ro.data(), int(ro.size()), &pp, c->st);
             phase("probe_write");
             if (total > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
             out.rows = total;
-            std::vector<RidOut> ro;
-            for (auto [side, s] : need) {
-                Inter& side_in = side == 1 ? B : P;
-                Buf    dst     = make_buf(std::max<uint64_t>(total, 1) * 4, c->st);
-                ro.push_back(RidOut{side, side_in.srcs[s].rid ? side_in.srcs[s].rid->as<uint32_t>() : nullptr,
-                                    dst->as<uint32_t>()});
-                out.srcs.push_back(Source{side_in.srcs[s].table, dst});
+            for (size_t i = 0; i < ro.size(); ++i) {
+                if (total > pkc.n) {
+                    Buf            more = make_buf(total * 4, c->st);
+                    const uint64_t d    = probe_direct(pp);
+                    if (d) HJ_CUDA(cudaMemcpyAsync(more->p, dst[i]->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
+                    dst[i]    = more;
+                    ro[i].dst = more->as<uint32_t>();
+                }
+                const auto [side, s] = need[i];
+                out.srcs.push_back(Source{(side == 1 ? B : P).srcs[s].table, dst[i]});
             }
             if (total > 0) probe_write(t, pkc, pp, ro.data(), int(ro.size()), c->st);
         } catch (...) {
@@ -1042,6 +1053,7 @@ ProbeParams  context_probe_params(const hj_context* c) {
     p.light_max = int(c->light_max);
     p.group     = int(c->probe_group);
     p.pinned    = c->pinned;
+    p.counters  = c->counters;
     return p;
 }
 void         context_set_error(hj_context* c, const char* msg) { c->err = msg; }
@@ -1104,6 +1116,8 @@ hj_context* hj_context_create(int device) {
         uint64_t keep = ~0ull;  // keep freed blocks for reuse
         HJ_CUDA(cudaMemPoolSetAttribute(mp, cudaMemPoolAttrReleaseThreshold, &keep));
         HJ_CUDA(cudaMallocHost(&c->pinned, 64 * sizeof(uint64_t)));
+        HJ_CUDA(cudaMalloc(&c->counters, 8 * sizeof(uint64_t)));
+        HJ_CUDA(cudaMemsetAsync(c->counters, 0, 8 * sizeof(uint64_t), c->st));
         int pageable = 0;
         if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) != cudaSuccess) {
             cudaGetLastError();
@@ -1135,6 +1149,7 @@ void hj_context_destroy(hj_context* c) {
         if (e) cudaEventDestroy(e);
     if (c->staging) cudaFreeHost(c->staging);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->counters) cudaFree(c->counters);
     c->pool.reset();
     c->batch_exec.clear();
     if (c->st) cudaStreamDestroy(c->st);
@@ -1489,19 +1504,31 @@ int hj_table_probe(hj_context* c, const hj_hash_table* t, const int32_t* keys, c
         col.plain = keys;
         col.valid = valid;
         hj::KeyCol      pk{col, nullptr, n};
-        hj::ProbeParams prm;
-        prm.light_max = int(c->light_max);
-        prm.group     = int(c->probe_group);
-        prm.pinned    = c->pinned;
-        hj::ProbePlan* pp = nullptr;
+        const hj::ProbeParams prm = hj::context_probe_params(c);
+        hj::ProbePlan*        pp  = nullptr;
+        // nothing may be written before the matches are known to fit, so the
+        // directly written pairs go to buffers of the call's own
+        hj::Buf dp, db;
+        int     nout = 0;
+        if (out_probe && out_build && capacity && n) {
+            dp   = hj::make_buf(n * 4, c->st);
+            db   = hj::make_buf(n * 4, c->st);
+            nout = 2;
+        }
+        const hj::RidOut tmp[2] = {{0, nullptr, dp ? dp->as<uint32_t>() : nullptr},
+                                   {1, nullptr, db ? db->as<uint32_t>() : nullptr}};
         try {
-            const uint64_t total = hj::probe_count(t->t, pk, prm, &pp, c->st);
+            const uint64_t total = hj::probe_count(t->t, pk, prm, tmp, nout, &pp, c->st);
             *num_matches         = total;
             if (total > capacity) {
                 status = HJ_ERR_CAPACITY;
             } else if (total > 0) {
                 if (!out_probe || !out_build) throw hj::Error(HJ_ERR_INVALID, "null output buffer");
-                hj::RidOut ro[2] = {{0, nullptr, out_probe}, {1, nullptr, out_build}};
+                const hj::RidOut ro[2] = {{0, nullptr, out_probe}, {1, nullptr, out_build}};
+                if (const uint64_t d = hj::probe_direct(pp)) {
+                    HJ_CUDA(cudaMemcpyAsync(out_probe, dp->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
+                    HJ_CUDA(cudaMemcpyAsync(out_build, db->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
+                }
                 hj::probe_write(t->t, pk, pp, ro, 2, c->st);
             }
         } catch (...) {

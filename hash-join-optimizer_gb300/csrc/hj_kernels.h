@@ -120,17 +120,22 @@ struct ProbeParams {
     int       light_max = 32;       // larger buckets are not scanned by one thread
     int       group     = 8;        // threads per probe key in the write pass (1, 4, 8, 32)
     uint64_t* pinned    = nullptr;  // >= 8 words of pinned host memory for count readback
+    uint64_t* counters  = nullptr;  // 8 zeroed device words; zero again after each probe (probe_free)
     std::function<void()> after_count;  // called once the count kernels are enqueued
 };
 
 struct ProbePlan;  // opaque match list between the count and write passes
 
-// Count pass: returns the number of matches; keeps the hit list in *pp.
-uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, ProbePlan** pp,
-                     cudaStream_t st);
-// Write pass: emits the row-id streams for the matches found by probe_count
-// (all `nout` streams have probe_count() slots); the caller frees *pp with
-// probe_free afterwards.
+// Count pass: returns the number of matches; keeps the hit list in *pp.  With
+// outputs (streams of pk.n slots each), tiles of rows with at most one match
+// each are written at once: probe_direct() rows, the first of the result; the
+// list holds the others.
+uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, const RidOut* outs, int nout,
+                     ProbePlan** pp, cudaStream_t st);
+uint64_t probe_direct(const ProbePlan* pp);
+// Write pass: emits the listed matches' row ids after the directly written
+// ones (all `nout` streams have probe_count() slots; the direct rows are there
+// already); the caller frees *pp with probe_free afterwards.
 void probe_write(const Table& t, const KeyCol& pk, ProbePlan* pp, const RidOut* outs, int nout,
                  cudaStream_t st);
 void probe_free(ProbePlan* pp, cudaStream_t st);

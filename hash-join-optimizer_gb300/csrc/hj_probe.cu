@@ -86,9 +86,11 @@ struct Lists {
     uint32_t *m_row, *m_s, *m_e, *m_cnt;    // mixed hits: tuples [s, e) compared with m_key
     int32_t*  m_key;
     // 0 staged hits << 32 | staged matches mod 2^32, 1 mixed hits, 2 staged
-    // matches, 3 mixed matches, 4 staging waits that gave up (an error)
+    // matches, 3 mixed matches, 4 staging waits that gave up (an error),
+    // 5 rows written directly, 6 blocks that are done
     unsigned long long* ctr;
 };
+constexpr int kCtr = 8;  // counters
 
 struct Outs {
     int    n;
@@ -162,17 +164,24 @@ __device__ __forceinline__ bool tile_key(const KeyCol& pk, const uint8_t* stage,
     }
 }
 
+// Bucket of a key (directories have at most 26 bits).
+__device__ __forceinline__ uint32_t slot_of(const ProbeTab& T, int32_t key) {
+    return T.b ? fib_hi(key) >> (32 - T.b) : 0u;
+}
+
 template <int SRC>
 __global__ void __launch_bounds__(kPT, 4)
-    k_probe_count(ProbeTab T, KeyCol pk, int light_max, Lists Ls, uint64_t ntiles) {
+    k_probe_count(ProbeTab T, KeyCol pk, int light_max, Lists Ls, uint64_t ntiles, Outs outs,
+                  unsigned long long* host_ctr) {
     extern __shared__ __align__(128) uint8_t dyn[];
     constexpr uint32_t SB  = stage_bytes(SRC);
     constexpr int      kW  = kPT / 32;
     uint8_t*           stg = dyn;  // 2 stages
     __shared__ uint64_t bar[2];
     __shared__ uint32_t s_cov;
-    // per warp: staged hits and their matches (mod 2^32), turned into the
-    // warp's bases within the tile by thread 0; exact match counts
+    // per warp: hits (and kMany); for the list, matches (mod 2^32), turned into
+    // the warp's base within the tile by thread 0, and exact match counts
+    constexpr uint32_t            kMany = 1u << 31;  // the warp has a hit that only the list can hold
     __shared__ uint32_t           s_wh[kW], s_wc[kW];
     __shared__ unsigned long long s_wx[kW];
     __shared__ uint32_t           s_hb, s_ob;
@@ -226,54 +235,60 @@ __global__ void __launch_bounds__(kPT, 4)
             w[it]            = 0;
             if (i < nrows) ok[it] = tile_key<SRC>(pk, stage, cov, i, r0 + i, key[it]);
             // through L1: with skewed probe keys the hot buckets' summaries stay there
-            if (ok[it]) w[it] = __ldg(T.sum + bucket_of(fib_hash(key[it]), T.b));
+            if (ok[it]) w[it] = __ldg(T.sum + slot_of(T, key[it]));
         }
-        // classify: 0 miss, 1 hit staged here, 2 mixed bucket counted later.
-        // Directory words are read only for mixed buckets and for uniform
-        // buckets whose length saturated the summary's field.
+        // classify: a row is a miss, a hit staged here (bit `it` of hit), or in
+        // a mixed bucket counted later.  Directory words are read only for mixed
+        // buckets and for uniform buckets whose length saturated the summary's
+        // field.  s: the build row of a single tuple (bit of one), the first
+        // tuple of a bucket with a mask, else the bucket.
         uint32_t s[kStep], L[kStep], msk[kStep];
-        int      cls[kStep];
+        uint32_t hit = 0, one = 0, many = 0;  // many: hits that only the list can hold
 #pragma unroll
         for (int it = 0; it < kStep; ++it) {
-            const uint64_t h = fib_hash(key[it]);
-            L[it]            = sum_len(w[it]);
-            msk[it]          = 0;
-            cls[it]          = 0;
+            L[it]    = sum_len(w[it]);
+            msk[it]  = 0;
+            int  cls = 0;
             if (ok[it] && L[it] != 0) {
                 if (!sum_mixed(w[it])) {
                     // a bucket of one key: its first key decides exactly (a matching
                     // key's Bloom bits are always in the bucket's tag)
-                    cls[it] = sum_head(w[it]) == key[it] ? 1 : 0;
+                    cls = sum_head(w[it]) == key[it] ? 1 : 0;
                 } else {
-                    const uint32_t m = bloom_mask(h);
-                    cls[it]          = (sum_bloom(w[it]) & m) == m ? 2 : 0;
+                    const uint32_t m = bloom_mask(fib_hash(key[it]));
+                    cls              = (sum_bloom(w[it]) & m) == m ? 2 : 0;
                 }
             }
-            const uint64_t p = bucket_of(h, T.b);
-            s[it]            = uint32_t(p);
+            const uint32_t p = slot_of(T, key[it]);
+            s[it]            = p;
             uint32_t e       = 0;
-            if (cls[it] == 2 || (cls[it] == 1 && L[it] == kSumLenMax)) {
+            if (cls == 1 && sum_single(w[it])) {
+                s[it] = sum_row(w[it]);
+                one |= 1u << it;
+            } else if (cls == 2 || (cls == 1 && L[it] == kSumLenMax)) {
                 const uint32_t b0 = uint32_t(__ldg(T.dir + p) >> 16);
                 L[it]             = uint32_t(__ldg(T.dir + p + 1) >> 16) - b0;
-                if (cls[it] == 2) s[it] = b0;
+                if (cls == 2) s[it] = b0;
                 e = b0 + L[it];
             }
             // a small mixed bucket: compared here, its matches as a mask
-            if (cls[it] == 2 && L[it] <= small) {
+            if (cls == 2 && L[it] <= small) {
                 uint32_t mm = 0;
                 for (uint32_t q = 0; q < L[it]; ++q) mm |= uint32_t(__ldg(T.keys + s[it] + q) == key[it]) << q;
                 msk[it] = mm;
                 L[it]   = __popc(mm);
-                cls[it] = mm ? 1 : 0;
+                cls     = mm ? 1 : 0;
             }
+            hit |= uint32_t(cls == 1) << it;
+            many |= uint32_t(cls == 2 || (cls == 1 && L[it] != 1)) << it;
             // larger mixed buckets: counted later; rare, so warp-aggregated
             // global atomics
-            const unsigned bal = __ballot_sync(0xffffffffu, cls[it] == 2);
+            const unsigned bal = __ballot_sync(0xffffffffu, cls == 2);
             if (bal) {
                 unsigned long long q0 = 0;
                 if (lane == 0) q0 = atomicAdd(Ls.ctr + 1, (unsigned long long)__popc(bal));
                 q0 = __shfl_sync(0xffffffffu, q0, 0);
-                if (cls[it] == 2) {
+                if (cls == 2) {
                     const uint64_t q = q0 + __popc(bal & lt);
                     Ls.m_row[q]      = uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x);
                     Ls.m_s[q]        = s[it];
@@ -284,28 +299,66 @@ __global__ void __launch_bounds__(kPT, 4)
             }
         }
         // the warp's hits in (it, lane) order, so the hits of one round are
-        // consecutive list slots (coalesced stores): per round a ballot ranks
-        // them and a warp scan of their counts gives their first output rows
-        // within the warp -- a ballot suffices when no hit has more than one
-        // match (32-bit prefix sums; the exact total is summed beside them)
-        uint32_t           nh = 0, nc = 0;
+        // consecutive slots (coalesced stores): a ballot per round ranks them
+        uint32_t nh = 0, slot[kStep];
+#pragma unroll
+        for (int it = 0; it < kStep; ++it) {
+            const unsigned bal = __ballot_sync(0xffffffffu, (hit >> it) & 1u);
+            slot[it]           = nh + __popc(bal & lt);
+            nh += __popc(bal);
+        }
+        if (__any_sync(0xffffffffu, many) || outs.n == 0) nh |= kMany;
+        if (lane == 0) s_wh[warp] = nh;
+        __syncthreads();
+        uint32_t hw = 0, hs = 0, any = 0;  // hits of the warps before this one, and of all
+#pragma unroll
+        for (uint32_t q = 0; q < uint32_t(kW); ++q) {
+            const uint32_t h = s_wh[q];
+            any |= h;
+            hw += q < warp ? h & ~kMany : 0u;
+            hs += h & ~kMany;
+        }
+        if (!(any & kMany)) {
+            // one match a hit: its row ids straight to the output, which takes
+            // the place of a list entry, the list's passes and their launches
+            if (threadIdx.x == 0) s_ob = hs ? uint32_t(atomicAdd(Ls.ctr + 5, (unsigned long long)hs)) : 0u;
+#pragma unroll
+            for (int it = 0; it < kStep; ++it)
+                if (((hit & ~one) >> it) & 1u)
+                    s[it] = __ldg(T.rows + (msk[it] ? s[it] + uint32_t(__ffs(msk[it]) - 1)
+                                                    : uint32_t(__ldg(T.dir + s[it]) >> 16)));
+            __syncthreads();
+            const uint32_t ob = s_ob + hw;
+            for (int oi = 0; oi < outs.n; ++oi) {
+                const RidOut o = outs.o[oi];
+                if (o.src) {
+                    uint32_t v[kStep];
+#pragma unroll
+                    for (int it = 0; it < kStep; ++it)
+                        if ((hit >> it) & 1u)
+                            v[it] = __ldg(o.src + (o.side == 0 ? uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x) : s[it]));
+#pragma unroll
+                    for (int it = 0; it < kStep; ++it)
+                        if ((hit >> it) & 1u) o.dst[ob + slot[it]] = v[it];
+                } else {
+#pragma unroll
+                    for (int it = 0; it < kStep; ++it)
+                        if ((hit >> it) & 1u)
+                            o.dst[ob + slot[it]] = o.side == 0 ? uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x) : s[it];
+                }
+            }
+            continue;
+        }
+        // to the list: a warp scan of a round's counts gives their first output
+        // rows within the warp (32-bit prefix sums; the exact total is summed
+        // beside them)
+        uint32_t           nc = 0, oo[kStep];
         unsigned long long lx = 0;
-        uint32_t           slot[kStep], oo[kStep];
         static_assert(kStep % 2 == 0, "rounds are scanned in pairs");
 #pragma unroll
         for (int it = 0; it < kStep; it += 2) {
-            const bool     h0 = cls[it] == 1, h1 = cls[it + 1] == 1;
-            const uint32_t c0 = h0 ? L[it] : 0u, c1 = h1 ? L[it + 1] : 0u;
-            const unsigned b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
-            const uint32_t r0 = __popc(b0 & lt), r1 = __popc(b1 & lt);
-            slot[it]          = nh + r0;
-            slot[it + 1]      = nh + __popc(b0) + r1;
-            nh += __popc(b0) + __popc(b1);
-            if (!__any_sync(0xffffffffu, (c0 | c1) > 1)) {  // one match per hit: the ranks
-                oo[it]     = nc + r0;
-                oo[it + 1] = nc + __popc(b0) + r1;
-                nc += __popc(b0) + __popc(b1);
-            } else if (__all_sync(0xffffffffu, (c0 | c1) < 2048)) {
+            const uint32_t c0 = (hit >> it) & 1u ? L[it] : 0u, c1 = (hit >> (it + 1)) & 1u ? L[it + 1] : 0u;
+            if (__all_sync(0xffffffffu, (c0 | c1) < 2048)) {
                 // both rounds in one scan of 16-bit halves (a half sums to < 2^16)
                 const uint32_t v   = c0 | (c1 << 16);
                 const uint32_t inc = warp_inclusive_scan<uint32_t>(v);
@@ -326,20 +379,17 @@ __global__ void __launch_bounds__(kPT, 4)
         }
         const unsigned long long nx = warp_sum<unsigned long long>(lx);
         if (lane == 0) {
-            s_wh[warp] = nh;
             s_wc[warp] = nc;
             s_wx[warp] = nx;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
-            uint32_t           hs = 0, cs = 0;
+            uint32_t           cs = 0;
             unsigned long long xs = 0;
 #pragma unroll
             for (int q = 0; q < kW; ++q) {
-                const uint32_t h = s_wh[q], c = s_wc[q];
-                s_wh[q] = hs;
+                const uint32_t c = s_wc[q];
                 s_wc[q] = cs;
-                hs += h;
                 cs += c;
                 xs += s_wx[q];
             }
@@ -349,13 +399,13 @@ __global__ void __launch_bounds__(kPT, 4)
             s_ob = uint32_t(base);
         }
         __syncthreads();
-        const uint32_t hb = s_hb + s_wh[warp], ob = s_ob + s_wc[warp];
+        const uint32_t hb = s_hb + hw, ob = s_ob + s_wc[warp];
 #pragma unroll
         for (int it = 0; it < kStep; ++it) {
-            if (cls[it] == 1) {
+            if ((hit >> it) & 1u) {
                 const uint32_t q = hb + slot[it];
                 Ls.u_row[q]      = uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x);
-                Ls.u_sp[q]       = s[it];
+                Ls.u_sp[q]       = (one >> it) & 1u ? slot_of(T, key[it]) : s[it];
                 Ls.u_off[q]      = ob + oo[it];
                 Ls.u_mask[q]     = msk[it];
             }
@@ -368,6 +418,20 @@ __global__ void __launch_bounds__(kPT, 4)
             atomicAdd(Ls.ctr + 4, 1ull);
             if (iss0) mbar_wait_bounded(&bar[0], (iss0 - 1) & 1, kWaitPolls);
             if (iss1) mbar_wait_bounded(&bar[1], (iss1 - 1) & 1, kWaitPolls);
+        }
+    }
+    // the block that is done last hands the counters to the host and clears
+    // them for the next probe (not the mixed hits, which are still to be counted)
+    if (host_ctr && threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(Ls.ctr + 6, 1ull) == gridDim.x - 1) {
+            __threadfence();
+            for (int q = 0; q < 6; ++q) {
+                const unsigned long long v = atomicAdd(Ls.ctr + q, 0ull);
+                host_ctr[q]                = v;
+                if (q != 1) Ls.ctr[q] = 0;
+            }
+            Ls.ctr[6] = 0;
         }
     }
 }
@@ -654,28 +718,39 @@ int key_source(const KeyCol& pk) {
 }
 
 template <int SRC>
-void launch_count_src(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, cudaStream_t st) {
+void launch_count_src(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, const Outs& outs,
+                      uint64_t* host_ctr, cudaStream_t st) {
     const uint64_t ntiles = (pk.n + kTileRows - 1) / kTileRows;
     const size_t   smem   = std::max<size_t>(16, 2 * size_t(stage_bytes(SRC)));
-    HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     // shared memory for the resident blocks only; the rest of the unified
     // L1 / shared memory caches bucket summaries
-    HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 30));
+    static OncePerDevice    once;
+    static std::atomic<int> resident{0};
+    once([&] {
+        int n = 0;
+        HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 30));
+        HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_probe_count<SRC>, kPT, smem));
+        resident.store(n);
+    });
     // resident blocks walk the tiles (each prefetching its next tile)
-    int per_sm = 0;
-    HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_probe_count<SRC>, kPT, smem));
+    const int per_sm = resident.load();
     const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(num_sms()) * std::max(1, per_sm)));
-    k_probe_count<SRC><<<unsigned(grid), kPT, smem, st>>>(T, pk, light_max, L, ntiles);
+    k_probe_count<SRC><<<unsigned(grid), kPT, smem, st>>>(T, pk, light_max, L, ntiles, outs,
+                                                          reinterpret_cast<unsigned long long*>(host_ctr));
     HJ_LAUNCH_CHECK();
 }
 
-// Count kernels over a probe column: uniform and mixed lists, counters in L.ctr.
-void launch_count(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, cudaStream_t st) {
+// Count kernels over a probe column: uniform and mixed lists, counters in
+// L.ctr; with outs, tiles of single matches straight to the output (pk.n rows
+// each); with host_ctr, the counters to the host and cleared.
+void launch_count(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, const Outs& outs,
+                  uint64_t* host_ctr, cudaStream_t st) {
     switch (key_source(pk)) {
-    case kSrcPages: launch_count_src<kSrcPages>(T, pk, light_max, L, st); break;
-    case kSrcPlain: launch_count_src<kSrcPlain>(T, pk, light_max, L, st); break;
-    case kSrcTagged: launch_count_src<kSrcTagged>(T, pk, light_max, L, st); break;
-    default: launch_count_src<kSrcGather>(T, pk, light_max, L, st); break;
+    case kSrcPages: launch_count_src<kSrcPages>(T, pk, light_max, L, outs, host_ctr, st); break;
+    case kSrcPlain: launch_count_src<kSrcPlain>(T, pk, light_max, L, outs, host_ctr, st); break;
+    case kSrcTagged: launch_count_src<kSrcTagged>(T, pk, light_max, L, outs, host_ctr, st); break;
+    default: launch_count_src<kSrcGather>(T, pk, light_max, L, outs, host_ctr, st); break;
     }
 }
 
@@ -708,9 +783,15 @@ template <int G>
 void launch_uniform_g(const ProbeTab& T, const Lists& L, uint64_t n_u, const uint32_t* chunk_first, uint64_t total,
                       const Outs& outs, cudaStream_t st) {
     const size_t smem = write_uniform_smem(G);
-    HJ_CUDA(cudaFuncSetAttribute(k_write_uniform<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int per_sm = 0;
-    HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_write_uniform<G>, 256, smem));
+    static OncePerDevice    once;
+    static std::atomic<int> resident{0};
+    once([&] {
+        int n = 0;
+        HJ_CUDA(cudaFuncSetAttribute(k_write_uniform<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_write_uniform<G>, 256, smem));
+        resident.store(n);
+    });
+    const int per_sm = resident.load();
     const uint64_t nchunks = (total + warp_chunk(G) - 1) / warp_chunk(G);
     const uint64_t grid    = std::max<uint64_t>(1, std::min<uint64_t>((nchunks + 7) / 8, uint64_t(num_sms()) * std::max(1, per_sm)));
     k_write_uniform<G><<<unsigned(grid), 256, smem, st>>>(T, L, n_u, chunk_first, total, outs);
@@ -748,21 +829,20 @@ void check_staging(const uint64_t* host_ctr) {
 
 struct ProbePlan {
     Lists     ls{};
-    uint64_t  cap     = 0;
-    uint64_t  n_u = 0, n_m = 0, tot_u = 0, tot_m = 0;
+    uint64_t  n_u = 0, n_m = 0, tot_u = 0, tot_m = 0, tot_d = 0;
     uint64_t* host    = nullptr;  // pinned readback of the counters (owned by the caller)
     int       group   = 8;
 };
 
-uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, ProbePlan** out,
-                     cudaStream_t st) {
+uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, const RidOut* ro, int nout,
+                     ProbePlan** out, cudaStream_t st) {
+    if (nout > kMaxRidOut) throw Error(HJ_ERR_INVALID, "too many output row-id streams");
     auto* pp  = new ProbePlan();
     *out      = pp;
     pp->group = prm.group;
     if (t.n_tuples == 0 || pk.n == 0) return 0;
     if (pk.n > 0xffffffffull) throw Error(HJ_ERR_INVALID, "more than 2^32 probe rows");
     const uint64_t n = pk.n;
-    pp->cap          = n;
     Lists& L         = pp->ls;
     L.u_row = dalloc_n<uint32_t>(n, st);
     L.u_sp  = dalloc_n<uint32_t>(n, st);
@@ -773,30 +853,37 @@ uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, P
     L.m_e   = dalloc_n<uint32_t>(n, st);
     L.m_cnt = dalloc_n<uint32_t>(n, st);
     L.m_key = dalloc_n<int32_t>(n, st);
-    L.ctr   = dalloc_n<unsigned long long>(8, st);
-    HJ_CUDA(cudaMemsetAsync(L.ctr, 0, 8 * sizeof(unsigned long long), st));
-    launch_count(tab_of(t), pk, prm.light_max, L, st);
-    if (prm.after_count) prm.after_count();
+    L.ctr   = reinterpret_cast<unsigned long long*>(prm.counters);
+    Outs outs{};
+    outs.n = nout;
+    for (int i = 0; i < nout; ++i) outs.o[i] = ro[i];
     pp->host = prm.pinned;
-    readback(pp->host, L.ctr, 5 * sizeof(uint64_t), true, st);  // page-locked scratch
+    launch_count(tab_of(t), pk, prm.light_max, L, outs, pp->host, st);
+    if (prm.after_count) prm.after_count();
     HJ_CUDA(cudaStreamSynchronize(st));
+    pp->n_m = pp->host[1];  // probe_free clears their counters
     check_staging(pp->host);
     count_mixed(tab_of(t), L, pp->host, st);
     pp->n_u   = pp->host[0] >> 32;
-    pp->n_m   = pp->host[1];
     pp->tot_u = pp->host[2];
     pp->tot_m = pp->host[3];
-    return pp->tot_u + pp->tot_m;
+    pp->tot_d = pp->host[5];
+    return pp->tot_d + pp->tot_u + pp->tot_m;
 }
+
+uint64_t probe_direct(const ProbePlan* pp) { return pp->tot_d; }
 
 void probe_write(const Table& t, const KeyCol& pk, ProbePlan* pp, const RidOut* ro, int nout,
                  cudaStream_t st) {
     (void)pk;
     if (nout > kMaxRidOut) throw Error(HJ_ERR_INVALID, "too many output row-id streams");
+    if (nout == 0) return;
     Outs outs{};
     outs.n = nout;
-    for (int i = 0; i < nout; ++i) outs.o[i] = ro[i];
-    if (pp->cap == 0 || nout == 0) return;
+    for (int i = 0; i < nout; ++i) {
+        outs.o[i] = ro[i];
+        outs.o[i].dst += pp->tot_d;  // the directly written rows come first
+    }
     const ProbeTab T = tab_of(t);
     Lists&         L = pp->ls;
     if (pp->n_u) {
@@ -849,7 +936,7 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
     Lists     L{};
     uint64_t *m_off, *tmp;
     Carve     c{scratch};
-    L.ctr   = c.take<unsigned long long>(8);
+    L.ctr   = c.take<unsigned long long>(kCtr);
     L.u_row = c.take<uint32_t>(n);
     L.u_sp  = c.take<uint32_t>(n);
     L.u_off = c.take<uint32_t>(n);
@@ -864,7 +951,7 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
     // the scratch keeps the previous call's contents: the counters restart at zero
     HJ_CUDA(cudaMemsetAsync(L.ctr, 0, 8 * sizeof(unsigned long long), st));
     const ProbeTab T = tab_of(t);
-    launch_count(T, pk, prm.light_max, L, st);
+    launch_count(T, pk, prm.light_max, L, Outs{}, nullptr, st);
     uint64_t* h = prm.pinned;
     readback(h, L.ctr, 5 * sizeof(uint64_t), true, st);  // page-locked scratch
     HJ_CUDA(cudaStreamSynchronize(st));
@@ -893,8 +980,9 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
 void probe_free(ProbePlan* pp, cudaStream_t st) {
     if (!pp) return;
     Lists& L = pp->ls;
+    if (pp->n_m) cudaMemsetAsync(L.ctr, 0, kCtr * sizeof(unsigned long long), st);
     for (void* p : {(void*)L.u_row, (void*)L.u_sp, (void*)L.u_off, (void*)L.u_mask, (void*)L.m_row, (void*)L.m_s, (void*)L.m_e,
-                    (void*)L.m_cnt, (void*)L.m_key, (void*)L.ctr})
+                    (void*)L.m_cnt, (void*)L.m_key})
         if (p) dfree(p, st);
     delete pp;
 }
