@@ -872,13 +872,15 @@ struct Exec {
         ProbePlan* pp = nullptr;
         uint64_t total = 0;
         try {
-            // streams for one match a probe row, which the count pass fills as
-            // far as that is so; a larger result gets larger ones
+            // streams for one match a probe row and some slack for keys with
+            // several, which the count pass fills as far as matches are single;
+            // a result beyond them gets larger ones (its direct rows copied)
+            const uint64_t      cap = pkc.n + std::min<uint64_t>(3 * pkc.n, 16u << 20);
             std::vector<RidOut> ro;
             std::vector<Buf>    dst;
             for (auto [side, s] : need) {
                 Inter& side_in = side == 1 ? B : P;
-                dst.push_back(make_buf(std::max<uint64_t>(pkc.n, 1) * 4, c->st));
+                dst.push_back(make_buf(std::max<uint64_t>(cap, 1) * 4, c->st));
                 ro.push_back(RidOut{side, side_in.srcs[s].rid ? side_in.srcs[s].rid->as<uint32_t>() : nullptr,
                                     dst.back()->as<uint32_t>()});
             }
@@ -887,7 +889,7 @@ struct Exec {
             if (total > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
             out.rows = total;
             for (size_t i = 0; i < ro.size(); ++i) {
-                if (total > pkc.n) {
+                if (total > cap) {
                     Buf            more = make_buf(total * 4, c->st);
                     const uint64_t d    = probe_direct(pp);
                     if (d) HJ_CUDA(cudaMemcpyAsync(more->p, dst[i]->p, d * 4, cudaMemcpyDeviceToDevice, c->st));

@@ -4,7 +4,7 @@
 // The reference applies a scan's Comparison while loading the table and
 // hands execute() only the passing rows, in order (src/build_table.cpp:
 // 321-370).  Here the passing rows become the scan's row ids.  (With option
-// fuse_filters a filtered probe side skips this and k_probe_count, in
+// fuse_filters a filtered probe side skips this and the probe's count pass, in
 // hj_probe.cu, evaluates the predicate on the raw rows instead.)
 //
 // Two passes over 4096-row tiles (8 warps x 16 steps x 32 rows):

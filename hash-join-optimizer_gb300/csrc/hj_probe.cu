@@ -6,33 +6,25 @@
 // Bloom early-reject on the bucket's tag, then every tuple of the bucket with
 // an equal key is a match.
 //
-// Count pass (k_probe_count).  A block walks tiles of 1984 probe rows (one
-// dense INT32 page).  The tile's keys are staged in shared memory by bulk
-// asynchronous copies (TMA) while the previous tile is probed: whole pages
-// for a dense column read in place, else the decoded int32 / value_t array.
-// Per key the probe issues ONE global load, the bucket's 8-byte summary
-// (first key, Bloom tag, length, mixed flag; hj_common.cuh), eight keys per
-// thread in flight:
+// Count pass, k_probe_tile for one tile of 1984 probe rows (one dense INT32
+// page), whose matches keep their order, and k_probe_stream for more.  Per key
+// the probe issues ONE global load, the bucket's 8-byte summary (first key, and
+// the tuple's build row or Bloom tag, length and mixed flag; hj_common.cuh):
 //   miss     empty bucket, or the Bloom tag rejects the key;
+//   single   bucket of one tuple: its key decides, its build row is there;
 //   uniform  bucket of one key (mixed flag clear): the key matches every tuple
 //            of the bucket or none, decided by the first key; the hit is
 //            (probe row, bucket, length from the summary) -- no further load;
-//   mixed    bucket of several keys: a bucket of at most min(light_max, 32)
-//            tuples is compared by the probing thread itself, which records
-//            the matching tuples as a 32-bit mask over the bucket and stages
-//            the hit with the uniform ones; larger buckets go to a list
-//            counted by a warp or block per hit (k_mixed_count*).
-// A hit stays in the registers of the thread that found it.  Within a warp,
-// hits are ordered round by round (the eight keys of a thread are eight
-// rounds), so a ballot ranks a round's hits into consecutive list slots
-// (coalesced stores) and a warp scan of their match counts gives their first
-// output rows.  The kernel keeps its shared memory small (the two key
-// stages): the rest of the SM's 256 KB stays L1, where the summaries of
-// frequently probed buckets are cached.  Per tile,
-// ONE global 64-bit atomic reserves both the block's list slots (high word)
-// and its output rows (low word), so list order and output order agree and no
+//   mixed    bucket of several keys: the tuples of a bucket of at most
+//            min(light_max, 31) are compared and the matching ones noted as a
+//            mask over the bucket (one match: as its build row); larger buckets
+//            go to a list counted by a warp or block per hit (k_mixed_count*).
+// A match that is the only one of its probe row is written at once, its row
+// ids straight to the output.  Other hits go to a list with their first output
+// rows: ONE global 64-bit atomic a flush reserves both list slots (high word)
+// and output rows (low word), so list order and output order agree and no
 // device-wide prefix sum is needed (the reference's per-thread work-stealing
-// counter becomes this per-block reservation).
+// counter becomes this reservation).  The listed matches follow the direct ones.
 //
 // Write pass.  k_write_uniform walks the OUTPUT positions in chunks of
 // 32 x G per warp (G outputs per thread, option probe_group): a chunk's hits
@@ -47,25 +39,35 @@
 // requested output stream, composed through the sides' row-id vectors (late
 // materialisation).
 #include <algorithm>
+#include <type_traits>
 
 #include "hj_block.cuh"
 #include "hj_common.cuh"
 #include "hj_kernels.h"
-#include "hj_tma.cuh"
 
 namespace hj {
 
 namespace {
 
-constexpr int      kPT        = 256;                    // threads of the count kernel
-constexpr int      kStep      = 8;                      // rows per thread in flight
-constexpr uint32_t kTileRows  = uint32_t(kDenseRows);   // 1984 rows per staged tile (one page)
-static_assert(kTileRows <= uint32_t(kPT) * kStep, "a tile is one pass of the count kernel");
-static_assert(kPT * kStep == 2048 && kPT == 256, "the staged-hit scan covers 8 warps x 8 rows of 32");
+constexpr int      kPT        = 256;                    // threads of the stream kernel
+constexpr uint32_t kTileRows  = uint32_t(kDenseRows);   // 1984 rows per tile (one page)
 constexpr uint32_t kUncounted = 0xffffffffu;            // mixed hit still to be counted
 constexpr uint32_t kMixedWarpMax = 4096;                // mixed buckets up to this size: one warp each
-constexpr uint32_t kWaitPolls    = 1u << 20;            // bound of a staging wait (mbarrier polls)
 
+// L2 cache policy (createpolicy) for stores of lines written once and read
+// back later in order (output row ids): they leave L2 first.
+__device__ __forceinline__ uint64_t l2_evict_first() {
+    uint64_t p;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
+// 16-byte stores with an L2 cache policy.
+__device__ __forceinline__ void st_hint(uint4* p, uint4 v, uint64_t policy) {
+    asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
+                 "r"(v.w), "l"(policy)
+                 : "memory");
+}
 __host__ __device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
 enum KeySrc : int { kSrcPages = 0, kSrcPlain = 1, kSrcTagged = 2, kSrcGather = 3 };
@@ -75,22 +77,22 @@ struct ProbeTab {
     const uint64_t* sum;
     const int32_t*  keys;
     const uint32_t* rows;
-    uint32_t        b;
+    uint32_t        nb;  // buckets, a power of two
 };
 
 struct Lists {
     // staged hits, in output order: hit h owns output rows [off[h], off[h + 1])
     // (the last up to the staged total); mask 0: the whole bucket sp matches,
-    // else the tuples sp + i for the set bits i of mask
+    // kRowHit: build row sp, else the tuples sp + i for the set bits i of mask
     uint32_t *u_row, *u_sp, *u_off, *u_mask;
     uint32_t *m_row, *m_s, *m_e, *m_cnt;    // mixed hits: tuples [s, e) compared with m_key
     int32_t*  m_key;
     // 0 staged hits << 32 | staged matches mod 2^32, 1 mixed hits, 2 staged
-    // matches, 3 mixed matches, 4 staging waits that gave up (an error),
-    // 5 rows written directly, 6 blocks that are done
+    // matches, 3 mixed matches, 5 rows written directly, 6 blocks that are done
     unsigned long long* ctr;
 };
-constexpr int kCtr = 8;  // counters
+constexpr int      kCtr    = 8;            // counters
+constexpr uint32_t kRowHit = 0xffffffffu;  // no mask of a mixed bucket: one of its tuples differs
 
 struct Outs {
     int    n;
@@ -106,53 +108,20 @@ __device__ __forceinline__ void emit(const Outs& outs, uint64_t pos, uint32_t pr
     }
 }
 
-// Bytes of one staged tile of each key source (0: no staging).
-__host__ __device__ constexpr uint32_t stage_bytes(int src) {
-    return src == kSrcPages    ? uint32_t(kPage)
-         : src == kSrcPlain    ? kTileRows * 4u
-         : src == kSrcTagged   ? kTileRows * 8u
-                               : 0u;
-}
-
-// Issues the bulk copy of tile `tile` of the key column into `dst`; returns
-// the rows of the tile that the copy covers (the rest are read directly).
+// Key of row i of tile `tile`; false for NULL and past the end.
 template <int SRC>
-__device__ __forceinline__ uint32_t stage_tile(const KeyCol& pk, uint64_t tile, uint8_t* dst, uint64_t* bar) {
-    const uint64_t r0    = tile * kTileRows;
-    const uint32_t nrows = uint32_t(umin64(kTileRows, pk.n - r0));
-    uint32_t       bytes = 0, covered = 0;
-    const void*    src   = nullptr;
+__device__ __forceinline__ bool tile_key(const KeyCol& pk, uint64_t tile, uint32_t i, int32_t& key) {
+    const uint64_t r = tile * kTileRows + i;
+    key              = 0;
+    if (i >= kTileRows || r >= pk.n) return false;
     if (SRC == kSrcPages) {
-        bytes   = kPage;
-        src     = pk.col.pages + tile * kPage;
-        covered = nrows;
-    } else if (SRC == kSrcPlain) {
-        covered = nrows & ~3u;
-        bytes   = covered * 4u;
-        src     = pk.col.plain + r0;
-    } else {
-        covered = nrows & ~1u;
-        bytes   = covered * 8u;
-        src     = pk.col.tagged + r0;
-    }
-    fence_proxy_async_smem();
-    mbar_arrive_expect(bar, bytes);
-    if (bytes) bulk_load(dst, src, bytes, bar);
-    return covered;
-}
-
-// Key of tile row i (row r of the key column); false for NULL.
-template <int SRC>
-__device__ __forceinline__ bool tile_key(const KeyCol& pk, const uint8_t* stage, uint32_t covered, uint32_t i,
-                                         uint64_t r, int32_t& key) {
-    if (SRC == kSrcPages) {
-        key = reinterpret_cast<const int32_t*>(stage + 4)[i];
+        key = __ldcs(reinterpret_cast<const int32_t*>(pk.col.pages + tile * kPage + 4) + i);
         return true;
     } else if (SRC == kSrcPlain) {
-        key = i < covered ? reinterpret_cast<const int32_t*>(stage)[i] : __ldg(pk.col.plain + r);
+        key = __ldcs(pk.col.plain + r);
         return bit_valid(pk.col.valid, r);
     } else if (SRC == kSrcTagged) {
-        const uint64_t t = i < covered ? reinterpret_cast<const uint64_t*>(stage)[i] : __ldg(pk.col.tagged + r);
+        const uint64_t t = __ldcs(pk.col.tagged + r);
         key              = int32_t(uint32_t(t));
         return (t >> 62) == 1;
     } else {
@@ -165,275 +134,364 @@ __device__ __forceinline__ bool tile_key(const KeyCol& pk, const uint8_t* stage,
 }
 
 // Bucket of a key (directories have at most 26 bits).
-__device__ __forceinline__ uint32_t slot_of(const ProbeTab& T, int32_t key) {
-    return T.b ? fib_hi(key) >> (32 - T.b) : 0u;
+__device__ __forceinline__ uint32_t slot_of(const ProbeTab& T, int32_t key) { return __umulhi(fib_hi(key), T.nb); }
+
+// The block that is done last hands the counters to the host and clears them
+// for the next probe (not the mixed hits, which are still to be counted).
+// Called by every thread after the block's last update of the counters.
+__device__ __forceinline__ void hand_over(const Lists& Ls, unsigned long long* host_ctr) {
+    if (!host_ctr || threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(Ls.ctr + 6, 1ull) != gridDim.x - 1) return;
+    __threadfence();
+    for (int q = 0; q < 6; ++q) {
+        host_ctr[q] = atomicAdd(Ls.ctr + q, 0ull);
+        if (q != 1) Ls.ctr[q] = 0;
+    }
+    Ls.ctr[6] = 0;
 }
+
+// Tuples of bucket p that equal key k, as a mask over the bucket, for a small
+// mixed bucket with the high summary word hi; b0: its first tuple, row: the
+// build row of a single match.
+__device__ __forceinline__ uint32_t compare_mixed(const ProbeTab& T, int32_t k, uint32_t hi, uint32_t& b0, uint32_t& row) {
+    const uint32_t bm = bloom_mask(fib_hash(k)), len = (hi >> 16) & kSumLenMax;
+    uint32_t       mm = 0;
+    b0 = row = 0;
+    if ((hi & bm) != bm) return 0;
+    b0 = uint32_t(__ldg(T.dir + slot_of(T, k)) >> 16);
+    for (uint32_t q = 0; q < len; ++q) mm |= uint32_t(__ldg(T.keys + b0 + q) == k) << q;
+    if (__popc(mm) == 1) row = __ldg(T.rows + b0 + __ffs(mm) - 1);
+    return mm;
+}
+
+// A hit in a large mixed bucket: listed, to be counted later (rare: one atomic each).
+__device__ __forceinline__ void list_mixed(const ProbeTab& T, const Lists& Ls, uint32_t row, int32_t k, uint32_t hi) {
+    const uint32_t bm = bloom_mask(fib_hash(k)), p = slot_of(T, k);
+    if ((hi & bm) != bm) return;
+    const uint64_t q = atomicAdd(Ls.ctr + 1, 1ull);
+    Ls.m_row[q]      = row;
+    Ls.m_s[q]        = uint32_t(__ldg(T.dir + p) >> 16);
+    Ls.m_e[q]        = uint32_t(__ldg(T.dir + p + 1) >> 16);
+    Ls.m_key[q]      = k;
+    Ls.m_cnt[q]      = kUncounted;
+}
+
+__device__ __forceinline__ uint32_t bucket_tuples(const ProbeTab& T, uint32_t p) {
+    return uint32_t(__ldg(T.dir + p + 1) >> 16) - uint32_t(__ldg(T.dir + p) >> 16);
+}
+
+constexpr uint32_t kMaskTuples = 31;  // tuples of a small mixed bucket, at most
+
+// Count pass of a probe column of one tile: one block, two rows a thread, so
+// bound by the latency of its few dependent reads.  Matches keep an order (the
+// tile's rows by (i / 32) % 8, then i / 256, then i % 32): a warp takes two
+// runs of 32 rows that follow each other in it.  The block writes the counters
+// itself.  8 rows a thread with a staged copy of the keys took 11-18 us.
+constexpr int kTT = 1024;
+template <int SRC>
+__global__ void __launch_bounds__(kTT)
+    k_probe_tile(ProbeTab T, KeyCol pk, int light_max, Lists Ls, Outs outs, unsigned long long* host_ctr) {
+    constexpr uint32_t            kMany = 1u << 31;  // the warp has a hit that only the list can hold
+    constexpr int                 kR    = 2;
+    __shared__ uint32_t           s_wh[kTT / 32], s_wc[kTT / 32];
+    __shared__ unsigned long long s_wx[kTT / 32];
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, lt = (1u << lane) - 1;
+    const uint32_t small = min(uint32_t(light_max), kMaskTuples);
+    // a hit: c matches; x = kRowHit: build row s, 0: bucket s, else the mask x over the tuples from s on
+    uint32_t s[kR], x[kR], c[kR], row[kR], many = outs.n == 0;
+    int32_t  k[kR];
+    uint64_t w[kR];
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        row[u] = ((warp & 3) * kR + u) * 256 + (warp >> 2) * 32 + lane;
+        w[u]   = tile_key<SRC>(pk, 0, row[u], k[u]) ? __ldg(T.sum + slot_of(T, k[u])) : 0ull;
+    }
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const int32_t  hi  = int32_t(uint32_t(w[u] >> 32));
+        const uint32_t len = (uint32_t(hi) >> 16) & kSumLenMax;
+        s[u] = x[u] = c[u] = 0;
+        // a bucket of one key (hi > 0): its first key decides exactly (a
+        // matching key's Bloom bits are always in the bucket's tag)
+        if (hi > 0 && sum_head(w[u]) == k[u]) {
+            if ((hi >> 30) == 1) {
+                s[u] = uint32_t(hi) & 0x3fffffffu;
+                x[u] = kRowHit;
+                c[u] = 1;
+            } else {
+                s[u] = slot_of(T, k[u]);
+                c[u] = len == kSumLenMax ? bucket_tuples(T, s[u]) : len;
+                many |= 1;  // (also one tuple whose row does not fit the summary)
+            }
+        } else if (hi < 0 && len <= small) {
+            uint32_t one;
+            x[u] = compare_mixed(T, k[u], uint32_t(hi), s[u], one);
+            c[u] = __popc(x[u]);
+            many |= c[u] > 1;
+            if (c[u] == 1) {
+                s[u] = one;
+                x[u] = kRowHit;
+            }
+        } else if (hi < 0) {
+            list_mixed(T, Ls, row[u], k[u], uint32_t(hi));
+        }
+    }
+    uint32_t nh = 0, slot[kR];
+#pragma unroll
+    for (int u = 0; u < kR; ++u) {
+        const unsigned bal = __ballot_sync(0xffffffffu, c[u] > 0);
+        slot[u]            = nh + __popc(bal & lt);
+        nh += __popc(bal);
+    }
+    many = __any_sync(0xffffffffu, many);
+    if (lane == 0) s_wh[warp] = nh | (many ? kMany : 0u);
+    __syncthreads();
+    const uint32_t h  = s_wh[lane];
+    const bool     direct = !__any_sync(0xffffffffu, h & kMany);
+    const uint32_t hinc = warp_inclusive_scan(h & ~kMany), hs = __shfl_sync(0xffffffffu, hinc, 31);
+    const uint32_t hw   = warp ? __shfl_sync(0xffffffffu, hinc, int(warp) - 1) : 0u;
+    unsigned long long total = 0;
+    if (direct) {
+        for (int oi = 0; oi < outs.n; ++oi) {
+            const RidOut o = outs.o[oi];
+#pragma unroll
+            for (int u = 0; u < kR; ++u)
+                if (c[u]) {
+                    const uint32_t v         = o.side == 0 ? row[u] : s[u];
+                    o.dst[hw + slot[u]] = o.src ? __ldg(o.src + v) : v;
+                }
+        }
+    } else {
+        // first output rows from scans of the counts (32-bit prefix sums; the exact total beside them)
+        const uint32_t i0 = warp_inclusive_scan(c[0]), t0 = __shfl_sync(0xffffffffu, i0, 31);
+        const uint32_t i1 = warp_inclusive_scan(c[1]), t1 = __shfl_sync(0xffffffffu, i1, 31);
+        const unsigned long long tx = warp_sum<unsigned long long>((unsigned long long)c[0] + c[1]);
+        if (lane == 0) {
+            s_wc[warp] = t0 + t1;
+            s_wx[warp] = tx;
+        }
+        __syncthreads();
+        const uint32_t cinc = warp_inclusive_scan(s_wc[lane]);
+        const uint32_t cw   = warp ? __shfl_sync(0xffffffffu, cinc, int(warp) - 1) : 0u;
+        total               = warp_sum(s_wx[lane]);
+        const uint32_t oo[kR] = {cw + i0 - c[0], cw + t0 + i1 - c[1]};
+#pragma unroll
+        for (int u = 0; u < kR; ++u)
+            if (c[u]) {
+                const uint32_t q = hw + slot[u];
+                Ls.u_row[q]      = row[u];
+                Ls.u_sp[q]       = s[u];
+                Ls.u_off[q]      = oo[u];
+                Ls.u_mask[q]     = x[u];
+            }
+    }
+    if (threadIdx.x == 0) {
+        unsigned long long* to = host_ctr ? host_ctr : Ls.ctr;
+        const unsigned long long mixed = atomicAdd(Ls.ctr + 1, 0ull);  // (the block's barriers are behind its listings)
+        to[0] = direct ? 0ull : (uint64_t(hs) << 32) | uint32_t(total);
+        to[1] = mixed;
+        to[2] = total;
+        to[3] = 0;
+        to[5] = direct ? hs : 0u;
+    }
+}
+
+// Count pass of a probe column of several tiles.  A warp works by itself, kSU
+// rows a lane at a time, and puts off what only some rows need until a warp
+// is full of it: hits wait in its queue until 256 go out together (single
+// matches straight to the output, others to the list: one reservation each,
+// coalesced stores), rows that met a small mixed bucket until 32 are compared,
+// a lane each.  A block per tile with barriers and one reservation (as for a
+// single tile, to keep its order) took 126 us for 10M keys against 1M, 70%
+// matching; this 80.  Bound by the L1, whose random reads take a line each: the
+// queues leave 92 KB of it at 256 hits; at 384 the same probe takes 140 us, at
+// 128 (reservations twice as often) 103, with four rows a lane 253.
+constexpr int      kSU   = 2;    // rows per lane in flight
+constexpr uint32_t kQ     = 256;  // hits that a flush takes (reservations on one word run at 1.6e9/s in all)
+constexpr uint32_t kQMore = 32 * kSU;  // what a step adds at most before the next flush
+struct StreamQueues {
+    // hits: probe row, s, and kRowHit, a mask, or kLen | tuples of bucket s
+    uint32_t row[kQ + kQMore], s[kQ + kQMore], x[kQ + kQMore];
+    uint32_t m_row[31 + kQMore + 1], m_hi[31 + kQMore + 1];
+    int32_t  m_key[31 + kQMore + 1];  // rows that met a small mixed bucket: key and its summary's high word
+};
+constexpr uint32_t kLen = 1u << 31;
 
 template <int SRC>
 __global__ void __launch_bounds__(kPT, 4)
-    k_probe_count(ProbeTab T, KeyCol pk, int light_max, Lists Ls, uint64_t ntiles, Outs outs,
-                  unsigned long long* host_ctr) {
+    k_probe_stream(ProbeTab T, KeyCol pk, int light_max, Lists Ls, uint64_t ntiles, Outs outs,
+                   unsigned long long* host_ctr) {
     extern __shared__ __align__(128) uint8_t dyn[];
-    constexpr uint32_t SB  = stage_bytes(SRC);
-    constexpr int      kW  = kPT / 32;
-    uint8_t*           stg = dyn;  // 2 stages
-    __shared__ uint64_t bar[2];
-    __shared__ uint32_t s_cov;
-    // per warp: hits (and kMany); for the list, matches (mod 2^32), turned into
-    // the warp's base within the tile by thread 0, and exact match counts
-    constexpr uint32_t            kMany = 1u << 31;  // the warp has a hit that only the list can hold
-    __shared__ uint32_t           s_wh[kW], s_wc[kW];
-    __shared__ unsigned long long s_wx[kW];
-    __shared__ uint32_t           s_hb, s_ob;
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt   = (1u << lane) - 1;
-    uint32_t       cov0 = 0, cov1 = 0;   // thread 0: rows each stage's copy covers
-    uint32_t       iss0 = 0, iss1 = 0;   // thread 0: copies issued into each stage
-    bool           gave_up = false;  // a staging wait ran out of polls (an error)
-    if (SRC != kSrcGather && threadIdx.x == 0) {
-        mbar_init(&bar[0]);
-        mbar_init(&bar[1]);
-    }
-    __syncthreads();
-    if (SRC != kSrcGather && threadIdx.x == 0 && uint64_t(blockIdx.x) < ntiles) {
-        cov0 = stage_tile<SRC>(pk, blockIdx.x, stg, &bar[0]);
-        iss0 = 1;
-    }
-    const uint32_t small = min(uint32_t(light_max), 32u);
-    uint32_t       k     = 0;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++k) {
-        const uint32_t st = k & 1;
-        if (SRC != kSrcGather) {
-            // the other stage was last read before the previous iteration's
-            // barriers: refill it with the next tile now
-            const uint64_t next = tile + gridDim.x;
-            if (threadIdx.x == 0 && next < ntiles) {
-                const uint32_t c = stage_tile<SRC>(pk, next, stg + (st ^ 1) * SB, &bar[st ^ 1]);
-                if (st) { cov0 = c; ++iss0; } else { cov1 = c; ++iss1; }
+    const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+    StreamQueues&  Q    = reinterpret_cast<StreamQueues*>(dyn)[threadIdx.x >> 5];
+    const uint32_t small = min(uint32_t(light_max), kMaskTuples);  // masks of 31 tuples leave kLen and kRowHit apart
+    uint32_t       nq = 0, nm = 0;  // entries of the queues (the same in every lane)
+    unsigned long long listed = 0;  // this lane's listed matches
+    // The queue's last kQ hits out: matches of one build row each to the output
+    // (to the list when there is none), the others to the list.
+    auto flush = [&](uint32_t keep) {
+        while (nq > keep) {
+            __syncwarp();
+            const uint32_t n = min(nq, kQ);
+            nq -= n;
+            const uint32_t *qr = Q.row + nq, *qs = Q.s + nq, *qx = Q.x + nq;
+            auto one = [&](uint32_t e) { return outs.n != 0 && qx[e] == kRowHit; };
+            uint32_t nd = 0, tot = 0;  // direct entries; listed matches
+            for (uint32_t e = lane; e - lane < n; e += 32) {
+                const bool     on = e < n, d = on && one(e);
+                const uint32_t x  = on && !d ? qx[e] : 0u;
+                nd += __popc(__ballot_sync(0xffffffffu, d));
+                tot += x == kRowHit ? 1u : x & kLen ? x & ~kLen : uint32_t(__popc(x));
             }
-            gave_up = !mbar_wait_bounded(&bar[st], (k >> 1) & 1, kWaitPolls);
-            // thread 0 holds the covered counts; every thread needs this tile's
-            if (threadIdx.x == 0) s_cov = st ? cov1 : cov0;
+            listed += tot;
+            uint32_t           db = 0;
+            unsigned long long lb = 0;
+            if (nd < n) tot = warp_sum(tot);
+            if (lane == 0) {
+                if (nd) db = uint32_t(atomicAdd(Ls.ctr + 5, (unsigned long long)nd));
+                if (nd < n) lb = atomicAdd(Ls.ctr + 0, (uint64_t(n - nd) << 32) + tot);
+            }
+            db = __shfl_sync(0xffffffffu, db, 0);
+            if (nd == n) {
+                for (int oi = 0; oi < outs.n; ++oi) {
+                    const RidOut o = outs.o[oi];
+                    const uint32_t* v = o.side == 0 ? qr : qs;
+#pragma unroll 4
+                    for (uint32_t e = lane; e < n; e += 32) o.dst[db + e] = o.src ? __ldg(o.src + v[e]) : v[e];
+                }
+                __syncwarp();
+                continue;
+            }
+            lb = __shfl_sync(0xffffffffu, lb, 0);
+            uint32_t li = uint32_t(lb >> 32), off = uint32_t(lb);
+            for (uint32_t e = lane; e - lane < n; e += 32) {
+                const bool     on = e < n, d = on && one(e);
+                const unsigned bd = __ballot_sync(0xffffffffu, d), bl = __ballot_sync(0xffffffffu, on && !d);
+                const uint32_t x  = on && !d ? qx[e] : 0u;
+                const uint32_t c  = x == kRowHit ? 1u : x & kLen ? x & ~kLen : uint32_t(__popc(x));
+                const uint32_t in = warp_inclusive_scan(c);
+                if (d) {
+                    for (int oi = 0; oi < outs.n; ++oi) {
+                        const RidOut   o = outs.o[oi];
+                        const uint32_t v = o.side == 0 ? qr[e] : qs[e];
+                        o.dst[db + __popc(bd & lt)] = o.src ? __ldg(o.src + v) : v;
+                    }
+                } else if (on) {
+                    const uint32_t h = li + __popc(bl & lt);
+                    Ls.u_row[h]  = qr[e];
+                    Ls.u_sp[h]   = qs[e];
+                    Ls.u_off[h]  = off + in - c;
+                    Ls.u_mask[h] = x != kRowHit && (x & kLen) ? 0u : x;
+                }
+                db += __popc(bd);
+                li += __popc(bl);
+                off += __shfl_sync(0xffffffffu, in, 31);
+            }
+            __syncwarp();
         }
-        // one barrier that also tells every thread whether any gave up
-        if (__syncthreads_or(gave_up)) {
-            gave_up = true;
-            break;
+    };
+    // a lane's hit to the queue; every lane of the warp calls it
+    auto push = [&](bool on, uint32_t row, uint32_t s, uint32_t x) {
+        const unsigned bal = __ballot_sync(0xffffffffu, on);
+        if (on) {
+            const uint32_t q = nq + __popc(bal & lt);
+            Q.row[q] = row;
+            Q.s[q]   = s;
+            Q.x[q]   = x;
         }
-        const uint32_t cov   = SRC != kSrcGather ? s_cov : 0u;
-        const uint64_t r0    = tile * kTileRows;
-        const uint32_t nrows = uint32_t(umin64(kTileRows, pk.n - r0));
-        const uint8_t* stage = stg + st * SB;
-        int32_t  key[kStep];
-        bool     ok[kStep];
-        uint64_t w[kStep];
+        nq += __popc(bal);
+    };
+    // rows that met a small mixed bucket: its tuples compared, the matching ones as a mask
+    auto compare = [&](uint32_t keep) {
+        while (nm > keep) {
+            __syncwarp();
+            const uint32_t n = min(nm, 32u);
+            nm -= n;
+            uint32_t mm = 0, row = 0, b0 = 0, one = 0;
+            if (lane < n) {
+                row = Q.m_row[nm + lane];
+                mm  = compare_mixed(T, Q.m_key[nm + lane], Q.m_hi[nm + lane], b0, one);
+            }
+            __syncwarp();
+            const bool single = __popc(mm) == 1;
+            push(mm != 0, row, single ? one : b0, single ? kRowHit : mm);
+            flush(kQ - 1);
+        }
+    };
+    int32_t  nk[kSU];
+    uint32_t nok = 0;  // keys of the next step, and which are valid
+    auto     fetch = [&](uint64_t tile, uint32_t x0) {
+        nok = 0;
 #pragma unroll
-        for (int it = 0; it < kStep; ++it) {
-            const uint32_t i = uint32_t(it) * kPT + threadIdx.x;
-            ok[it]           = false;
-            key[it]          = 0;
-            w[it]            = 0;
-            if (i < nrows) ok[it] = tile_key<SRC>(pk, stage, cov, i, r0 + i, key[it]);
+        for (int u = 0; u < kSU; ++u)
+            nok |= uint32_t(tile_key<SRC>(pk, tile, x0 + u * kPT + threadIdx.x, nk[u])) << u;
+    };
+    uint64_t tile = blockIdx.x;
+    uint32_t x0   = 0;
+    if (tile < ntiles) fetch(tile, 0);
+    while (tile < ntiles) {
+        int32_t        k[kSU];
+        uint64_t       w[kSU];
+        const uint32_t ok = nok;
+        const uint32_t r0 = uint32_t(tile * kTileRows + x0 + threadIdx.x);
+#pragma unroll
+        for (int u = 0; u < kSU; ++u) {
+            k[u] = nk[u];
             // through L1: with skewed probe keys the hot buckets' summaries stay there
-            if (ok[it]) w[it] = __ldg(T.sum + slot_of(T, key[it]));
+            w[u] = (ok >> u) & 1u ? __ldg(T.sum + slot_of(T, k[u])) : 0ull;
         }
-        // classify: a row is a miss, a hit staged here (bit `it` of hit), or in
-        // a mixed bucket counted later.  Directory words are read only for mixed
-        // buckets and for uniform buckets whose length saturated the summary's
-        // field.  s: the build row of a single tuple (bit of one), the first
-        // tuple of a bucket with a mask, else the bucket.
-        uint32_t s[kStep], L[kStep], msk[kStep];
-        uint32_t hit = 0, one = 0, many = 0;  // many: hits that only the list can hold
+        x0 += kSU * kPT;
+        if (x0 >= kTileRows) {
+            x0 = 0;
+            tile += gridDim.x;
+        }
+        if (tile < ntiles) fetch(tile, x0);
 #pragma unroll
-        for (int it = 0; it < kStep; ++it) {
-            L[it]    = sum_len(w[it]);
-            msk[it]  = 0;
-            int  cls = 0;
-            if (ok[it] && L[it] != 0) {
-                if (!sum_mixed(w[it])) {
-                    // a bucket of one key: its first key decides exactly (a matching
-                    // key's Bloom bits are always in the bucket's tag)
-                    cls = sum_head(w[it]) == key[it] ? 1 : 0;
-                } else {
-                    const uint32_t m = bloom_mask(fib_hash(key[it]));
-                    cls              = (sum_bloom(w[it]) & m) == m ? 2 : 0;
+        for (int u = 0; u < kSU; ++u) {
+            const int32_t  hi  = int32_t(uint32_t(w[u] >> 32));
+            const uint32_t row = r0 + u * kPT, len = (uint32_t(hi) >> 16) & kSumLenMax;
+            // a bucket of one key (hi > 0): its first key decides exactly (a
+            // matching key's Bloom bits are always in the bucket's tag)
+            const bool hit  = hi > 0 && sum_head(w[u]) == k[u];
+            const bool one  = hit && (hi >> 30) == 1;
+            const bool mix  = hi < 0 && len <= small;
+            const bool rare = (hi < 0 && len > small) || (hit && !one && len == kSumLenMax);
+            push(hit && !rare, row, one ? uint32_t(hi) & 0x3fffffffu : slot_of(T, k[u]), one ? kRowHit : kLen | len);
+            if (__any_sync(0xffffffffu, hi < 0 || rare)) {
+                const unsigned bal = __ballot_sync(0xffffffffu, mix);
+                if (mix) {
+                    const uint32_t q = nm + __popc(bal & lt);
+                    Q.m_row[q]       = row;
+                    Q.m_key[q]       = k[u];
+                    Q.m_hi[q]        = uint32_t(hi);
                 }
-            }
-            const uint32_t p = slot_of(T, key[it]);
-            s[it]            = p;
-            uint32_t e       = 0;
-            if (cls == 1 && sum_single(w[it])) {
-                s[it] = sum_row(w[it]);
-                one |= 1u << it;
-            } else if (cls == 2 || (cls == 1 && L[it] == kSumLenMax)) {
-                const uint32_t b0 = uint32_t(__ldg(T.dir + p) >> 16);
-                L[it]             = uint32_t(__ldg(T.dir + p + 1) >> 16) - b0;
-                if (cls == 2) s[it] = b0;
-                e = b0 + L[it];
-            }
-            // a small mixed bucket: compared here, its matches as a mask
-            if (cls == 2 && L[it] <= small) {
-                uint32_t mm = 0;
-                for (uint32_t q = 0; q < L[it]; ++q) mm |= uint32_t(__ldg(T.keys + s[it] + q) == key[it]) << q;
-                msk[it] = mm;
-                L[it]   = __popc(mm);
-                cls     = mm ? 1 : 0;
-            }
-            hit |= uint32_t(cls == 1) << it;
-            many |= uint32_t(cls == 2 || (cls == 1 && L[it] != 1)) << it;
-            // larger mixed buckets: counted later; rare, so warp-aggregated
-            // global atomics
-            const unsigned bal = __ballot_sync(0xffffffffu, cls == 2);
-            if (bal) {
-                unsigned long long q0 = 0;
-                if (lane == 0) q0 = atomicAdd(Ls.ctr + 1, (unsigned long long)__popc(bal));
-                q0 = __shfl_sync(0xffffffffu, q0, 0);
-                if (cls == 2) {
-                    const uint64_t q = q0 + __popc(bal & lt);
-                    Ls.m_row[q]      = uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x);
-                    Ls.m_s[q]        = s[it];
-                    Ls.m_e[q]        = e;
-                    Ls.m_key[q]      = key[it];
-                    Ls.m_cnt[q]      = kUncounted;
+                nm += __popc(bal);
+                if (rare) {
+                    // a length beyond its field (listed at once), or a large mixed bucket
+                    if (hi > 0) {
+                        const uint32_t           p = slot_of(T, k[u]), n = bucket_tuples(T, p);
+                        const unsigned long long base = atomicAdd(Ls.ctr + 0, (1ull << 32) + n);
+                        Ls.u_row[base >> 32]  = row;
+                        Ls.u_sp[base >> 32]   = p;
+                        Ls.u_off[base >> 32]  = uint32_t(base);
+                        Ls.u_mask[base >> 32] = 0;
+                        listed += n;
+                    } else {
+                        list_mixed(T, Ls, row, k[u], uint32_t(hi));
+                    }
                 }
             }
         }
-        // the warp's hits in (it, lane) order, so the hits of one round are
-        // consecutive slots (coalesced stores): a ballot per round ranks them
-        uint32_t nh = 0, slot[kStep];
-#pragma unroll
-        for (int it = 0; it < kStep; ++it) {
-            const unsigned bal = __ballot_sync(0xffffffffu, (hit >> it) & 1u);
-            slot[it]           = nh + __popc(bal & lt);
-            nh += __popc(bal);
-        }
-        if (__any_sync(0xffffffffu, many) || outs.n == 0) nh |= kMany;
-        if (lane == 0) s_wh[warp] = nh;
-        __syncthreads();
-        uint32_t hw = 0, hs = 0, any = 0;  // hits of the warps before this one, and of all
-#pragma unroll
-        for (uint32_t q = 0; q < uint32_t(kW); ++q) {
-            const uint32_t h = s_wh[q];
-            any |= h;
-            hw += q < warp ? h & ~kMany : 0u;
-            hs += h & ~kMany;
-        }
-        if (!(any & kMany)) {
-            // one match a hit: its row ids straight to the output, which takes
-            // the place of a list entry, the list's passes and their launches
-            if (threadIdx.x == 0) s_ob = hs ? uint32_t(atomicAdd(Ls.ctr + 5, (unsigned long long)hs)) : 0u;
-#pragma unroll
-            for (int it = 0; it < kStep; ++it)
-                if (((hit & ~one) >> it) & 1u)
-                    s[it] = __ldg(T.rows + (msk[it] ? s[it] + uint32_t(__ffs(msk[it]) - 1)
-                                                    : uint32_t(__ldg(T.dir + s[it]) >> 16)));
-            __syncthreads();
-            const uint32_t ob = s_ob + hw;
-            for (int oi = 0; oi < outs.n; ++oi) {
-                const RidOut o = outs.o[oi];
-                if (o.src) {
-                    uint32_t v[kStep];
-#pragma unroll
-                    for (int it = 0; it < kStep; ++it)
-                        if ((hit >> it) & 1u)
-                            v[it] = __ldg(o.src + (o.side == 0 ? uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x) : s[it]));
-#pragma unroll
-                    for (int it = 0; it < kStep; ++it)
-                        if ((hit >> it) & 1u) o.dst[ob + slot[it]] = v[it];
-                } else {
-#pragma unroll
-                    for (int it = 0; it < kStep; ++it)
-                        if ((hit >> it) & 1u)
-                            o.dst[ob + slot[it]] = o.side == 0 ? uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x) : s[it];
-                }
-            }
-            continue;
-        }
-        // to the list: a warp scan of a round's counts gives their first output
-        // rows within the warp (32-bit prefix sums; the exact total is summed
-        // beside them)
-        uint32_t           nc = 0, oo[kStep];
-        unsigned long long lx = 0;
-        static_assert(kStep % 2 == 0, "rounds are scanned in pairs");
-#pragma unroll
-        for (int it = 0; it < kStep; it += 2) {
-            const uint32_t c0 = (hit >> it) & 1u ? L[it] : 0u, c1 = (hit >> (it + 1)) & 1u ? L[it + 1] : 0u;
-            if (__all_sync(0xffffffffu, (c0 | c1) < 2048)) {
-                // both rounds in one scan of 16-bit halves (a half sums to < 2^16)
-                const uint32_t v   = c0 | (c1 << 16);
-                const uint32_t inc = warp_inclusive_scan<uint32_t>(v);
-                const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
-                const uint32_t ex  = inc - v;
-                oo[it]             = nc + (ex & 0xffffu);
-                oo[it + 1]         = nc + (tot & 0xffffu) + (ex >> 16);
-                nc += (tot & 0xffffu) + (tot >> 16);
-            } else {
-                const uint32_t i0 = warp_inclusive_scan<uint32_t>(c0);
-                oo[it]            = nc + i0 - c0;
-                nc += __shfl_sync(0xffffffffu, i0, 31);
-                const uint32_t i1 = warp_inclusive_scan<uint32_t>(c1);
-                oo[it + 1]        = nc + i1 - c1;
-                nc += __shfl_sync(0xffffffffu, i1, 31);
-            }
-            lx += uint64_t(c0) + c1;
-        }
-        const unsigned long long nx = warp_sum<unsigned long long>(lx);
-        if (lane == 0) {
-            s_wc[warp] = nc;
-            s_wx[warp] = nx;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t           cs = 0;
-            unsigned long long xs = 0;
-#pragma unroll
-            for (int q = 0; q < kW; ++q) {
-                const uint32_t c = s_wc[q];
-                s_wc[q] = cs;
-                cs += c;
-                xs += s_wx[q];
-            }
-            const unsigned long long base = hs ? atomicAdd(Ls.ctr + 0, (uint64_t(hs) << 32) + cs) : 0ull;
-            if (xs) atomicAdd(Ls.ctr + 2, xs);
-            s_hb = uint32_t(base >> 32);
-            s_ob = uint32_t(base);
-        }
-        __syncthreads();
-        const uint32_t hb = s_hb + hw, ob = s_ob + s_wc[warp];
-#pragma unroll
-        for (int it = 0; it < kStep; ++it) {
-            if ((hit >> it) & 1u) {
-                const uint32_t q = hb + slot[it];
-                Ls.u_row[q]      = uint32_t(r0 + uint32_t(it) * kPT + threadIdx.x);
-                Ls.u_sp[q]       = (one >> it) & 1u ? slot_of(T, key[it]) : s[it];
-                Ls.u_off[q]      = ob + oo[it];
-                Ls.u_mask[q]     = msk[it];
-            }
-        }
+        flush(kQ - 1);
+        compare(31);
     }
-    if (SRC != kSrcGather) {
-        // a block that gave up waits (bounded) for the copies it issued, so no
-        // copy lands in shared memory after the block has exited
-        if (gave_up && threadIdx.x == 0) {
-            atomicAdd(Ls.ctr + 4, 1ull);
-            if (iss0) mbar_wait_bounded(&bar[0], (iss0 - 1) & 1, kWaitPolls);
-            if (iss1) mbar_wait_bounded(&bar[1], (iss1 - 1) & 1, kWaitPolls);
-        }
-    }
-    // the block that is done last hands the counters to the host and clears
-    // them for the next probe (not the mixed hits, which are still to be counted)
-    if (host_ctr && threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(Ls.ctr + 6, 1ull) == gridDim.x - 1) {
-            __threadfence();
-            for (int q = 0; q < 6; ++q) {
-                const unsigned long long v = atomicAdd(Ls.ctr + q, 0ull);
-                host_ctr[q]                = v;
-                if (q != 1) Ls.ctr[q] = 0;
-            }
-            Ls.ctr[6] = 0;
-        }
-    }
+    compare(0);
+    flush(0);
+    listed = warp_sum(listed);
+    if (lane == 0 && listed) atomicAdd(Ls.ctr + 2, listed);
+    __syncthreads();
+    hand_over(Ls, host_ctr);
 }
 
 // Mixed hits still uncounted: a warp each for buckets of up to kMixedWarpMax
@@ -575,7 +633,8 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
 #pragma unroll
                 for (int i = 0; i < G; ++i) {
                     const uint32_t idx = q0 + i - orel;  // match number within the hit
-                    brow[i]            = q0 + i < len ? __ldg(T.rows + t0 + (m ? nth_bit(m, idx) : idx)) : 0u;
+                    brow[i]            = q0 + i >= len ? 0u
+                                       : m == kRowHit ? t0 : __ldg(T.rows + t0 + (m ? nth_bit(m, idx) : idx));
                 }
                 const bool full = q0 + G <= len;
                 for (int oi = 0; oi < outs.n; ++oi) {
@@ -632,7 +691,7 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
                     const uint32_t idx = q - s_orel[k];  // match number within the hit
                     const uint32_t m   = s_msk[k];
                     prow[i]            = s_pr[k];
-                    brow[i]            = __ldg(T.rows + s_s[k] + (m ? nth_bit(m, idx) : idx));
+                    brow[i]            = m == kRowHit ? s_s[k] : __ldg(T.rows + s_s[k] + (m ? nth_bit(m, idx) : idx));
                 }
             }
             const bool full = q0 + G <= len;
@@ -702,55 +761,49 @@ __global__ void __launch_bounds__(512)
     }
 }
 
-ProbeTab tab_of(const Table& t) { return ProbeTab{t.dir, t.summary, t.keys, t.rows, t.dir_bits}; }
+ProbeTab tab_of(const Table& t) { return ProbeTab{t.dir, t.summary, t.keys, t.rows, 1u << t.dir_bits}; }
 
-// How the count kernel reads a probe column's keys.  A bulk copy needs a
-// 16-byte aligned source; tiles start at multiples of 3968 rows (of 16-byte
-// multiples for every form), so the column's base address decides.  Columns
-// at other addresses (a caller's array at an arbitrary 4-byte offset) are
-// read by direct loads.
+// How the count kernels read a probe column's keys.
 int key_source(const KeyCol& pk) {
-    auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (pk.rid || pk.filt.n) return kSrcGather;
-    if (pk.col.tagged) return aligned(pk.col.tagged) ? kSrcTagged : kSrcGather;
-    if (pk.col.plain) return aligned(pk.col.plain) ? kSrcPlain : kSrcGather;
-    return aligned(pk.col.pages) ? kSrcPages : kSrcGather;
+    return pk.col.tagged ? kSrcTagged : pk.col.plain ? kSrcPlain : kSrcPages;
 }
 
 template <int SRC>
-void launch_count_src(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, const Outs& outs,
-                      uint64_t* host_ctr, cudaStream_t st) {
-    const uint64_t ntiles = (pk.n + kTileRows - 1) / kTileRows;
-    const size_t   smem   = std::max<size_t>(16, 2 * size_t(stage_bytes(SRC)));
-    // shared memory for the resident blocks only; the rest of the unified
-    // L1 / shared memory caches bucket summaries
+void launch_stream_src(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, const Outs& outs,
+                       uint64_t* host_ctr, cudaStream_t st) {
+    const uint64_t       ntiles = (pk.n + kTileRows - 1) / kTileRows;
+    constexpr size_t     smem   = sizeof(StreamQueues) * (kPT / 32);
     static OncePerDevice    once;
     static std::atomic<int> resident{0};
     once([&] {
         int n = 0;
-        HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        HJ_CUDA(cudaFuncSetAttribute(k_probe_count<SRC>, cudaFuncAttributePreferredSharedMemoryCarveout, 30));
-        HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_probe_count<SRC>, kPT, smem));
+        HJ_CUDA(cudaFuncSetAttribute(k_probe_stream<SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        HJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_probe_stream<SRC>, kPT, smem));
         resident.store(n);
     });
-    // resident blocks walk the tiles (each prefetching its next tile)
-    const int per_sm = resident.load();
-    const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>(ntiles, uint64_t(num_sms()) * std::max(1, per_sm)));
-    k_probe_count<SRC><<<unsigned(grid), kPT, smem, st>>>(T, pk, light_max, L, ntiles, outs,
-                                                          reinterpret_cast<unsigned long long*>(host_ctr));
+    const uint64_t grid = std::min<uint64_t>(ntiles, uint64_t(num_sms()) * std::max(1, resident.load()));
+    k_probe_stream<SRC><<<unsigned(grid), kPT, smem, st>>>(T, pk, light_max, L, ntiles, outs,
+                                                           reinterpret_cast<unsigned long long*>(host_ctr));
     HJ_LAUNCH_CHECK();
 }
 
 // Count kernels over a probe column: uniform and mixed lists, counters in
-// L.ctr; with outs, tiles of single matches straight to the output (pk.n rows
-// each); with host_ctr, the counters to the host and cleared.
+// L.ctr; with outs, matches of one build row a probe row straight to the
+// output (pk.n rows each); with host_ctr, the counters to the host and cleared.
 void launch_count(const ProbeTab& T, const KeyCol& pk, int light_max, const Lists& L, const Outs& outs,
                   uint64_t* host_ctr, cudaStream_t st) {
+    auto run = [&](auto src) {
+        constexpr int S = decltype(src)::value;
+        if (pk.n > kTileRows) return launch_stream_src<S>(T, pk, light_max, L, outs, host_ctr, st);
+        k_probe_tile<S><<<1, kTT, 0, st>>>(T, pk, light_max, L, outs, reinterpret_cast<unsigned long long*>(host_ctr));
+        HJ_LAUNCH_CHECK();
+    };
     switch (key_source(pk)) {
-    case kSrcPages: launch_count_src<kSrcPages>(T, pk, light_max, L, outs, host_ctr, st); break;
-    case kSrcPlain: launch_count_src<kSrcPlain>(T, pk, light_max, L, outs, host_ctr, st); break;
-    case kSrcTagged: launch_count_src<kSrcTagged>(T, pk, light_max, L, outs, host_ctr, st); break;
-    default: launch_count_src<kSrcGather>(T, pk, light_max, L, outs, host_ctr, st); break;
+    case kSrcPages: run(std::integral_constant<int, kSrcPages>{}); break;
+    case kSrcPlain: run(std::integral_constant<int, kSrcPlain>{}); break;
+    case kSrcTagged: run(std::integral_constant<int, kSrcTagged>{}); break;
+    default: run(std::integral_constant<int, kSrcGather>{}); break;
     }
 }
 
@@ -819,12 +872,6 @@ void launch_mixed_writers(const ProbeTab& T, const Lists& L, const uint64_t* mix
     HJ_LAUNCH_CHECK();
 }
 
-void check_staging(const uint64_t* host_ctr) {
-    if (host_ctr[4])
-        throw Error(HJ_ERR_DEVICE_STATUS, "probe: " + std::to_string(host_ctr[4])
-                                              + " blocks gave up waiting for their staged key tiles");
-}
-
 }  // namespace
 
 struct ProbePlan {
@@ -862,7 +909,6 @@ uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, c
     if (prm.after_count) prm.after_count();
     HJ_CUDA(cudaStreamSynchronize(st));
     pp->n_m = pp->host[1];  // probe_free clears their counters
-    check_staging(pp->host);
     count_mixed(tab_of(t), L, pp->host, st);
     pp->n_u   = pp->host[0] >> 32;
     pp->tot_u = pp->host[2];
@@ -955,7 +1001,6 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
     uint64_t* h = prm.pinned;
     readback(h, L.ctr, 5 * sizeof(uint64_t), true, st);  // page-locked scratch
     HJ_CUDA(cudaStreamSynchronize(st));
-    check_staging(h);
     count_mixed(T, L, h, st);
     const uint64_t n_u = h[0] >> 32, n_m = h[1], tot_u = h[2], total = h[2] + h[3];
     *num_matches = total;
