@@ -840,7 +840,6 @@ void prefer_shared(K kernel) {
                                  int(cudaSharedmemCarveoutMaxShared)));
 }
 
-constexpr uint64_t kDirectKeys = 1u << 16;  // most keys of a one-launch build
 constexpr uint64_t kDirectPart = 2048;      // tuples of one of its partitions, about
 constexpr uint32_t kDirectBits = 13;        // bucket bits of one, at most
 
@@ -853,12 +852,6 @@ void alloc_table(Table& t, uint32_t b, uint64_t nv, cudaStream_t st) {
     t.rows            = dalloc_n<uint32_t>(nv, st);
     t.mixed           = dalloc_n<uint32_t>((nb + 31) / 32, st);
     t.summary         = dalloc_n<uint64_t>(nb, st);
-}
-
-uint32_t ceil_log2(uint64_t n) {
-    uint32_t b = 0;
-    while ((1ull << b) < n) ++b;
-    return b;
 }
 
 template <class K>

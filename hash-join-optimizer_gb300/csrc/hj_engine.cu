@@ -840,7 +840,48 @@ struct Exec {
         else if (!bkc.rid) hint = int64_t(bd.non_null);
         const uint64_t bres = plan.inputs[bk.table].resident;
         std::shared_ptr<Table> cached;
-        if (c->table_cache && !bkc.rid && bres) {
+        const bool cacheable = c->table_cache && !bkc.rid && bres;
+        int        bits      = int(c->dir_bits);
+        // A short probe side meets few build rows: only those are built on (the
+        // matches, and their order in the tile, are as before).  A join without
+        // and with it, us: 66,000 x 1,984 rows 98 / 70, 1M x 1,984 116 / 72, 10M x
+        // 1,984 325 / 106, 10M x 8,192 338 / 267; Zipf probe keys 1M x 1,984 117 /
+        // 68; one key's 20M pairs 1M x 1,984 339 / 282.  It loses where one key
+        // takes a quarter of the build rows, which then stay: 300,000 x 30 154 /
+        // 168, 1M x 400 338 / 368.  At 2^16 rows and less a build is one launch.  The
+        // table over the probe side instead was as fast for distinct keys, but a
+        // repeated one made its buckets heavy (Zipf, 1M x 31,250: 122 / 149).
+        std::vector<int> ss{bk.src};  // the build side's sources that are read
+        for (auto [side, s] : need)
+            if (side == 1 && s != bk.src) ss.push_back(s);
+        if (!cacheable && ss.size() <= size_t(kMaxRidOut) && bkc.n > (1u << 16) && bkc.n <= 0xffffffffull &&
+            pkc.n > 0 && pkc.n <= kReduceKeys && pkc.n <= bkc.n / 16) {
+            std::vector<RidOut> ro;
+            std::vector<Buf>    dst;
+            for (int s : ss) {
+                dst.push_back(make_buf(bkc.n * 4, c->st));
+                ro.push_back(RidOut{1, B.srcs[s].rid ? B.srcs[s].rid->as<uint32_t>() : nullptr,
+                                    dst.back()->as<uint32_t>()});
+            }
+            ProbeParams rp;
+            rp.pinned        = c->pinned;
+            rp.counters      = c->counters;
+            const uint64_t m = reduce_build(bkc, pkc, rp, ro.data(), int(ro.size()), c->st);
+            // not worth it when most rows stay: the streams are dropped
+            if (m <= bkc.n / 2) {
+                for (size_t i = 0; i < ss.size(); ++i) B.srcs[ss[i]].rid = dst[i];
+                B.rows = m;
+                // a sparse directory (32 buckets a row, at most what all rows would
+                // get): what passed by chance seldom shares a bucket with a heavy
+                // key, whose matches would then lose their place in the tile
+                const int full = int(ceil_log2(std::max<uint64_t>(hint >= 0 ? uint64_t(hint) : bkc.n, 1)));
+                if (bits < 0 && m > 0) bits = std::min({full, int(ceil_log2(m)) + 5, m <= kDirectKeys ? 20 : 64,
+                                                        std::max(0, int(c->dir_cap_bits))});
+                bkc  = key_col(B, bk);
+                hint = int64_t(m);
+            }
+        }
+        if (cacheable) {
             const BuiltKey key{bres, bk.col, c->dir_bits, c->radix_bits, c->dir_cap_bits};
             {
                 std::lock_guard<std::mutex> g(c->store->mu);
@@ -860,7 +901,7 @@ struct Exec {
             }
             t = *cached;
         } else {
-            build_table(bkc, int(c->dir_bits), int(c->radix_bits), t, c->pinned, c->st, hint,
+            build_table(bkc, bits, int(c->radix_bits), t, c->pinned, c->st, hint,
                         int(c->dir_cap_bits));
         }
         ++joins;

@@ -96,6 +96,12 @@ struct Table {
     uint64_t* summary   = nullptr;  // 2^dir_bits bucket summaries (make_summary, hj_common.cuh)
 };
 
+inline uint32_t ceil_log2(uint64_t n) {
+    uint32_t b = 0;
+    while ((1ull << b) < n) ++b;
+    return b;
+}
+
 // Builds `t` over the valid keys of `kc`.  dir_bits < 0: next_pow2(#valid).
 // radix_bits < 0: automatic.  Allocates t's arrays with dalloc.  n_valid: the
 // number of valid keys when the caller knows it (>= 0), else the build reads
@@ -104,6 +110,7 @@ struct Table {
 // directory stays cache resident; 64 = UnchainedHash sizing exactly.
 void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint64_t* scratch_host,
                  cudaStream_t st, int64_t n_valid = -1, int dir_cap_bits = 64);
+constexpr uint64_t kDirectKeys = 1u << 16;  // most keys of a one-launch build
 void free_table(Table& t, cudaStream_t st);
 
 // ---- probe (hj_probe.cu) ---------------------------------------------------
@@ -123,6 +130,14 @@ struct ProbeParams {
     uint64_t* counters  = nullptr;  // 8 zeroed device words; zero again after each probe (probe_free)
     std::function<void()> after_count;  // called once the count kernels are enqueued
 };
+
+// Build rows whose key may occur among the probe keys (all that do, and a few
+// that share a bit with one; no NULL keys), in any order: their number, and per
+// stream o.dst[k] = o.src ? o.src[row] : row (b.n slots each).  One host
+// synchronisation.  p.n <= kReduceKeys, b.n < 2^32.
+constexpr uint64_t kReduceKeys = 8192;
+uint64_t reduce_build(const KeyCol& b, const KeyCol& p, const ProbeParams& prm, const RidOut* outs, int nout,
+                      cudaStream_t st);
 
 struct ProbePlan;  // opaque match list between the count and write passes
 
