@@ -13,21 +13,23 @@
 // adjacency array on the host with per-thread slab buffers
 // (include/slab_allocator.h) and three phases.  Here the slabs are replaced by
 // a two-level MSD radix partition:
-//   1. k_part_hist      histogram of the top R hash bits (R = b - 12)
-//   2. k_part_offsets   partition offsets and per-partition chunk counts
+//   1. k_part_hist      histogram of the top R hash bits (R = b - 12), then
+//   2. (its last block) partition offsets and per-partition chunk counts
 //   3. k_part_scatter   (key, row) pairs scattered to their partition
 // Partitions of at most kFuseMax tuples are then built by one block each
-// (k_bucket_local); the larger ones (Zipf-heavy keys) take steps 4-7, with
-// their counters cleared first (k_bucket_zero):
-//   4. k_bucket_count   per 8192-tuple chunk: shared-memory bucket counts and
-//                       Bloom tags over the partition's 2^12 buckets
-//   5. k_bucket_dir     per partition: prefix sum -> directory words
-//   6. k_bucket_scatter per chunk: tuples to their final adjacency slots
-//   7. k_bucket_mixed   flags buckets that hold more than one distinct key
+// (k_bucket_local); the larger ones (Zipf-heavy keys) take steps 4-7 as the
+// phases of one kernel (k_bucket_big):
+//   4. per 8192-tuple chunk: shared-memory bucket counts and Bloom tags over
+//      the partition's 2^12 buckets
+//   5. per partition: prefix sum -> directory words
+//   6. per chunk: tuples to their final adjacency slots
+//   7. flags buckets that hold more than one distinct key, then summaries
 // Shared-memory histograms per chunk keep Zipf-heavy keys (one key can own
 // millions of tuples) off global atomics: a chunk adds one atomic per
 // non-empty bucket, and warp-aggregated shared atomics absorb duplicates.
 #include <algorithm>
+
+#include <cooperative_groups.h>
 
 #include "hj_block.cuh"
 #include "hj_common.cuh"
@@ -41,8 +43,7 @@ constexpr int kMaxRadix    = 14;
 constexpr int kThreads     = 512;
 constexpr int kItems       = 16;
 constexpr int kTile        = kThreads * kItems;  // rows per partition-scatter tile
-constexpr int kChunkTiles  = 1;
-constexpr int kChunk       = kChunkTiles * kTile;  // tuples per bucket chunk
+constexpr int kChunk       = kTile;              // tuples per bucket chunk
 // Partitions of at most kFuseMax tuples are built by one block each
 // (k_bucket_local); the chunked kernels take the larger ones.
 constexpr uint32_t kFuseMax = 12288;
@@ -58,11 +59,44 @@ __device__ __forceinline__ bool load_key(const KeyCol& kc, uint64_t i, int32_t& 
     return int_get(kc.col, kc.rid ? uint64_t(__ldg(kc.rid + i)) : i, key);
 }
 
-// 1. Partition histogram + count of valid keys.
-__global__ void __launch_bounds__(kThreads)
-    k_part_hist(KeyCol kc, uint32_t R, uint32_t* __restrict__ part_cnt,
-                unsigned long long* __restrict__ n_valid) {
+// 2. Exclusive scans of partition sizes and chunk counts, by one block.  Only
+//    the partitions k_bucket_local does not take are cut into chunks; each
+//    chunk's partition is written to chunk_part, so that a block finds a
+//    chunk's partition with one load.
+struct Parts {
+    uint32_t *cnt, *off, *cursor, *chunk_off, *chunk_part;
+    unsigned long long* n_valid;  // [1]: blocks of k_part_hist that are done, [2..3]: k_bucket_big's tickets
+};
+__device__ __forceinline__ void part_offsets(const Parts& d, uint32_t P, uint32_t* sm) {
+    uint32_t run_t = 0, run_c = 0;
+    for (uint32_t base = 0; base < P; base += blockDim.x) {
+        const uint32_t i  = base + threadIdx.x;
+        const uint32_t c  = i < P ? __ldcg(d.cnt + i) : 0;  // (other blocks' atomics)
+        const uint32_t ch = c > kFuseMax ? (c + kChunk - 1) / kChunk : 0u;
+        uint32_t       tot_t, tot_c;
+        const uint32_t et = block_exclusive_scan<uint32_t>(c, sm, &tot_t);
+        const uint32_t ec = block_exclusive_scan<uint32_t>(ch, sm, &tot_c);
+        if (i < P) {
+            d.off[i]       = run_t + et;
+            d.cursor[i]    = run_t + et;
+            d.chunk_off[i] = run_c + ec;
+            for (uint32_t q = 0; q < ch; ++q) d.chunk_part[run_c + ec + q] = i;
+        }
+        run_t += tot_t;
+        run_c += tot_c;
+    }
+    if (threadIdx.x == 0) {
+        d.off[P]       = run_t;
+        d.chunk_off[P] = run_c;
+    }
+}
+
+// 1. Partition histogram + count of valid keys; the block that is done last
+//    makes the offsets (2).
+__global__ void __launch_bounds__(kThreads) k_part_hist(KeyCol kc, uint32_t R, Parts d) {
     extern __shared__ uint32_t hist[];
+    __shared__ uint32_t        sm[33];
+    __shared__ bool            last;
     const uint32_t P = 1u << R;
     for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) hist[i] = 0;
     __syncthreads();
@@ -84,43 +118,16 @@ __global__ void __launch_bounds__(kThreads)
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < P; i += blockDim.x)
-        if (hist[i]) atomicAdd(part_cnt + i, hist[i]);
+        if (hist[i]) atomicAdd(d.cnt + i, hist[i]);
     mine = warp_sum(mine);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(n_valid, (unsigned long long)mine);
-}
-
-// 2. Exclusive scans of partition sizes and chunk counts (one block).  Only
-//    the partitions k_bucket_local does not take are cut into chunks; each
-//    chunk's partition is written to chunk_part, so a chunk kernel's block
-//    finds its partition with one load.
-__global__ void __launch_bounds__(1024)
-    k_part_offsets(const uint32_t* __restrict__ part_cnt, uint32_t P, uint32_t* __restrict__ part_off,
-                   uint32_t* __restrict__ part_cursor, uint32_t* __restrict__ chunk_off,
-                   uint32_t* __restrict__ chunk_part) {
-    __shared__ uint32_t sm[33];
-    uint32_t            run_t = 0, run_c = 0;
-    for (uint32_t base = 0; base < P; base += blockDim.x) {
-        const uint32_t i  = base + threadIdx.x;
-        const uint32_t c  = i < P ? part_cnt[i] : 0;
-        const uint32_t ch = c > kFuseMax ? (c + kChunk - 1) / kChunk : 0u;
-        uint32_t       tot_t, tot_c;
-        const uint32_t et = block_exclusive_scan<uint32_t>(c, sm, &tot_t);
-        const uint32_t ec = block_exclusive_scan<uint32_t>(ch, sm, &tot_c);
-        if (i < P) {
-            part_off[i]    = run_t + et;
-            part_cursor[i] = run_t + et;
-            chunk_off[i]   = run_c + ec;
-        }
-        run_t += tot_t;
-        run_c += tot_c;
-    }
-    if (threadIdx.x == 0) {
-        part_off[P]  = run_t;
-        chunk_off[P] = run_c;
-    }
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(d.n_valid, (unsigned long long)mine);
+    __threadfence();
     __syncthreads();
-    for (uint32_t p = threadIdx.x; p < P; p += blockDim.x)
-        for (uint32_t c = chunk_off[p]; c < chunk_off[p + 1]; ++c) chunk_part[c] = p;
+    if (threadIdx.x == 0) last = atomicAdd(d.n_valid + 1, 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    part_offsets(d, P, sm);
 }
 
 // 3. Scatter (key, row) to partitions.  Each block owns a tile of kTile rows:
@@ -246,37 +253,51 @@ __device__ __forceinline__ uint32_t bucket_add(uint32_t* addr, uint32_t slot, un
     return atomicAdd(addr + slot, 1u);
 }
 
-// Zeroes the bucket counters and Bloom tags of the partitions cut into more
-// than one chunk (k_bucket_count accumulates those with global atomics; a
-// single-chunk partition's are stored whole, and k_bucket_local's partitions
-// use neither).  One block per partition.
-__global__ void __launch_bounds__(256)
-    k_bucket_zero(Geo g, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ part_off,
-                  uint32_t* __restrict__ gcnt, uint32_t* __restrict__ gbloom) {
-    const uint32_t part = blockIdx.x;
-    if (fused_part(part_off, part) || chunk_off[part + 1] - chunk_off[part] <= 1) return;
-    const uint32_t nl = 1u << g.L;
-    const uint64_t gb = uint64_t(part) << g.L;
+// ---- partitions above kFuseMax tuples, in phases of one kernel (k_bucket_big) ----
+// What a phase reads of an earlier one takes plain loads: other blocks of the
+// same launch wrote it (no read-only loads), and a heavy key's warps all read
+// the same words, which have to come from the L1 (from the L2, 16M tuples of
+// one key: 525 -> 676 us).
+// Most tuples of a build that takes these phases in one launch.  hj_table_build
+// before (a launch a phase) / in one launch, us: distinct keys, which have
+// nothing to do here, 300,000 78 / 51, 1M 88 / 61, 4M 151 / 132; one key only 4M
+// 194 / 188; Zipf(1.1) keys 4M 212 / 208, but 6M 290 / 299 and 16M 569 / 589, where
+// counting and comparing want more threads than the scatter's registers leave.
+constexpr uint64_t kBigOne = 1u << 22;
+struct Big {
+    Geo             g;
+    const uint32_t *chunk_off, *chunk_part, *part_off;
+    const int32_t*  tkey;
+    const uint32_t* trow;
+    uint32_t *      cnt, *bloom;  // bucket counters (then cursors) and Bloom tags
+    uint64_t*       dir;
+    int32_t*        okey;
+    uint32_t *      orow, *mixed;
+    uint64_t*       summary;
+    uint32_t*       ticket;  // the next chunk of each of the three chunk phases, zeroed
+};
+
+// Counters and Bloom tags of a partition cut into more than one chunk (its
+// chunks add to them; a single chunk's are stored whole), and the mixed bits.
+__device__ __forceinline__ void big_zero(const Big& d, uint32_t part) {
+    const uint32_t nl = 1u << d.g.L;
+    const uint64_t gb = uint64_t(part) << d.g.L;
+    const bool     many = d.chunk_off[part + 1] - d.chunk_off[part] > 1;
     for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) {
-        gcnt[gb + i]   = 0;
-        gbloom[gb + i] = 0;
+        if (many) d.cnt[gb + i] = d.bloom[gb + i] = 0;
+        if (nl >= 32 && i < nl / 32) d.mixed[(gb >> 5) + i] = 0;
     }
 }
 
 // 4. Per-chunk bucket counts and Bloom tags.
-__global__ void __launch_bounds__(kThreads)
-    k_bucket_count(Geo g, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_part,
-                   const uint32_t* __restrict__ part_off,
-                   const int32_t* __restrict__ tkey, uint32_t* __restrict__ gcnt,
-                   uint32_t* __restrict__ gbloom) {
-    extern __shared__ uint32_t sh[];
-    const uint32_t nl = 1u << g.L;
+__device__ __forceinline__ void big_count(const Big& d, uint32_t cid, uint32_t* sh) {
+    const Geo      g   = d.g;
+    const uint32_t nl  = 1u << g.L;
     uint32_t*      cnt = sh;
     uint32_t*      blm = sh + nl;
     uint32_t       part, s, e;
     bool           single;
-    if (!chunk_range(blockIdx.x, chunk_off, chunk_part, part_off, 1u << g.R, part, s, e, single)) return;
-    if (fused_part(part_off, part)) return;  // k_bucket_local
+    if (!chunk_range(cid, d.chunk_off, d.chunk_part, d.part_off, 1u << g.R, part, s, e, single)) return;
     for (uint32_t i = threadIdx.x; i < 2 * nl; i += blockDim.x) sh[i] = 0;
     __syncthreads();
     const uint32_t lmask = nl - 1;
@@ -286,7 +307,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
             const uint32_t j = b0 + uint32_t(u) * blockDim.x + threadIdx.x;
-            key[u]           = j < e ? __ldg(tkey + j) : 0;
+            key[u]           = j < e ? __ldg(d.tkey + j) : 0;
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -312,81 +333,57 @@ __global__ void __launch_bounds__(kThreads)
     const uint64_t gb = uint64_t(part) << g.L;
     for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) {
         if (single) {
-            gcnt[gb + i]   = cnt[i];
-            gbloom[gb + i] = blm[i];
+            d.cnt[gb + i]   = cnt[i];
+            d.bloom[gb + i] = blm[i];
         } else if (cnt[i]) {
-            atomicAdd(gcnt + gb + i, cnt[i]);
-            atomicOr(gbloom + gb + i, blm[i]);
+            atomicAdd(d.cnt + gb + i, cnt[i]);
+            atomicOr(d.bloom + gb + i, blm[i]);
         }
-    }
-}
+    }}
 
-// 5. Directory words.  One block per partition; gcnt becomes the scatter cursor.
-__global__ void __launch_bounds__(1024)
-    k_bucket_dir(Geo g, const uint32_t* __restrict__ part_off, uint32_t* __restrict__ gcnt,
-                 const uint32_t* __restrict__ gbloom, uint64_t* __restrict__ dir) {
-    __shared__ uint32_t sm[33];
-    const uint32_t part = blockIdx.x;
-    const uint32_t nl   = 1u << g.L;
-    const uint64_t gb   = uint64_t(part) << g.L;
-    uint32_t       run  = part_off[part];
-    if (fused_part(part_off, part)) return;  // k_bucket_local (also writes the sentinel word)
-    if (part_off[part + 1] == run) {  // empty partition: all buckets empty
-        for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) {
-            dir[gb + i]  = uint64_t(run) << 16;
-            gcnt[gb + i] = run;
+// 5. Directory words of a partition; the counters become the scatter cursors.
+__device__ __forceinline__ void big_dir(const Big& d, uint32_t part, uint32_t* sm) {
+    const uint32_t nl  = 1u << d.g.L;
+    const uint64_t gb  = uint64_t(part) << d.g.L;
+    uint32_t       run = d.part_off[part];
+    for (uint32_t base = 0; base < nl; base += blockDim.x) {
+        const uint32_t i = base + threadIdx.x;
+        const uint32_t c = i < nl ? d.cnt[gb + i] : 0;
+        uint32_t       tot;
+        const uint32_t ex = block_exclusive_scan<uint32_t>(c, sm, &tot);
+        if (i < nl) {
+            const uint32_t start = run + ex;
+            d.dir[gb + i]        = (uint64_t(start) << 16) | (d.bloom[gb + i] & 0xffffu);
+            d.cnt[gb + i]        = start;
         }
-    } else {
-        for (uint32_t base = 0; base < nl; base += blockDim.x) {
-            const uint32_t i = base + threadIdx.x;
-            const uint32_t c = i < nl ? gcnt[gb + i] : 0;
-            uint32_t       tot;
-            const uint32_t ex = block_exclusive_scan<uint32_t>(c, sm, &tot);
-            if (i < nl) {
-                const uint32_t start = run + ex;
-                dir[gb + i]          = (uint64_t(start) << 16) | (gbloom[gb + i] & 0xffffu);
-                gcnt[gb + i]         = start;
-            }
-            run += tot;
-        }
+        run += tot;
     }
 }
 
 // 6. Final scatter into bucket order.
-__global__ void __launch_bounds__(kThreads, 2)
-    k_bucket_scatter(Geo g, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_part,
-                     const uint32_t* __restrict__ part_off,
-                     const int32_t* __restrict__ tkey, const uint32_t* __restrict__ trow,
-                     uint32_t* __restrict__ cursor, int32_t* __restrict__ okey,
-                     uint32_t* __restrict__ orow) {
-    extern __shared__ uint32_t sh[];
+__device__ __forceinline__ void big_scatter(const Big& d, uint32_t cid, uint32_t* sh) {
+    const Geo      g  = d.g;
     const uint32_t nl = 1u << g.L;
     uint32_t       part, s, e;
     bool           single;
-    if (!chunk_range(blockIdx.x, chunk_off, chunk_part, part_off, 1u << g.R, part, s, e, single)) return;
-    if (fused_part(part_off, part)) return;  // k_bucket_local
+    if (!chunk_range(cid, d.chunk_off, d.chunk_part, d.part_off, 1u << g.R, part, s, e, single)) return;
     for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) sh[i] = 0;
     __syncthreads();
     const uint32_t lmask = nl - 1;
-    // a chunk is kSub tiles of kTile tuples: all are counted, then placed
-    // (a one-tile chunk keeps its keys in registers between the two)
-    constexpr int kSub = kChunk / kTile;
-    int32_t       keys[kItems];
-    for (uint32_t b0 = s; b0 < e; b0 += kTile) {
+    // the chunk's keys stay in registers between the count and the placing
+    int32_t keys[kItems];
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t j = b0 + uint32_t(k) * kThreads + threadIdx.x;
-            keys[k]          = j < e ? __ldg(tkey + j) : 0;
-            // the rows are stored after the counts: bring their lines into L1 now
-            if (kSub == 1 && j < e) asm volatile("prefetch.global.L1 [%0];" ::"l"(trow + j));
-        }
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t j = s + uint32_t(k) * kThreads + threadIdx.x;
+        keys[k]          = j < e ? __ldg(d.tkey + j) : 0;
+        // the rows are stored after the counts: bring their lines into L1 now
+        if (j < e) asm volatile("prefetch.global.L1 [%0];" ::"l"(d.trow + j));
+    }
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t j  = b0 + uint32_t(k) * kThreads + threadIdx.x;
-            const bool     ok = j < e;
-            const unsigned act = __ballot_sync(0xffffffffu, ok);
-            if (ok) bucket_add(sh, uint32_t(bucket_of(fib_hash(keys[k]), g.b)) & lmask, act);
-        }
+    for (int k = 0; k < kItems; ++k) {
+        const bool     ok  = s + uint32_t(k) * kThreads + threadIdx.x < e;
+        const unsigned act = __ballot_sync(0xffffffffu, ok);
+        if (ok) bucket_add(sh, uint32_t(bucket_of(fib_hash(keys[k]), g.b)) & lmask, act);
     }
     __syncthreads();
     const uint64_t gb = uint64_t(part) << g.L;
@@ -399,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         for (int q = 0; q < kPer; ++q) {
             const uint32_t i = threadIdx.x + uint32_t(q) * kThreads;
             const uint32_t n = i < nl ? sh[i] : 0u;
-            c[q]             = n == 0 ? 0u : (single ? cursor[gb + i] : atomicAdd(cursor + gb + i, n));
+            c[q]             = n == 0 ? 0u : (single ? d.cnt[gb + i] : atomicAdd(d.cnt + gb + i, n));
         }
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
@@ -408,24 +405,20 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
     }
     __syncthreads();
-    for (uint32_t b0 = s; b0 < e; b0 += kTile) {
-        uint32_t rows[kItems];
+    uint32_t rows[kItems];
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t j = b0 + uint32_t(k) * kThreads + threadIdx.x;
-            if (kSub > 1) keys[k] = j < e ? __ldg(tkey + j) : 0;
-            rows[k] = j < e ? __ldg(trow + j) : 0u;
-        }
+    for (int k = 0; k < kItems; ++k) {
+        const uint32_t j = s + uint32_t(k) * kThreads + threadIdx.x;
+        rows[k]          = j < e ? __ldg(d.trow + j) : 0u;
+    }
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const uint32_t j   = b0 + uint32_t(k) * kThreads + threadIdx.x;
-            const bool     ok  = j < e;
-            const unsigned act = __ballot_sync(0xffffffffu, ok);
-            if (ok) {
-                const uint32_t pos = bucket_add(sh, uint32_t(bucket_of(fib_hash(keys[k]), g.b)) & lmask, act);
-                okey[pos]          = keys[k];
-                orow[pos]          = rows[k];
-            }
+    for (int k = 0; k < kItems; ++k) {
+        const bool     ok  = s + uint32_t(k) * kThreads + threadIdx.x < e;
+        const unsigned act = __ballot_sync(0xffffffffu, ok);
+        if (ok) {
+            const uint32_t pos = bucket_add(sh, uint32_t(bucket_of(fib_hash(keys[k]), g.b)) & lmask, act);
+            d.okey[pos]        = keys[k];
+            d.orow[pos]        = rows[k];
         }
     }
 }
@@ -565,37 +558,11 @@ __global__ void __launch_bounds__(kLT, 1)
     }
 }
 
-// Bucket summaries of the partitions the chunked kernels built (the others
-// come from k_bucket_local): one block per partition.
-__global__ void __launch_bounds__(256)
-    k_bucket_summary(Geo g, const uint32_t* __restrict__ part_off, const uint64_t* __restrict__ dir,
-                     const int32_t* __restrict__ key, const uint32_t* __restrict__ row,
-                     const uint32_t* __restrict__ mixed, uint64_t* __restrict__ summary) {
-    const uint32_t part = blockIdx.x;
-    if (fused_part(part_off, part)) return;
-    const uint32_t nl = 1u << g.L;
-    const uint64_t gb = uint64_t(part) << g.L;
-    for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) {
-        const uint64_t p   = gb + i;
-        const uint64_t d0  = __ldg(dir + p);
-        const uint32_t b0  = uint32_t(d0 >> 16);
-        const uint32_t len = uint32_t(__ldg(dir + p + 1) >> 16) - b0;
-        summary[p] = len == 0 ? 0ull
-                              : make_summary(__ldg(key + b0), uint32_t(d0) & 0xffffu, len,
-                                             (__ldg(mixed + (p >> 5)) >> (p & 31)) & 1u, len == 1 ? __ldg(row + b0) : 0u);
-    }
-}
-
-// 7. mixed[p] bit set when bucket p holds two different keys (chunks of the
-//    partitions k_bucket_local does not take).
-__global__ void __launch_bounds__(kThreads)
-    k_bucket_mixed(Geo g, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ chunk_part,
-                   const uint32_t* __restrict__ part_off,
-                   const uint64_t* __restrict__ dir, const int32_t* __restrict__ key, uint32_t* __restrict__ mixed) {
+// 7. mixed[p] bit set when bucket p holds two different keys.
+__device__ __forceinline__ void big_mixed(const Big& d, uint32_t cid) {
     uint32_t part, s, e;
     bool     single;
-    if (!chunk_range(blockIdx.x, chunk_off, chunk_part, part_off, 1u << g.R, part, s, e, single)) return;
-    if (fused_part(part_off, part)) return;  // set by k_bucket_local
+    if (!chunk_range(cid, d.chunk_off, d.chunk_part, d.part_off, 1u << d.g.R, part, s, e, single)) return;
     // kMU tuples per thread at a time: keys, then directory words, then first keys
     constexpr int kMU = 8;
     for (uint32_t j0 = s + threadIdx.x; j0 < e; j0 += kMU * blockDim.x) {
@@ -604,17 +571,89 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
         for (int u = 0; u < kMU; ++u) {
             const uint32_t j = j0 + u * blockDim.x;
-            k[u]             = j < e ? key[j] : 0;
+            k[u]             = j < e ? d.okey[j] : 0;
         }
 #pragma unroll
         for (int u = 0; u < kMU; ++u) {
-            p[u]     = uint32_t(bucket_of(fib_hash(k[u]), g.b));
-            first[u] = j0 + u * blockDim.x < e ? uint32_t(__ldg(dir + p[u]) >> 16) : 0u;
+            p[u]     = uint32_t(bucket_of(fib_hash(k[u]), d.g.b));
+            first[u] = j0 + u * blockDim.x < e ? uint32_t(d.dir[p[u]] >> 16) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < kMU; ++u)
-            if (j0 + u * blockDim.x < e && key[first[u]] != k[u]) atomicOr(mixed + (p[u] >> 5), 1u << (p[u] & 31));
+            if (j0 + u * blockDim.x < e && d.okey[first[u]] != k[u])
+                atomicOr(d.mixed + (p[u] >> 5), 1u << (p[u] & 31));
     }
+}
+
+// Bucket summaries of a partition (those of the others come from k_bucket_local).
+__device__ __forceinline__ void big_summary(const Big& d, uint32_t part) {
+    const uint32_t nl = 1u << d.g.L;
+    const uint64_t gb = uint64_t(part) << d.g.L;
+    for (uint32_t i = threadIdx.x; i < nl; i += blockDim.x) {
+        const uint64_t p   = gb + i;
+        const uint64_t d0  = d.dir[p];
+        const uint32_t b0  = uint32_t(d0 >> 16);
+        const uint32_t len = uint32_t(d.dir[p + 1] >> 16) - b0;
+        d.summary[p] = len == 0 ? 0ull
+                                : make_summary(d.okey[b0], uint32_t(d0) & 0xffffu, len,
+                                               (d.mixed[(p >> 5)] >> (p & 31)) & 1u,
+                                               len == 1 ? d.orow[b0] : 0u);
+    }
+}
+
+// 4-7 for the partitions that k_bucket_local leaves, after it: one cooperative
+// launch (its blocks are resident together, so that they can wait for each
+// other between the phases), which returns at once when there are none, as
+// for most builds; six launches that found nothing to do took 1.6 us each on
+// the GPU and some 2.7 us each on the host.
+constexpr int kBigBlocks = 2;  // per SM
+__global__ void __launch_bounds__(kThreads, kBigBlocks) k_bucket_big(Big d) {
+    extern __shared__ uint32_t sh[];
+    __shared__ uint32_t        sm[33];
+    const uint32_t P = 1u << d.g.R, nc = d.chunk_off[P];
+    if (nc == 0) return;
+    const auto grid  = cooperative_groups::this_grid();
+    auto       parts = [&](auto f) {
+        for (uint32_t p = blockIdx.x; p < P; p += gridDim.x)
+            if (!fused_part(d.part_off, p)) f(p);
+    };
+    // chunks go to whichever block is free: the first by its index, the others by tickets
+    __shared__ uint32_t next;
+    auto                chunks = [&](uint32_t* ticket, auto f) {
+        for (uint32_t c = blockIdx.x; c < nc;) {
+            f(c);
+            __syncthreads();
+            if (threadIdx.x == 0) next = gridDim.x + atomicAdd(ticket, 1u);
+            __syncthreads();
+            c = next;
+        }
+    };
+    parts([&](uint32_t p) { big_zero(d, p); });
+    grid.sync();
+    chunks(d.ticket + 0, [&](uint32_t c) { big_count(d, c, sh); });
+    grid.sync();
+    parts([&](uint32_t p) { big_dir(d, p, sm); });
+    grid.sync();
+    chunks(d.ticket + 1, [&](uint32_t c) { big_scatter(d, c, sh); });
+    grid.sync();
+    chunks(d.ticket + 2, [&](uint32_t c) { big_mixed(d, c); });
+    grid.sync();
+    parts([&](uint32_t p) { big_summary(d, p); });
+}
+
+// The same phases as a launch each, with as many blocks as a phase has chunks
+// or partitions and (but for the scatter) twice the threads on an SM.
+template <int PHASE>
+__global__ void __launch_bounds__(kThreads, PHASE == 3 ? 2 : 4) k_bucket_phase(Big d) {
+    extern __shared__ uint32_t sh[];
+    __shared__ uint32_t        sm[33];
+    if (PHASE == 1) return big_count(d, blockIdx.x, sh);
+    if (PHASE == 3) return big_scatter(d, blockIdx.x, sh);
+    if (PHASE == 4) return big_mixed(d, blockIdx.x);
+    if (fused_part(d.part_off, blockIdx.x)) return;
+    if (PHASE == 0) big_zero(d, blockIdx.x);
+    if (PHASE == 2) big_dir(d, blockIdx.x, sm);
+    if (PHASE == 5) big_summary(d, blockIdx.x);
 }
 
 // Small builds in one launch: every block owns one partition of the directory
@@ -920,57 +959,59 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
         prefer_shared(k_part_hist);
         prefer_shared(k_part_scatter<1024>);
         prefer_shared(k_part_scatter<kThreads>);
-        prefer_shared(k_bucket_count);
-        prefer_shared(k_bucket_scatter);
+        prefer_shared(k_bucket_big);
+        prefer_shared(k_bucket_phase<1>);
+        prefer_shared(k_bucket_phase<3>);
         prefer_shared(k_bucket_local);
         max_dynamic_smem(k_part_hist, sizeof(uint32_t) << kMaxRadix);
         max_dynamic_smem(k_part_scatter<1024>, 200 * 1024);
         max_dynamic_smem(k_part_scatter<kThreads>, (8u << kMaxRadix) + size_t(kTile) * 10);
-        max_dynamic_smem(k_bucket_count, 8u << kLocalBits);
         max_dynamic_smem(k_bucket_local, local_smem(kLocalBits));
-        max_dynamic_smem(k_bucket_scatter, 4u << kLocalBits);
+        max_dynamic_smem(k_bucket_big, 8u << kLocalBits);
     });
-    unsigned long long* d_nvalid = dalloc_n<unsigned long long>(1, st);
-    uint32_t*           part_cnt = nullptr;
+    // counters that start at zero in one piece: valid keys, finished blocks, partition sizes
+    Parts d{};
+    auto  free_parts = [&] {
+        for (void* p : {(void*)d.n_valid, (void*)d.off, (void*)d.cursor, (void*)d.chunk_off, (void*)d.chunk_part})
+            dfree(p, st);
+    };
+    // chunks of the partitions above kFuseMax tuples, at most
+    const uint64_t n_most       = n_valid >= 0 ? uint64_t(n_valid) : kc.n;
+    const uint64_t chunks_upper = (n_most + kChunk - 1) / kChunk + n_most / kFuseMax + 1;
     auto run_hist = [&](uint32_t r) {
         const uint32_t P = 1u << r;
-        part_cnt         = dalloc_n<uint32_t>(P, st);
-        HJ_CUDA(cudaMemsetAsync(part_cnt, 0, P * sizeof(uint32_t), st));
-        HJ_CUDA(cudaMemsetAsync(d_nvalid, 0, sizeof(unsigned long long), st));
+        const size_t   z = 4 * sizeof(unsigned long long) + P * sizeof(uint32_t);
+        d.n_valid        = reinterpret_cast<unsigned long long*>(dalloc_n<uint8_t>(z, st));
+        d.cnt            = reinterpret_cast<uint32_t*>(d.n_valid + 4);
+        d.off            = dalloc_n<uint32_t>(P + 1, st);
+        d.cursor         = dalloc_n<uint32_t>(P, st);
+        d.chunk_off      = dalloc_n<uint32_t>(P + 1, st);
+        d.chunk_part     = dalloc_n<uint32_t>(chunks_upper, st);
+        HJ_CUDA(cudaMemsetAsync(d.n_valid, 0, z, st));
         const size_t smem = P * sizeof(uint32_t);
-        k_part_hist<<<grid_for(kc.n, kThreads), kThreads, smem, st>>>(kc, r, part_cnt, d_nvalid);
+        k_part_hist<<<grid_for(kc.n, kThreads), kThreads, smem, st>>>(kc, r, d);
         HJ_LAUNCH_CHECK();
         if (n_valid < 0) {
-            readback(scratch_host, d_nvalid, sizeof(uint64_t), true, st);  // page-locked scratch
+            readback(scratch_host, d.n_valid, sizeof(uint64_t), true, st);  // page-locked scratch
             HJ_CUDA(cudaStreamSynchronize(st));
         }
     };
     run_hist(R);
     const uint64_t nv = n_valid >= 0 ? uint64_t(n_valid) : scratch_host[0];
     if (nv == 0) {  // UnchainedHash with no tuples: no directory, every probe misses
-        dfree(part_cnt, st);
-        dfree(d_nvalid, st);
+        free_parts();
         return;
     }
     if (nv > 0xffffffffull) throw Error(HJ_ERR_INVALID, "more than 2^32 build tuples");
     const uint32_t b = dir_bits >= 0 ? uint32_t(dir_bits) : std::min(cap, ceil_log2(nv));
     if (R > b) {  // NULLs shrank the directory below the partition fan-out
-        dfree(part_cnt, st);
+        free_parts();
         R = b;
         run_hist(R);
     }
     if (b - R > kLocalBits) throw Error(HJ_ERR_INVALID, "radix_bits too small for the directory");
     const Geo      g{b, R, b - R};
     const uint32_t P = 1u << R;
-
-    uint32_t* part_off    = dalloc_n<uint32_t>(P + 1, st);
-    uint32_t* part_cursor = dalloc_n<uint32_t>(P, st);
-    uint32_t* chunk_off   = dalloc_n<uint32_t>(P + 1, st);
-    // chunks of the partitions above kFuseMax tuples, at most
-    const unsigned chunks_upper = unsigned((nv + kChunk - 1) / kChunk + nv / kFuseMax + 1);
-    uint32_t*      chunk_part   = dalloc_n<uint32_t>(chunks_upper, st);
-    k_part_offsets<<<1, 1024, 0, st>>>(part_cnt, P, part_off, part_cursor, chunk_off, chunk_part);
-    HJ_LAUNCH_CHECK();
 
     int32_t*  tkey = dalloc_n<int32_t>(nv, st);
     uint32_t* trow = dalloc_n<uint32_t>(nv, st);
@@ -980,10 +1021,10 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
         auto smem_for = [&](size_t tile) { return (2 * size_t(P) + 2 * tile) * sizeof(uint32_t) + tile * sizeof(uint16_t); };
         const size_t big = smem_for(size_t(1024) * kItems);
         if (big <= 200 * 1024) {
-            k_part_scatter<1024><<<div_up(kc.n, 1024 * kItems), 1024, big, st>>>(kc, R, part_cursor, tkey, trow);
+            k_part_scatter<1024><<<div_up(kc.n, 1024 * kItems), 1024, big, st>>>(kc, R, d.cursor, tkey, trow);
         } else {
             const size_t smem = smem_for(kTile);
-            k_part_scatter<kThreads><<<div_up(kc.n, kTile), kThreads, smem, st>>>(kc, R, part_cursor, tkey, trow);
+            k_part_scatter<kThreads><<<div_up(kc.n, kTile), kThreads, smem, st>>>(kc, R, d.cursor, tkey, trow);
         }
         HJ_LAUNCH_CHECK();
     }
@@ -992,38 +1033,37 @@ void build_table(const KeyCol& kc, int dir_bits, int radix_bits, Table& t, uint6
     alloc_table(t, b, nv, st);
     uint32_t* gcnt        = dalloc_n<uint32_t>(nb, st);
     uint32_t* gbloom      = dalloc_n<uint32_t>(nb, st);
-    HJ_CUDA(cudaMemsetAsync(t.mixed, 0, ((nb + 31) / 32) * sizeof(uint32_t), st));
-    k_bucket_zero<<<P, 256, 0, st>>>(g, chunk_off, part_off, gcnt, gbloom);
+    // partitions of less than a word of mixed bits share one
+    if (g.L < 5) HJ_CUDA(cudaMemsetAsync(t.mixed, 0, ((nb + 31) / 32) * sizeof(uint32_t), st));
+    k_bucket_local<<<std::min<uint32_t>(P, uint32_t(num_sms())), kLT, local_smem(g.L), st>>>(
+        g, d.off, tkey, trow, t.dir, t.keys, t.rows, t.mixed, t.summary);
     HJ_LAUNCH_CHECK();
+    if (nv > kFuseMax) {  // (else no partition is larger)
+        Big          big{g, d.chunk_off, d.chunk_part, d.off, tkey, trow, gcnt, gbloom, t.dir, t.keys, t.rows, t.mixed, t.summary,
+                         reinterpret_cast<uint32_t*>(d.n_valid + 2)};
+        if (nv <= kBigOne) {
+            void*          args[] = {&big};
+            const uint64_t grid   = std::min<uint64_t>(std::max<uint64_t>(P, chunks_upper), kBigBlocks * uint64_t(num_sms()));
+            HJ_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(k_bucket_big), dim3(unsigned(grid)),
+                                                dim3(kThreads), args, 8u << g.L, st));
+            HJ_LAUNCH_CHECK();
+        } else {
+            const unsigned nc = unsigned((nv + kChunk - 1) / kChunk + nv / kFuseMax + 1);
+            auto           go = [&](auto kernel, unsigned blocks, size_t smem) {
+                kernel<<<blocks, kThreads, smem, st>>>(big);
+                HJ_LAUNCH_CHECK();
+            };
+            go(k_bucket_phase<0>, P, 0);
+            go(k_bucket_phase<1>, nc, 8u << g.L);
+            go(k_bucket_phase<2>, P, 0);
+            go(k_bucket_phase<3>, nc, 4u << g.L);
+            go(k_bucket_phase<4>, nc, 0);
+            go(k_bucket_phase<5>, P, 0);
+        }
+    }
 
-    {
-        const size_t smem = 2 * (size_t(1) << g.L) * sizeof(uint32_t);
-        k_bucket_count<<<chunks_upper, kThreads, smem, st>>>(g, chunk_off, chunk_part, part_off, tkey, gcnt, gbloom);
-        HJ_LAUNCH_CHECK();
-    }
-    k_bucket_dir<<<P, 1024, 0, st>>>(g, part_off, gcnt, gbloom, t.dir);
-    HJ_LAUNCH_CHECK();
-    {
-        const size_t smem = local_smem(g.L);
-        k_bucket_local<<<std::min<uint32_t>(P, uint32_t(num_sms())), kLT, smem, st>>>(g, part_off, tkey, trow, t.dir,
-                                                                                t.keys, t.rows, t.mixed,
-                                                                                t.summary);
-        HJ_LAUNCH_CHECK();
-    }
-    {
-        const size_t smem = (size_t(1) << g.L) * sizeof(uint32_t);
-        k_bucket_scatter<<<chunks_upper, kThreads, smem, st>>>(g, chunk_off, chunk_part, part_off, tkey, trow, gcnt,
-                                                              t.keys, t.rows);
-        HJ_LAUNCH_CHECK();
-    }
-    k_bucket_mixed<<<chunks_upper, kThreads, 0, st>>>(g, chunk_off, chunk_part, part_off, t.dir, t.keys, t.mixed);
-    HJ_LAUNCH_CHECK();
-    k_bucket_summary<<<P, 256, 0, st>>>(g, part_off, t.dir, t.keys, t.rows, t.mixed, t.summary);
-    HJ_LAUNCH_CHECK();
-
-    for (void* p : {(void*)d_nvalid, (void*)part_cnt, (void*)part_off, (void*)part_cursor,
-                    (void*)chunk_off, (void*)chunk_part, (void*)tkey, (void*)trow, (void*)gcnt, (void*)gbloom})
-        dfree(p, st);
+    free_parts();
+    for (void* p : {(void*)tkey, (void*)trow, (void*)gcnt, (void*)gbloom}) dfree(p, st);
 }
 
 void free_table(Table& t, cudaStream_t st) {
