@@ -408,6 +408,7 @@ namespace {
 thread_local std::string g_create_error;
 
 constexpr size_t kSlot = 64ull << 20;  // pinned staging slot (two slots)
+constexpr size_t kPinnedWords = 64;    // page-locked scratch for small readbacks
 
 void ensure_staging(hj_context* c) {
     if (c->staging) return;
@@ -966,13 +967,7 @@ struct Exec {
     void materialize(const Inter& in, const hj_node_desc& root, hj_result* res) {
         phase("materialize");
         res->cols.assign(root.num_attrs, hj_result::Col{0, 0, nullptr});
-        struct IntOut {
-            uint32_t        a;
-            IntCol          col;
-            const uint32_t* rid;
-            uint64_t        rows;
-        };
-        std::vector<IntOut>                          iout;  // written after the VARCHAR page counts are known
+        std::vector<IntPages>                        iout;  // written after the VARCHAR page counts are known
         std::vector<std::pair<uint32_t, VarcharOut>> vout;  // (column, plan)
         for (uint32_t a = 0; a < root.num_attrs; ++a) {
             const ColRef&   cr  = in.cols[a];
@@ -997,7 +992,7 @@ struct Exec {
                 }
                 oc.num_pages = (rows + kDenseRows - 1) / kDenseRows;
                 oc.pages     = make_buf(oc.num_pages * kPage, c->st);  // allocated while earlier work runs
-                iout.push_back({a, col, rid, rows});
+                iout.push_back(IntPages{col, rid, rows, oc.pages->as<uint8_t>()});
             } else if (ty == HJ_VARCHAR) {
                 VarcharOut v{};
                 if (d.type == HJ_INT32) {
@@ -1015,32 +1010,36 @@ struct Exec {
                 vout.emplace_back(a, v);
             }
         }
-        std::vector<VarcharOut*> vptr;
-        for (auto& kv : vout) vptr.push_back(&kv.second);
-        if (!vout.empty()) {
-            phase("mat_varchar_plan");
-            varchar_plan(vptr, c->st);
+        std::vector<VarcharOut*> vptr, part;
+        std::vector<uint64_t>    vpages;
+        if (!vout.empty()) phase("mat_varchar_plan");
+        for (auto& kv : vout) {
+            if (part.size() == kPinnedWords) {  // the page-locked scratch is full: its counts are waited for
+                varchar_plan(part, c->st);
+                HJ_CUDA(cudaStreamSynchronize(c->st));
+                vpages.insert(vpages.end(), c->pinned, c->pinned + part.size());
+                part.clear();
+            }
+            kv.second.host_pages = c->pinned + part.size();
+            part.push_back(&kv.second);
+            vptr.push_back(&kv.second);
         }
-        std::vector<uint64_t> vpages;
+        if (!part.empty()) varchar_plan(part, c->st);
         cudaEvent_t           counted = nullptr;
-        if (!vout.empty()) {  // one readback for the page counts of every VARCHAR column
+        if (!vout.empty()) {  // the page counts of every VARCHAR column are on their way
             phase("mat_sync");
-            for (size_t i = 0; i < vout.size(); ++i)
-                readback(c->pinned + i, vout[i].second.tile_off + vout[i].second.ntiles, sizeof(uint64_t), true,
-                         c->st);  // page-locked scratch
             HJ_CUDA(cudaEventCreateWithFlags(&counted, cudaEventDisableTiming));
             HJ_CUDA(cudaEventRecord(counted, c->st));
         }
         // the INT32 pages keep the GPU busy while the host waits for the page
         // counts and sizes the VARCHAR buffers
         phase("materialize");
-        for (const IntOut& o : iout)
-            launch_write_int32_pages(o.col, o.rid, o.rows, res->cols[o.a].pages->as<uint8_t>(), c->st);
+        launch_write_int32_pages(iout, c->st);
         if (counted) {
             const cudaError_t e = cudaEventSynchronize(counted);
             cudaEventDestroy(counted);
             HJ_CUDA(e);
-            vpages.assign(c->pinned, c->pinned + vout.size());
+            vpages.insert(vpages.end(), c->pinned, c->pinned + part.size());
         }
         if (!vout.empty()) {
             phase("mat_varchar_write");
@@ -1158,7 +1157,7 @@ hj_context* hj_context_create(int device) {
         HJ_CUDA(cudaDeviceGetDefaultMemPool(&mp, device));
         uint64_t keep = ~0ull;  // keep freed blocks for reuse
         HJ_CUDA(cudaMemPoolSetAttribute(mp, cudaMemPoolAttrReleaseThreshold, &keep));
-        HJ_CUDA(cudaMallocHost(&c->pinned, 64 * sizeof(uint64_t)));
+        HJ_CUDA(cudaMallocHost(&c->pinned, hj::kPinnedWords * sizeof(uint64_t)));
         HJ_CUDA(cudaMalloc(&c->counters, 8 * sizeof(uint64_t)));
         HJ_CUDA(cudaMemsetAsync(c->counters, 0, 8 * sizeof(uint64_t), c->st));
         int pageable = 0;

@@ -166,15 +166,20 @@ int    probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& p
 
 // ---- output pages (hj_materialize.cu) --------------------------------------
 // INT32 output column of n rows gathered through rid (nullptr = identity) from a
-// base column; writes ceil(n / 1984) pages.
-void launch_write_int32_pages(const IntCol& col, const uint32_t* rid, uint64_t n, uint8_t* out_pages,
-                              cudaStream_t st);
+// base column: ceil(n / 1984) pages.  Several columns share a launch.
+struct IntPages {
+    IntCol          col;
+    const uint32_t* rid;
+    uint64_t        n;
+    uint8_t*        out;
+};
+void launch_write_int32_pages(const std::vector<IntPages>& cols, cudaStream_t st);
 
 struct PageDesc;  // one output page of a VARCHAR column (hj_materialize.cu)
 
 // VARCHAR output columns in two steps, so that several columns share one
 // host synchronisation: plan (gather locators, pack pages, count them into
-// *page_count, a device word) then write (after the caller read the counts).
+// *host_pages) then write (after the caller waited for the counts).
 struct VarcharOut {
     const uint64_t* locs;        // locators of the base column
     const uint8_t*  base;        // its pages
@@ -188,10 +193,13 @@ struct VarcharOut {
     uint64_t        ntiles     = 0;
     PageDesc*       desc       = nullptr;  // varchar_write's page descriptors
     uint64_t*       recs       = nullptr;  // page starts per tile (packing scratch)
+    uint64_t*       host_pages = nullptr;  // where the page count goes (page-locked; set by the caller)
+    uint64_t        pages      = 0;        // varchar_write: the page count
+    uint8_t*        out        = nullptr;  // and the pages
 };
-// All VARCHAR columns of a result at once (their packing kernels share launches).
+// All VARCHAR columns of a result at once (their kernels share launches).
 void varchar_plan(std::vector<VarcharOut*>& vs, cudaStream_t st);
-// pages[i] = vs[i]->tile_off[ntiles] as read by the caller; returns the page buffers.
+// pages[i] = *vs[i]->host_pages, which the caller waited for; returns the page buffers.
 std::vector<uint8_t*> varchar_write(std::vector<VarcharOut*>& vs, const std::vector<uint64_t>& pages,
                                     cudaStream_t st);
 

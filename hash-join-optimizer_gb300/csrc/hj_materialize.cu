@@ -70,15 +70,34 @@ __device__ __forceinline__ void put_bits(uint8_t* img, uint32_t bm0, uint32_t nb
 constexpr int kIntRows = 8;
 static_assert(kMT * kIntRows >= kDenseRows, "one pass per page");
 
-__global__ void __launch_bounds__(kMT)
-    k_write_int32_pages(IntCol col, const uint32_t* __restrict__ rid, uint64_t n, uint8_t* __restrict__ out) {
+// The INT32 output columns of one materialisation share launches, as the
+// VARCHAR ones do: page q of the launch is page q - page0 of its column.  A
+// result of few pages is bound by the latency of each launch (5-8 us for one
+// page), a large one by the last wave of each: with a launch a column a
+// five-relation chain took 480 us, so 372; a join of 16M x 25.6M rows with six
+// columns 2.63 ms, so 2.52.
+constexpr int kMaxIntCols = 16;
+struct IntPagesOf {
+    IntPages c;
+    uint64_t page0;
+};
+struct IntCols {
+    int        n;
+    IntPagesOf c[kMaxIntCols];
+};
+
+__global__ void __launch_bounds__(kMT) k_write_int32_pages(IntCols cols, uint64_t npages) {
     __shared__ __align__(16) uint8_t img[kPage];
     __shared__ uint32_t              sm[33];
-    const bool     nullable = col.tagged != nullptr || col.valid != nullptr;
-    uint32_t*      words    = reinterpret_cast<uint32_t*>(img);
-    const uint64_t npg      = (n + kDenseRows - 1) / kDenseRows;
-    for (uint64_t p = blockIdx.x; p < npg; p += gridDim.x) {
-        const uint64_t r0 = p * kDenseRows;
+    uint32_t*                        words = reinterpret_cast<uint32_t*>(img);
+    int                              ci    = 0;
+    for (uint64_t q = blockIdx.x; q < npages; q += gridDim.x) {
+        while (ci + 1 < cols.n && cols.c[ci + 1].page0 <= q) ++ci;
+        const IntCol&                col      = cols.c[ci].c.col;
+        const uint32_t* __restrict__ rid      = cols.c[ci].c.rid;
+        const uint64_t               n        = cols.c[ci].c.n;
+        const bool                   nullable = col.tagged != nullptr || col.valid != nullptr;
+        const uint64_t p = q - cols.c[ci].page0, r0 = p * kDenseRows;
         const uint32_t nr = uint32_t(n - r0 < uint64_t(kDenseRows) ? n - r0 : uint64_t(kDenseRows));
         zero_img(img);
         const uint32_t i0 = threadIdx.x * kIntRows;
@@ -102,15 +121,15 @@ __global__ void __launch_bounds__(kMT)
             tot = nr;
             __syncthreads();  // the image is zeroed
         }
-        uint32_t q = rank;
+        uint32_t at = rank;
 #pragma unroll
         for (int k = 0; k < kIntRows; ++k)
-            if ((on >> k) & 1u) words[1 + q++] = uint32_t(v[k]);
+            if ((on >> k) & 1u) words[1 + at++] = uint32_t(v[k]);
         const uint32_t nbytes = (nr + 7) / 8;
         if (i0 < nr) img[kPage - nbytes + threadIdx.x] = uint8_t(on);
         if (threadIdx.x == 0) words[0] = nr | (tot << 16);
         __syncthreads();
-        store_page(out + p * kPage, img);
+        store_page(cols.c[ci].c.out + p * kPage, img);
         __syncthreads();
     }
 }
@@ -204,9 +223,12 @@ struct PackCol {
     const uint8_t*  base;
     uint64_t        npages, n, ntiles, tile_base;
     uint32_t*       tile_pages;
-    const uint64_t* tile_off;
+    uint64_t*       tile_off;
     PageDesc*       desc;
-    uint64_t*       recs;  // kRec page-start records per tile
+    uint64_t*       recs;        // kRec page-start records per tile
+    uint64_t*       host_pages;  // the column's page count, in page-locked memory
+    uint64_t        pages, page0;  // of the page writer: pages of the column, and of those before it
+    uint8_t*        out;
 };
 struct PackCols {
     int     n;
@@ -494,17 +516,22 @@ __device__ __forceinline__ void page_sync(unsigned slot) {
     if (kVWP > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(32 * kVWP) : "memory");
 }
 
-__global__ void __launch_bounds__(kVT, kVMin)
-    k_write_varchar_pages(const PageDesc* __restrict__ desc, uint64_t ndesc, const uint64_t* __restrict__ ol,
-                          const uint8_t* __restrict__ base, uint64_t npages, uint8_t* __restrict__ out) {
+__global__ void __launch_bounds__(kVT, kVMin) k_write_varchar_pages(PackCols P, uint64_t ndesc) {
     extern __shared__ __align__(16) uint8_t vimg[];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned slot = warp / kVWP, part = warp % kVWP;
     uint8_t*       img  = vimg + size_t(slot) * kPage;
     constexpr int  kQ   = kPage / 16 / (32 * kVWP);  // 16-byte words per lane of a part's share
     uint4*         w4   = reinterpret_cast<uint4*>(img) + part * 32 * kQ;  // this part's share of the image
-    for (uint64_t pi = uint64_t(blockIdx.x) * kVPB + slot; pi < ndesc; pi += uint64_t(gridDim.x) * kVPB) {
-        const PageDesc d = desc[pi];
+    int            ci   = 0;
+    for (uint64_t pg0 = uint64_t(blockIdx.x) * kVPB + slot; pg0 < ndesc; pg0 += uint64_t(gridDim.x) * kVPB) {
+        while (ci + 1 < P.n && P.c[ci + 1].page0 <= pg0) ++ci;
+        const PackCol&              v      = P.c[ci];
+        const uint64_t              pi     = pg0 - v.page0;
+        const uint64_t* __restrict__ ol    = v.ol;
+        const uint8_t* __restrict__ base   = v.base;
+        const uint64_t              npages = v.npages;
+        const PageDesc              d      = v.desc[pi];
 #pragma unroll
         for (int k = 0; k < kQ; ++k) w4[lane + 32 * k] = make_uint4(0, 0, 0, 0);
         page_sync(slot);  // strings may cross into the other parts' shares
@@ -550,10 +577,10 @@ __global__ void __launch_bounds__(kVT, kVMin)
                 next               = c + 32 + lane < r1 ? ol[d.row + c + 32 + lane] : 0;
                 const bool     on  = loc != 0;
                 const uint32_t len = on ? uint32_t(loc_len_field(loc)) : 0u;
-                const uint32_t v    = (on ? 0x10000u : 0u) | len;
-                const uint32_t inc  = warp_inclusive_scan<uint32_t>(v);
+                const uint32_t x    = (on ? 0x10000u : 0u) | len;
+                const uint32_t inc  = warp_inclusive_scan<uint32_t>(x);
                 const uint32_t tot  = __shfl_sync(0xffffffffu, inc, 31);
-                const uint32_t ex   = inc - v;
+                const uint32_t ex   = inc - x;
                 const uint32_t rank = rank0 + (ex >> 16);
                 const uint32_t boff = byte0 + (ex & 0xffffu);
                 // the packer guarantees both bounds; they are checked so that no
@@ -575,9 +602,37 @@ __global__ void __launch_bounds__(kVT, kVMin)
         page_sync(slot);  // image complete
         // each part stores its own share; the next page zeroes only that
         // share, and its first barrier orders the other parts' writes after
-        uint4* dst = reinterpret_cast<uint4*>(out + pi * kPage) + part * 32 * kQ;
+        uint4* dst = reinterpret_cast<uint4*>(P.c[ci].out + pi * kPage) + part * 32 * kQ;
 #pragma unroll
         for (int k = 0; k < kQ; ++k) dst[lane + 32 * k] = w4[lane + 32 * k];
+    }
+}
+
+// First page of each tile, and the column's page count to the host: a block per column.
+constexpr int kOffT = 1024, kOffU = 4;
+__global__ void __launch_bounds__(kOffT) k_pack_offsets(PackCols P) {
+    __shared__ uint32_t sm[33];
+    const PackCol&      v   = P.c[blockIdx.x];
+    uint64_t            run = 0;
+    for (uint64_t t0 = 0; t0 < v.ntiles; t0 += kOffT * kOffU) {
+        const uint64_t t = t0 + threadIdx.x * kOffU;
+        uint32_t       c[kOffU], sum = 0, tot;
+#pragma unroll
+        for (int k = 0; k < kOffU; ++k) {
+            c[k] = t + k < v.ntiles ? v.tile_pages[t + k] : 0u;
+            sum += c[k];
+        }
+        uint64_t at = run + block_exclusive_scan<uint32_t>(sum, sm, &tot);
+#pragma unroll
+        for (int k = 0; k < kOffU; ++k) {
+            if (t + k < v.ntiles) v.tile_off[t + k] = at;
+            at += c[k];
+        }
+        run += tot;
+    }
+    if (threadIdx.x == 0) {
+        v.tile_off[v.ntiles] = run;
+        *v.host_pages        = run;
     }
 }
 
@@ -587,12 +642,19 @@ unsigned grid_of(uint64_t items, uint64_t per_sm = 16) {
 
 }  // namespace
 
-void launch_write_int32_pages(const IntCol& col, const uint32_t* rid, uint64_t n, uint8_t* out_pages,
-                              cudaStream_t st) {
-    if (n == 0) return;
-    const uint64_t pages = (n + kDenseRows - 1) / kDenseRows;
-    k_write_int32_pages<<<grid_of(pages), kMT, 0, st>>>(col, rid, n, out_pages);
-    HJ_LAUNCH_CHECK();
+void launch_write_int32_pages(const std::vector<IntPages>& cols, cudaStream_t st) {
+    for (size_t g0 = 0; g0 < cols.size(); g0 += kMaxIntCols) {
+        IntCols  G{};
+        uint64_t pages = 0;
+        for (size_t i = g0; i < std::min(cols.size(), g0 + kMaxIntCols); ++i) {
+            if (cols[i].n == 0) continue;
+            G.c[G.n++] = IntPagesOf{cols[i], pages};
+            pages += (cols[i].n + kDenseRows - 1) / kDenseRows;
+        }
+        if (pages == 0) continue;
+        k_write_int32_pages<<<grid_of(pages), kMT, 0, st>>>(G, pages);
+        HJ_LAUNCH_CHECK();
+    }
 }
 
 namespace {
@@ -604,14 +666,15 @@ void for_pack_groups(std::vector<VarcharOut*>& vs, F&& f) {
         if (v->n) live.push_back(v);
     for (size_t g0 = 0; g0 < live.size(); g0 += kMaxPackCols) {
         PackCols P{};
-        uint64_t tiles = 0;
+        uint64_t tiles = 0, pages = 0;
         for (size_t i = g0; i < std::min(live.size(), g0 + kMaxPackCols); ++i) {
             VarcharOut& v = *live[i];
             P.c[P.n++]    = PackCol{v.locs, v.rid, v.ol, v.base, v.base_pages, v.n, v.ntiles, tiles,
-                                 v.tile_pages, v.tile_off, v.desc, v.recs};
+                                 v.tile_pages, v.tile_off, v.desc, v.recs, v.host_pages, v.pages, pages, v.out};
             tiles += v.ntiles;
+            pages += v.pages;
         }
-        f(P, tiles);
+        f(P, tiles, pages);
     }
 }
 }  // namespace
@@ -626,32 +689,33 @@ void varchar_plan(std::vector<VarcharOut*>& vs, cudaStream_t st) {
         v.tile_off   = dalloc_n<uint64_t>(v.ntiles + 1, st);
         v.recs       = dalloc_n<uint64_t>(v.ntiles * kRec, st);
     }
-    for_pack_groups(vs, [&](const PackCols& P, uint64_t tiles) {
+    for_pack_groups(vs, [&](const PackCols& P, uint64_t tiles, uint64_t) {
         k_pack_count<<<grid_of(tiles, 4), kPackT, 0, st>>>(P, tiles);
         HJ_LAUNCH_CHECK();
+        k_pack_offsets<<<P.n, kOffT, 0, st>>>(P);
+        HJ_LAUNCH_CHECK();
     });
-    for (auto* vp : vs)
-        if (vp->n) scan_exclusive_u32_to_u64(vp->tile_pages, vp->tile_off, vp->ntiles, st);
 }
 
 std::vector<uint8_t*> varchar_write(std::vector<VarcharOut*>& vs, const std::vector<uint64_t>& pages,
                                     cudaStream_t st) {
     std::vector<uint8_t*> out(vs.size(), nullptr);
-    for (size_t i = 0; i < vs.size(); ++i)
-        if (vs[i]->n) vs[i]->desc = static_cast<PageDesc*>(dalloc(std::max<uint64_t>(pages[i], 1) * sizeof(PageDesc), st));
-    for_pack_groups(vs, [&](const PackCols& P, uint64_t tiles) {
+    for (size_t i = 0; i < vs.size(); ++i) {
+        VarcharOut& v = *vs[i];
+        if (v.n == 0) continue;
+        v.pages = pages[i];
+        v.desc  = static_cast<PageDesc*>(dalloc(std::max<uint64_t>(pages[i], 1) * sizeof(PageDesc), st));
+        v.out = out[i] = static_cast<uint8_t*>(dalloc(std::max<uint64_t>(pages[i], 1) * kPage, st));
+    }
+    for_pack_groups(vs, [&](const PackCols& P, uint64_t tiles, uint64_t npages) {
         k_pack_emit<<<div_up(tiles * 32, 256), 256, 0, st>>>(P, tiles);
+        HJ_LAUNCH_CHECK();
+        k_write_varchar_pages<<<grid_of(div_up(npages, kVPB), kVMin), kVT, kVPB * kPage, st>>>(P, npages);
         HJ_LAUNCH_CHECK();
     });
     for (size_t i = 0; i < vs.size(); ++i) {
         VarcharOut& v = *vs[i];
         if (v.n == 0) continue;
-        out[i] = static_cast<uint8_t*>(dalloc(std::max<uint64_t>(pages[i], 1) * kPage, st));
-        HJ_CUDA(cudaFuncSetAttribute(k_write_varchar_pages, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kVPB * kPage));
-        k_write_varchar_pages<<<grid_of(div_up(pages[i], kVPB), kVMin), kVT, kVPB * kPage, st>>>(
-            v.desc, pages[i], v.ol, v.base, v.base_pages, out[i]);
-        HJ_LAUNCH_CHECK();
         for (void* p : {(void*)v.desc, (void*)v.ol, (void*)v.tile_pages, (void*)v.tile_off, (void*)v.recs})
             dfree(p, st);
         v.desc       = nullptr;
