@@ -143,76 +143,110 @@ __device__ __forceinline__ uint64_t global_warp() {
 }
 __device__ __forceinline__ uint64_t total_warps() { return (uint64_t(gridDim.x) * blockDim.x) >> 5; }
 
-__global__ void __launch_bounds__(kDecThreads)
-    k_decode_int32_tagged(const uint8_t* __restrict__ pages, uint64_t num_pages,
-                          const uint64_t* __restrict__ row_start, uint64_t* __restrict__ out) {
+__device__ __forceinline__ void decode_tagged(const uint8_t* __restrict__ pages, uint64_t p,
+                                              const uint64_t* __restrict__ row_start, uint64_t* __restrict__ out,
+                                              PageSmem& s) {
+    const uint8_t* pg   = pages + p * kPage;
+    const uint32_t nr   = __ldg(reinterpret_cast<const uint16_t*>(pg));
+    const uint32_t bm0  = stage_page(pg, nr, s);
+    const int32_t* data = reinterpret_cast<const int32_t*>(reinterpret_cast<const uint8_t*>(s.img) + 4);
+    uint64_t*      o    = out + __ldg(row_start + p);
+    for (uint32_t i = threadIdx.x; i < nr; i += kDecThreads) {
+        uint32_t   rank;
+        const bool on = row_rank(s, bm0, i, rank);
+        // a well-formed page has rank < num_non_null <= 2047; never read past it
+        o[i] = (on && rank < (kPage - 4) / 4) ? (uint64_t(uint32_t(data[rank])) | value_t::TAG_INT32) : 0ull;
+    }
+    __syncthreads();  // the next page overwrites the image
+}
+
+// By one warp, as decode_loc.
+__device__ __forceinline__ void decode_plain(const uint8_t* __restrict__ pages, uint64_t p,
+                                             const uint64_t* __restrict__ row_start, int32_t* __restrict__ out) {
+    const uint8_t* pg   = pages + p * kPage;
+    const uint32_t nr   = min(uint32_t(__ldg(reinterpret_cast<const uint16_t*>(pg))), uint32_t((kPage - 4) / 4));
+    const int32_t* data = reinterpret_cast<const int32_t*>(pg + 4);
+    int32_t*       o    = out + __ldg(row_start + p);
+    for (uint32_t i = threadIdx.x & 31; i < nr; i += 32) o[i] = __ldg(data + i);
+}
+
+__device__ __forceinline__ void decode_loc(const uint8_t* __restrict__ pages, uint64_t num_pages, uint64_t p,
+                                           const uint64_t* __restrict__ row_start, uint64_t* __restrict__ out) {
+    const uint8_t* pg = pages + p * kPage;
+    const uint32_t nr = __ldg(reinterpret_cast<const uint16_t*>(pg));
+    if (nr == 0xfffe) return;
+    if (nr == 0xffff) {
+        if ((threadIdx.x & 31) == 0) out[__ldg(row_start + p)] = make_loc(p * kPage, long_len(pages, p, num_pages), true);
+        return;
+    }
+    const uint32_t  nn    = __ldg(reinterpret_cast<const uint16_t*>(pg + 2));
+    const uint16_t* offs  = reinterpret_cast<const uint16_t*>(pg + 4);
+    const uint64_t  data0 = p * kPage + 4 + 2 * uint64_t(nn);
+    uint64_t*       o     = out + __ldg(row_start + p);
+    warp_rows(
+        pg, nr,
+        [&](bool on, uint32_t rank) {
+            uint64_t v = 0;
+            if (on && rank < nn && rank < (kPage - 4) / 2) {
+                const uint32_t start = rank == 0 ? 0u : __ldg(offs + rank - 1);
+                v                    = make_loc(data0 + start, uint32_t(__ldg(offs + rank)) - start, false);
+            }
+            return v;
+        },
+        [&](uint32_t i, uint64_t v) { o[i] = v; });
+}
+
+// The columns of a call share launches: unit u of one is a page of a tagged
+// column for the block, or a page for each of its warps of another one.  A
+// column of a few pages is bound by a launch's latency: with one each, the ten
+// columns of a five-relation chain took 36 us on the GPU, and the chain 373 us
+// instead of 328.
+constexpr int kMaxDecCols = 16;
+constexpr int kDecWarps   = kDecThreads / 32;
+struct DecodeOne {
+    DecodeCol c;
+    uint64_t  unit0;
+};
+struct DecodeCols {
+    int       n;
+    DecodeOne c[kMaxDecCols];
+};
+
+__global__ void __launch_bounds__(kDecThreads, 8) k_decode(DecodeCols cols, uint64_t units) {
     __shared__ PageSmem s;
-    for (uint64_t p = blockIdx.x; p < num_pages; p += gridDim.x) {
-        const uint8_t* pg  = pages + p * kPage;
-        const uint32_t nr  = *reinterpret_cast<const uint16_t*>(pg);
-        const uint32_t bm0 = stage_page(pg, nr, s);
-        const int32_t* data = reinterpret_cast<const int32_t*>(reinterpret_cast<const uint8_t*>(s.img) + 4);
-        uint64_t*      o    = out + row_start[p];
-        for (uint32_t i = threadIdx.x; i < nr; i += kDecThreads) {
-            uint32_t   rank;
-            const bool on = row_rank(s, bm0, i, rank);
-            // a well-formed page has rank < num_non_null <= 2047; never read past it
-            o[i] = (on && rank < (kPage - 4) / 4) ? (uint64_t(uint32_t(data[rank])) | value_t::TAG_INT32) : 0ull;
-        }
-        __syncthreads();  // the next page overwrites the image
-    }
-}
-
-__global__ void __launch_bounds__(kDecThreads)
-    k_decode_int32_plain(const uint8_t* __restrict__ pages, uint64_t num_pages,
-                         const uint64_t* __restrict__ row_start, int32_t* __restrict__ out) {
-    for (uint64_t p = global_warp(); p < num_pages; p += total_warps()) {
-        const uint8_t* pg   = pages + p * kPage;
-        const uint32_t nr   = min(uint32_t(*reinterpret_cast<const uint16_t*>(pg)), uint32_t((kPage - 4) / 4));
-        const int32_t* data = reinterpret_cast<const int32_t*>(pg + 4);
-        int32_t*       o    = out + row_start[p];
-        for (uint32_t i = threadIdx.x & 31; i < nr; i += 32) o[i] = __ldg(data + i);
-    }
-}
-
-__global__ void __launch_bounds__(kDecThreads, 8)
-    k_decode_varchar_loc(const uint8_t* __restrict__ pages, uint64_t num_pages,
-                         const uint64_t* __restrict__ row_start, uint64_t* __restrict__ out) {
-    for (uint64_t p = global_warp(); p < num_pages; p += total_warps()) {
-        const uint8_t* pg = pages + p * kPage;
-        const uint32_t nr = *reinterpret_cast<const uint16_t*>(pg);
-        if (nr == 0xfffe) continue;
-        if (nr == 0xffff) {
-            if ((threadIdx.x & 31) == 0) out[row_start[p]] = make_loc(p * kPage, long_len(pages, p, num_pages), true);
+    int                 ci = 0;
+    for (uint64_t u = blockIdx.x; u < units; u += gridDim.x) {
+        while (ci + 1 < cols.n && cols.c[ci + 1].unit0 <= u) ++ci;
+        const DecodeCol& c = cols.c[ci].c;
+        const uint64_t   v = u - cols.c[ci].unit0, p = v * kDecWarps + (threadIdx.x >> 5);
+        if (c.kind == kDecTagged)
+            decode_tagged(c.pages, v, c.row_start, static_cast<uint64_t*>(c.out), s);
+        else if (p >= c.num_pages)
             continue;
-        }
-        const uint32_t  nn    = *reinterpret_cast<const uint16_t*>(pg + 2);
-        const uint16_t* offs  = reinterpret_cast<const uint16_t*>(pg + 4);
-        const uint64_t  data0 = p * kPage + 4 + 2 * uint64_t(nn);
-        uint64_t*       o     = out + row_start[p];
-        warp_rows(
-            pg, nr,
-            [&](bool on, uint32_t rank) {
-                uint64_t v = 0;
-                if (on && rank < nn && rank < (kPage - 4) / 2) {
-                    const uint32_t start = rank == 0 ? 0u : offs[rank - 1];
-                    v                    = make_loc(data0 + start, uint32_t(offs[rank]) - start, false);
-                }
-                return v;
-            },
-            [&](uint32_t i, uint64_t v) { o[i] = v; });
+        else if (c.kind == kDecPlain)
+            decode_plain(c.pages, p, c.row_start, static_cast<int32_t*>(c.out));
+        else
+            decode_loc(c.pages, c.num_pages, p, c.row_start, static_cast<uint64_t*>(c.out));
     }
 }
 
-// one block per page
-unsigned block_page_grid(uint64_t num_pages) {
-    return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(num_pages, uint64_t(num_sms()) * 8)));
-}
-
-// one warp per page: kDecThreads / 32 pages per block
-unsigned page_grid(uint64_t num_pages) {
-    const uint64_t blocks = (num_pages + kDecThreads / 32 - 1) / (kDecThreads / 32);
-    return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(num_sms()) * 8)));
+// A column alone, without the look-up of its column (16M rows with NULLs in the
+// shared kernel: a scan of them 2 us longer).
+template <int KIND>
+__global__ void __launch_bounds__(kDecThreads, 8)
+    k_decode_one(const uint8_t* __restrict__ pages, uint64_t num_pages, const uint64_t* __restrict__ row_start,
+                 void* __restrict__ out) {
+    __shared__ PageSmem s;
+    if (KIND == kDecTagged) {
+        for (uint64_t p = blockIdx.x; p < num_pages; p += gridDim.x)
+            decode_tagged(pages, p, row_start, static_cast<uint64_t*>(out), s);
+        return;
+    }
+    for (uint64_t p = uint64_t(blockIdx.x) * kDecWarps + (threadIdx.x >> 5); p < num_pages;
+         p += uint64_t(gridDim.x) * kDecWarps) {
+        if (KIND == kDecPlain) decode_plain(pages, p, row_start, static_cast<int32_t*>(out));
+        else                   decode_loc(pages, num_pages, p, row_start, static_cast<uint64_t*>(out));
+    }
 }
 
 }  // namespace
@@ -223,25 +257,25 @@ void launch_page_rows(const uint8_t* pages, uint64_t num_pages, int32_t type, ui
     HJ_LAUNCH_CHECK();
 }
 
-void launch_decode_int32_tagged(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                                uint64_t* out, cudaStream_t st) {
-    if (num_pages == 0) return;
-    k_decode_int32_tagged<<<block_page_grid(num_pages), kDecThreads, 0, st>>>(pages, num_pages, row_start, out);
-    HJ_LAUNCH_CHECK();
-}
-
-void launch_decode_int32_plain(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                               int32_t* out, cudaStream_t st) {
-    if (num_pages == 0) return;
-    k_decode_int32_plain<<<page_grid(num_pages), kDecThreads, 0, st>>>(pages, num_pages, row_start, out);
-    HJ_LAUNCH_CHECK();
-}
-
-void launch_decode_varchar_loc(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                               uint64_t* out, cudaStream_t st) {
-    if (num_pages == 0) return;
-    k_decode_varchar_loc<<<page_grid(num_pages), kDecThreads, 0, st>>>(pages, num_pages, row_start, out);
-    HJ_LAUNCH_CHECK();
+void launch_decode(const std::vector<DecodeCol>& cols, cudaStream_t st) {
+    for (size_t g0 = 0; g0 < cols.size(); g0 += kMaxDecCols) {
+        DecodeCols G{};
+        uint64_t   units = 0;
+        for (size_t i = g0; i < std::min(cols.size(), g0 + kMaxDecCols); ++i) {
+            if (cols[i].num_pages == 0) continue;
+            G.c[G.n++] = DecodeOne{cols[i], units};
+            units += cols[i].kind == kDecTagged ? cols[i].num_pages : (cols[i].num_pages + kDecWarps - 1) / kDecWarps;
+        }
+        if (units == 0) continue;
+        const unsigned grid = unsigned(std::min<uint64_t>(units, uint64_t(num_sms()) * 8));
+        const DecodeCol& c = G.c[0].c;
+        auto one = [&](auto kernel) { kernel<<<grid, kDecThreads, 0, st>>>(c.pages, c.num_pages, c.row_start, c.out); };
+        if (G.n > 1)                   k_decode<<<grid, kDecThreads, 0, st>>>(G, units);
+        else if (c.kind == kDecTagged) one(k_decode_one<kDecTagged>);
+        else if (c.kind == kDecPlain)  one(k_decode_one<kDecPlain>);
+        else                           one(k_decode_one<kDecLoc>);
+        HJ_LAUNCH_CHECK();
+    }
 }
 
 }  // namespace hj

@@ -577,11 +577,9 @@ std::shared_ptr<DevTable> upload_table(hj_context* c, const hj_table_desc& t,
     return dt;
 }
 
-void decode_kernels(cudaStream_t st, DevColumn& d);
-
-// Decodes a device column (idempotent within one execute call); no host
-// synchronisation: sizes come from the page statistics.
-void decode_column(hj_context* c, DevColumn& d, uint32_t table_id, uint32_t col_idx) {
+// Checks a device column that a plan reads and adds it to `todo` if its pages are
+// still to be decoded (decode_kernels); once per column and execute call.
+void decode_column(DevColumn& d, uint32_t table_id, uint32_t col_idx, std::vector<DevColumn*>& todo) {
     if (d.decoded) return;
     d.decoded = true;
     if (d.type != HJ_INT32 && d.type != HJ_VARCHAR) {  // the reference's copy_scan skips these types
@@ -602,37 +600,41 @@ void decode_column(hj_context* c, DevColumn& d, uint32_t table_id, uint32_t col_
                                                  + " > " + std::to_string(StrRef::PAGE_MASK));
     }
     if (d.predecoded) return;  // decoded once when the resident table was prepared
-    decode_kernels(c->st, d);
+    todo.push_back(&d);
 }
 
-// The decode kernels of one column (no checks): pages -> plain / tagged / locators.
-void decode_kernels(cudaStream_t st, DevColumn& d) {
-    if (d.num_pages == 0 || d.rows == 0) return;
-    if (!d.pages) throw Error(HJ_ERR_INVALID, "column pages were not uploaded");
-    if (d.type == HJ_INT32 && d.dense1984) return;  // read in place (direct mode)
-    const uint64_t np = d.num_pages;
-    uint32_t*      pr = nullptr;
-    uint64_t*      rs = d.row_start ? d.row_start->as<uint64_t>() : nullptr;
-    if (!rs) {  // a column without host page statistics: row starts on the device
-        pr = dalloc_n<uint32_t>(np, st);
-        rs = dalloc_n<uint64_t>(np + 1, st);
-        launch_page_rows(d.pages->as<uint8_t>(), np, d.type, pr, st);
-        scan_exclusive_u32_to_u64(pr, rs, np, st);
+// The decode kernels of columns (no checks): pages -> plain / tagged / locators.
+// No host synchronisation: sizes come from the page statistics.
+void decode_kernels(cudaStream_t st, const std::vector<DevColumn*>& todo) {
+    std::vector<DecodeCol> cols;
+    std::vector<void*>     scratch;
+    cols.reserve(todo.size());
+    for (DevColumn* dp : todo) {
+        DevColumn& d = *dp;
+        if (d.num_pages == 0 || d.rows == 0) continue;
+        if (!d.pages) throw Error(HJ_ERR_INVALID, "column pages were not uploaded");
+        if (d.type == HJ_INT32 && d.dense1984) continue;  // read in place (direct mode)
+        const uint64_t np = d.num_pages;
+        uint64_t*      rs = d.row_start ? d.row_start->as<uint64_t>() : nullptr;
+        if (!rs) {  // a column without host page statistics: row starts on the device
+            uint32_t* pr = dalloc_n<uint32_t>(np, st);
+            rs           = dalloc_n<uint64_t>(np + 1, st);
+            scratch.push_back(pr);
+            scratch.push_back(rs);
+            launch_page_rows(d.pages->as<uint8_t>(), np, d.type, pr, st);
+            scan_exclusive_u32_to_u64(pr, rs, np, st);
+        }
+        DecodeKind kind = kDecLoc;
+        Buf*       out  = &d.locs;
+        if (d.type == HJ_INT32) {
+            kind = d.non_null == d.rows ? kDecPlain : kDecTagged;
+            out  = kind == kDecPlain ? &d.plain : &d.tagged;
+        }
+        *out = make_buf(d.rows * (kind == kDecPlain ? 4 : 8), st);
+        cols.push_back(DecodeCol{d.pages->as<uint8_t>(), np, rs, (*out)->p, kind});
     }
-    if (d.type == HJ_INT32 && d.non_null == d.rows) {
-        d.plain = make_buf(d.rows * 4, st);
-        launch_decode_int32_plain(d.pages->as<uint8_t>(), np, rs, d.plain->as<int32_t>(), st);
-    } else if (d.type == HJ_INT32) {
-        d.tagged = make_buf(d.rows * 8, st);
-        launch_decode_int32_tagged(d.pages->as<uint8_t>(), np, rs, d.tagged->as<uint64_t>(), st);
-    } else {
-        d.locs = make_buf(d.rows * 8, st);
-        launch_decode_varchar_loc(d.pages->as<uint8_t>(), np, rs, d.locs->as<uint64_t>(), st);
-    }
-    if (pr) {
-        dfree(pr, st);
-        dfree(rs, st);
-    }
+    launch_decode(cols, st);
+    for (void* p : scratch) dfree(p, st);
 }
 
 // ------------------------------------------------------------ intermediates --
@@ -693,7 +695,9 @@ struct Exec {
 
     DevColumn& column(uint32_t t, uint32_t col) {
         DevColumn& d = tables[t]->cols[col];
-        decode_column(c, d, t, col);
+        std::vector<DevColumn*> todo;
+        decode_column(d, t, col, todo);
+        if (!todo.empty()) decode_kernels(c->st, todo);
         return d;
     }
 
@@ -1284,11 +1288,13 @@ int hj_table_prepare(hj_context* c, uint64_t handle) {
         // decode into a private copy, then publish it: executions that copied
         // the table meanwhile keep decoding per call
         auto nt = std::make_shared<hj::DevTable>(*dt);
+        std::vector<hj::DevColumn*> todo;
         for (auto& col : nt->cols) {
             if (col.predecoded || (col.type != HJ_INT32 && col.type != HJ_VARCHAR)) continue;
-            hj::decode_kernels(c->st, col);
+            todo.push_back(&col);
             col.predecoded = true;
         }
+        hj::decode_kernels(c->st, todo);
         HJ_CUDA(cudaStreamSynchronize(c->st));
         std::lock_guard<std::mutex> g(c->store->mu);
         auto it = c->store->tables.find(handle);
@@ -1362,18 +1368,22 @@ int hj_execute(hj_context* c, const hj_plan_desc* plan, hj_result** out) {
         if (host_inputs) upload_turn.unlock();
         // copy_scan of every scanned column, before any join (execute.cpp:575-582)
         ex.phase("decode");
+        std::vector<hj::DevColumn*> todo;
+        todo.reserve(16);
+        auto add = [&](uint32_t t, uint32_t col) { hj::decode_column(ex.tables[t]->cols[col], t, col, todo); };
         for (uint32_t i = 0; i < plan->num_nodes; ++i) {
             const hj_node_desc& n = plan->nodes[i];
             if (n.kind != HJ_NODE_SCAN) continue;
             for (uint32_t a = 0; a < n.num_attrs; ++a) {
                 if (n.attrs[a].index >= ex.tables[n.base_table_id]->cols.size())
                     throw hj::Error(HJ_ERR_INVALID, "scan column out of range");
-                ex.column(uint32_t(n.base_table_id), uint32_t(n.attrs[a].index));
+                add(uint32_t(n.base_table_id), uint32_t(n.attrs[a].index));
             }
             for (uint32_t f = 0; f < n.num_filters && n.filters; ++f)
                 if (n.filters[f].column < ex.tables[n.base_table_id]->cols.size())
-                    ex.column(uint32_t(n.base_table_id), uint32_t(n.filters[f].column));
+                    add(uint32_t(n.base_table_id), uint32_t(n.filters[f].column));
         }
+        hj::decode_kernels(c->st, todo);
         hj::Inter root = ex.run(plan->root);
         ex.compact(root);  // a filtered scan as the root
         ex.materialize(root, plan->nodes[plan->root], res);

@@ -64,14 +64,18 @@ void   scan_exclusive_u32_to_u64_into(const uint32_t* in, uint64_t* out, uint64_
 // rows[p] = rows page p contributes to its column (VARCHAR: 0xffff -> 1, 0xfffe -> 0).
 void launch_page_rows(const uint8_t* pages, uint64_t num_pages, int32_t type, uint32_t* rows,
                       cudaStream_t st);
-// row_start: exclusive scan of page rows.  INT32 -> value_t per row; INT32
-// without NULLs -> int32 per row; VARCHAR -> locator per row (hj_common.cuh).
-void launch_decode_int32_tagged(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                                uint64_t* out, cudaStream_t st);
-void launch_decode_int32_plain(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                               int32_t* out, cudaStream_t st);
-void launch_decode_varchar_loc(const uint8_t* pages, uint64_t num_pages, const uint64_t* row_start,
-                               uint64_t* out, cudaStream_t st);
+// Columns to decode; row_start: exclusive scan of page rows.  INT32 -> value_t
+// per row; INT32 without NULLs -> int32 per row; VARCHAR -> locator per row
+// (hj_common.cuh).  Several columns share a launch.
+enum DecodeKind : int { kDecTagged, kDecPlain, kDecLoc };
+struct DecodeCol {
+    const uint8_t*  pages;
+    uint64_t        num_pages;
+    const uint64_t* row_start;
+    void*           out;
+    DecodeKind      kind;
+};
+void launch_decode(const std::vector<DecodeCol>& cols, cudaStream_t st);
 
 // ---- unchained table build (hj_build.cu) -----------------------------------
 struct KeyCol {
