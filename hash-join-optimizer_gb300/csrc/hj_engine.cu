@@ -751,7 +751,7 @@ struct Exec {
     void compact(Inter& in) {
         if (in.filt.n == 0) return;
         Buf rid = make_buf(std::max<uint64_t>(in.rows, 1) * 4, c->st);
-        in.rows = filter_compact(in.filt, in.rows, rid->as<uint32_t>(), c->pinned, c->st);
+        in.rows = filter_compact(in.filt, in.rows, rid->as<uint32_t>(), c->pinned, c->counters, c->st);
         in.srcs[0].rid = rid;
         in.filt.n      = 0;
     }

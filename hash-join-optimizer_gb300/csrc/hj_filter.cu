@@ -12,8 +12,8 @@
 //    32-row ballots) and a count per tile.  A warp issues the loads of its 16
 //    rows per lane before it compares any of them, so 16 loads per thread are
 //    in flight; the column is read once.
-//  * after an exclusive scan of the tile counts, k_filter_emit reads only the
-//    bit words and writes each passing row's id at its rank, so the ids come
+//  * after an exclusive scan of the tile counts (by the mask's last block),
+//    k_filter_emit reads only the bit words and writes each passing row's id at its rank, so the ids come
 //    out in base-row order.
 #include <algorithm>
 
@@ -77,9 +77,12 @@ __device__ __forceinline__ uint32_t load_steps(const IntCol& c, uint64_t r0, uin
     return valid;
 }
 
+// `ticket`: a zeroed device word (zero again afterwards) when the block that is
+// done last scans the tile counts into `off` and hands their sum to the host
+// (*host, page-locked); nullptr: neither.
 __global__ void __launch_bounds__(kFT, 4)
     k_filter_mask(Filters F, uint64_t n, uint64_t nwords, uint64_t ntiles, uint32_t* __restrict__ words,
-                  uint32_t* __restrict__ cnt) {
+                  uint32_t* cnt, unsigned long long* ticket, uint64_t* off, uint64_t* host) {
     __shared__ uint32_t wt[kFT / 32];
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -114,6 +117,37 @@ __global__ void __launch_bounds__(kFT, 4)
             cnt[tile] = t;
         }
         __syncthreads();
+    }
+    if (!ticket) return;
+    __shared__ uint32_t sm[33];
+    __shared__ bool     last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    uint64_t run = 0;
+    for (uint64_t t0 = 0; t0 < ntiles; t0 += kFT * kFStep) {
+        const uint64_t t = t0 + threadIdx.x * kFStep;
+        uint32_t       c[kFStep], sum = 0, tot;
+#pragma unroll
+        for (int k = 0; k < kFStep; ++k) {
+            c[k] = t + k < ntiles ? __ldcg(cnt + t + k) : 0u;
+            sum += c[k];
+        }
+        uint64_t at = run + block_exclusive_scan<uint32_t>(sum, sm, &tot);
+#pragma unroll
+        for (int k = 0; k < kFStep; ++k) {
+            if (t + k < ntiles) off[t + k] = at;
+            at += c[k];
+        }
+        run += tot;
+    }
+    if (threadIdx.x == 0) {
+        *host   = run;
+        *ticket = 0;
     }
 }
 
@@ -150,7 +184,14 @@ __global__ void __launch_bounds__(kFT)
 
 }  // namespace
 
-uint64_t filter_compact(const Filters& f, uint64_t n, uint32_t* rid_out, uint64_t* pinned, cudaStream_t st) {
+// Up to this many tiles (67M rows) the mask's last block scans them: four steps of
+// one block, where the scan's launches and the readback cost as many gaps; a
+// scan of 16M rows 241 us, so 226, with the host going on while the ids are
+// written.  More tiles take the scan's own launches, which share its work out.
+constexpr uint64_t kFOneScan = 1u << 14;
+
+uint64_t filter_compact(const Filters& f, uint64_t n, uint32_t* rid_out, uint64_t* pinned, uint64_t* counters,
+                        cudaStream_t st) {
     if (n == 0) return 0;
     if (n > 0xffffffffull) throw Error(HJ_ERR_INVALID, "a filtered scan has more than 2^32 rows");
     const uint64_t ntiles = (n + kFTile - 1) / kFTile;
@@ -159,13 +200,23 @@ uint64_t filter_compact(const Filters& f, uint64_t n, uint32_t* rid_out, uint64_
     uint32_t*      words  = dalloc_n<uint32_t>(nwords, st);
     uint32_t*      cnt    = dalloc_n<uint32_t>(ntiles, st);
     uint64_t*      off    = dalloc_n<uint64_t>(ntiles + 1, st);
-    k_filter_mask<<<grid, kFT, 0, st>>>(f, n, nwords, ntiles, words, cnt);
+    const bool     one    = ntiles <= kFOneScan;
+    cudaEvent_t    counted;
+    HJ_CUDA(cudaEventCreateWithFlags(&counted, cudaEventDisableTiming));
+    k_filter_mask<<<grid, kFT, 0, st>>>(f, n, nwords, ntiles, words, cnt,
+                                        one ? reinterpret_cast<unsigned long long*>(counters) : nullptr, off, pinned);
     HJ_LAUNCH_CHECK();
-    scan_exclusive_u32_to_u64(cnt, off, ntiles, st);
+    if (!one) {
+        scan_exclusive_u32_to_u64(cnt, off, ntiles, st);
+        readback(pinned, off + ntiles, sizeof(uint64_t), true, st);  // page-locked scratch
+    }
+    HJ_CUDA(cudaEventRecord(counted, st));
     k_filter_emit<<<grid, kFT, 0, st>>>(words, nwords, ntiles, off, rid_out);
     HJ_LAUNCH_CHECK();
-    readback(pinned, off + ntiles, sizeof(uint64_t), true, st);  // page-locked scratch
-    HJ_CUDA(cudaStreamSynchronize(st));
+    // the host goes on while the row ids are written
+    const cudaError_t e = cudaEventSynchronize(counted);
+    cudaEventDestroy(counted);
+    HJ_CUDA(e);
     const uint64_t kept = pinned[0];
     dfree(words, st);
     dfree(cnt, st);

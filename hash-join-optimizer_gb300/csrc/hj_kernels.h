@@ -87,8 +87,10 @@ struct KeyCol {
 
 // ---- scan predicates (hj_filter.cu) ----------------------------------------
 // Base rows 0..n-1 that pass `f`, in order, into rid_out (n slots); returns their
-// number (one host synchronisation through `pinned`).
-uint64_t filter_compact(const Filters& f, uint64_t n, uint32_t* rid_out, uint64_t* pinned, cudaStream_t st);
+// number (one host synchronisation through `pinned`; `counters`: a zeroed device
+// word, zero again afterwards).  The row ids may still be on their way.
+uint64_t filter_compact(const Filters& f, uint64_t n, uint32_t* rid_out, uint64_t* pinned, uint64_t* counters,
+                        cudaStream_t st);
 
 struct Table {
     uint32_t  dir_bits  = 0;
