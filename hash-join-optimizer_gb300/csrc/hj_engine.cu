@@ -356,6 +356,49 @@ struct Store {
 
 // ------------------------------------------------------------------ context --
 
+namespace hj {
+// Page-locked buffers for the small columns of results, given back when a
+// result is freed (by any thread; the pool lives as long as a result holds one
+// of its buffers).  At most kBuffers: a program that keeps more results reads
+// the others from the device.
+class HostPool : public std::enable_shared_from_this<HostPool> {
+public:
+    static constexpr size_t kBytes   = 1u << 20;
+    static constexpr int    kBuffers = 8;
+    using Ptr = std::shared_ptr<uint8_t>;
+    Ptr get() {
+        uint8_t* p = nullptr;
+        {
+            std::lock_guard<std::mutex> g(mu_);
+            if (!free_.empty()) {
+                p = free_.back();
+                free_.pop_back();
+            } else if (made_ < kBuffers) {
+                if (cudaMallocHost(&p, kBytes) != cudaSuccess) {
+                    (void)cudaGetLastError();
+                    return nullptr;
+                }
+                ++made_;
+            }
+        }
+        if (!p) return nullptr;
+        return Ptr(p, [self = shared_from_this()](uint8_t* q) {
+            std::lock_guard<std::mutex> g(self->mu_);
+            self->free_.push_back(q);
+        });
+    }
+    HostPool() { free_.reserve(kBuffers); }
+    ~HostPool() {
+        for (uint8_t* p : free_) cudaFreeHost(p);
+    }
+
+private:
+    std::mutex            mu_;
+    std::vector<uint8_t*> free_;
+    int                   made_ = 0;
+};
+}  // namespace hj
+
 struct hj_context {
     int                 device = 0;
     cudaStream_t        st     = nullptr;
@@ -372,6 +415,7 @@ struct hj_context {
     int64_t             batch_graph    = 1;    // batched joins: launch as one CUDA graph
     int64_t             batch_part_log2 = 12;  // batched joins: ~2^x build rows per partition
     uint64_t*           pinned      = nullptr;  // small readbacks
+    std::shared_ptr<hj::HostPool> host_pool = std::make_shared<hj::HostPool>();  // small result columns
     uint64_t*           counters    = nullptr;  // probe counters on the device, zero between probes
     uint8_t*            staging     = nullptr;  // pinned transfer ring
     size_t              staging_bytes = 0;
@@ -386,10 +430,12 @@ struct hj_context {
 struct hj_result {
     uint64_t num_rows = 0;
     struct Col {
-        int32_t  type;
-        uint64_t num_pages;
-        hj::Buf  pages;
+        int32_t        type;
+        uint64_t       num_pages;
+        hj::Buf        pages;
+        const uint8_t* host = nullptr;  // the pages in `host_pages`, when they are few
     };
+    hj::HostPool::Ptr host_pages;
     std::vector<Col> cols;
     uint64_t         build_tuples = 0, probe_tuples = 0, output_rows = 0;
     uint64_t         dir_words = 0, table_tuples = 0, joins = 0;  // summed over the joins
@@ -971,6 +1017,19 @@ struct Exec {
     void materialize(const Inter& in, const hj_node_desc& root, hj_result* res) {
         phase("materialize");
         res->cols.assign(root.num_attrs, hj_result::Col{0, 0, nullptr});
+        // A column of up to kHostPages pages is written to page-locked memory as
+        // well, so that fetching it is a copy by the host: a copy and a wait take
+        // 9 us a column, 64 KB by the host some 4.
+        constexpr uint64_t kHostPages = 8;
+        size_t             host_used  = 0;
+        auto               host_for   = [&](uint64_t pages) -> uint8_t* {
+            if (pages == 0 || pages > kHostPages || host_used + pages * kPage > HostPool::kBytes) return nullptr;
+            if (!res->host_pages) res->host_pages = c->host_pool->get();
+            if (!res->host_pages) return nullptr;
+            uint8_t* p = res->host_pages.get() + host_used;
+            host_used += pages * kPage;
+            return p;
+        };
         std::vector<IntPages>                        iout;  // written after the VARCHAR page counts are known
         std::vector<std::pair<uint32_t, VarcharOut>> vout;  // (column, plan)
         for (uint32_t a = 0; a < root.num_attrs; ++a) {
@@ -996,7 +1055,9 @@ struct Exec {
                 }
                 oc.num_pages = (rows + kDenseRows - 1) / kDenseRows;
                 oc.pages     = make_buf(oc.num_pages * kPage, c->st);  // allocated while earlier work runs
-                iout.push_back(IntPages{col, rid, rows, oc.pages->as<uint8_t>()});
+                uint8_t* hp  = host_for(oc.num_pages);
+                oc.host      = hp;
+                iout.push_back(IntPages{col, rid, rows, oc.pages->as<uint8_t>(), hp});
             } else if (ty == HJ_VARCHAR) {
                 VarcharOut v{};
                 if (d.type == HJ_INT32) {
@@ -1047,6 +1108,10 @@ struct Exec {
         }
         if (!vout.empty()) {
             phase("mat_varchar_write");
+            for (size_t i = 0; i < vout.size(); ++i) {
+                vout[i].second.host           = host_for(vpages[i]);
+                res->cols[vout[i].first].host = vout[i].second.host;
+            }
             const std::vector<uint8_t*> bufs = varchar_write(vptr, vpages, c->st);
             for (size_t i = 0; i < vout.size(); ++i) {
                 hj_result::Col& oc = res->cols[vout[i].first];
@@ -1398,8 +1463,8 @@ int hj_execute(hj_context* c, const hj_plan_desc* plan, hj_result** out) {
     });
     res->kernel_launches = hj::g_kernel_launches.load() - launches0;
     if (rc != HJ_OK) {
+        cudaStreamSynchronize(c->st);  // kernels may still write to its host pages
         delete res;
-        cudaStreamSynchronize(c->st);
         return rc;
     }
     *out = res;
@@ -1445,6 +1510,10 @@ int hj_result_copy_pages(hj_context* c, const hj_result* r, uint32_t col, void* 
     return hj::guarded(c, [&] {
         const auto& oc = r->cols[col];
         if (!oc.num_pages) return;
+        if (oc.host && std::all_of(dst, dst + oc.num_pages, [](const void* p) { return hj::host_memory(p); })) {
+            for (uint64_t i = 0; i < oc.num_pages; ++i) std::memcpy(dst[i], oc.host + i * hj::kPage, hj::kPage);
+            return;
+        }
         const auto runs = hj::locked_runs(dst, oc.num_pages, 64);
         if (!runs.empty()) {  // page-locked destination: copy engines, one copy per run
             for (const auto& q : runs)
@@ -1465,6 +1534,10 @@ int hj_result_copy_contiguous(hj_context* c, const hj_result* r, uint32_t col, v
     return hj::guarded(c, [&] {
         const auto& oc = r->cols[col];
         if (!oc.num_pages) return;
+        if (oc.host && hj::host_memory(dst)) {
+            std::memcpy(dst, oc.host, oc.num_pages * hj::kPage);
+            return;
+        }
         if (hj::locked_range(dst, oc.num_pages * hj::kPage)) {  // page-locked destination: copy engine
             HJ_CUDA(cudaMemcpyAsync(dst, oc.pages->p, oc.num_pages * hj::kPage, cudaMemcpyDeviceToHost, c->st));
             HJ_CUDA(cudaStreamSynchronize(c->st));

@@ -41,6 +41,8 @@ struct PageRun {
 std::vector<PageRun> locked_runs(const void* const* pages, uint64_t n, size_t max_runs);
 // Whether [p, p + bytes) starts and ends in page-locked host memory.
 bool locked_range(const void* p, uint64_t bytes);
+// p is memory that the host may write: page-locked or not known to CUDA.
+bool host_memory(const void* p);
 // Device -> host copy of a few bytes (counters, page headers).  kernel: the
 // GPU writes `host` itself (page-locked memory, or any host memory with
 // pageable host memory access), so the readback never waits behind large
@@ -178,6 +180,7 @@ struct IntPages {
     const uint32_t* rid;
     uint64_t        n;
     uint8_t*        out;
+    uint8_t*        host;  // the pages once more in page-locked memory, or nullptr
 };
 void launch_write_int32_pages(const std::vector<IntPages>& cols, cudaStream_t st);
 
@@ -202,6 +205,7 @@ struct VarcharOut {
     uint64_t*       host_pages = nullptr;  // where the page count goes (page-locked; set by the caller)
     uint64_t        pages      = 0;        // varchar_write: the page count
     uint8_t*        out        = nullptr;  // and the pages
+    uint8_t*        host       = nullptr;  // (set by the caller) the pages once more in page-locked memory
 };
 // All VARCHAR columns of a result at once (their kernels share launches).
 void varchar_plan(std::vector<VarcharOut*>& vs, cudaStream_t st);

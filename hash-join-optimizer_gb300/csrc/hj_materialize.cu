@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kMT) k_write_int32_pages(IntCols cols, uint64_
         if (threadIdx.x == 0) words[0] = nr | (tot << 16);
         __syncthreads();
         store_page(cols.c[ci].c.out + p * kPage, img);
+        if (cols.c[ci].c.host) store_page(cols.c[ci].c.host + p * kPage, img);
         __syncthreads();
     }
 }
@@ -228,7 +229,7 @@ struct PackCol {
     uint64_t*       recs;        // kRec page-start records per tile
     uint64_t*       host_pages;  // the column's page count, in page-locked memory
     uint64_t        pages, page0;  // of the page writer: pages of the column, and of those before it
-    uint8_t*        out;
+    uint8_t *       out, *host;
 };
 struct PackCols {
     int     n;
@@ -605,6 +606,11 @@ __global__ void __launch_bounds__(kVT, kVMin) k_write_varchar_pages(PackCols P, 
         uint4* dst = reinterpret_cast<uint4*>(P.c[ci].out + pi * kPage) + part * 32 * kQ;
 #pragma unroll
         for (int k = 0; k < kQ; ++k) dst[lane + 32 * k] = w4[lane + 32 * k];
+        if (P.c[ci].host) {
+            dst = reinterpret_cast<uint4*>(P.c[ci].host + pi * kPage) + part * 32 * kQ;
+#pragma unroll
+            for (int k = 0; k < kQ; ++k) dst[lane + 32 * k] = w4[lane + 32 * k];
+        }
     }
 }
 
@@ -670,7 +676,7 @@ void for_pack_groups(std::vector<VarcharOut*>& vs, F&& f) {
         for (size_t i = g0; i < std::min(live.size(), g0 + kMaxPackCols); ++i) {
             VarcharOut& v = *live[i];
             P.c[P.n++]    = PackCol{v.locs, v.rid, v.ol, v.base, v.base_pages, v.n, v.ntiles, tiles,
-                                 v.tile_pages, v.tile_off, v.desc, v.recs, v.host_pages, v.pages, pages, v.out};
+                                 v.tile_pages, v.tile_off, v.desc, v.recs, v.host_pages, v.pages, pages, v.out, v.host};
             tiles += v.ntiles;
             pages += v.pages;
         }

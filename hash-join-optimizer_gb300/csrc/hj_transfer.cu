@@ -119,6 +119,16 @@ bool locked_range(const void* p, uint64_t bytes) {
     return bytes > 0 && page_locked(p) && page_locked(static_cast<const uint8_t*>(p) + bytes - 1);
 }
 
+bool host_memory(const void* p) {
+    if (!p) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
+}
+
 void readback(void* host, const void* dev, uint64_t bytes, bool kernel, cudaStream_t st) {
     if (bytes == 0) return;
     if (!kernel) {
