@@ -1650,10 +1650,8 @@ int hj_table_probe(hj_context* c, const hj_hash_table* t, const int32_t* keys, c
             } else if (total > 0) {
                 if (!out_probe || !out_build) throw hj::Error(HJ_ERR_INVALID, "null output buffer");
                 const hj::RidOut ro[2] = {{0, nullptr, out_probe}, {1, nullptr, out_build}};
-                if (const uint64_t d = hj::probe_direct(pp)) {
-                    HJ_CUDA(cudaMemcpyAsync(out_probe, dp->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
-                    HJ_CUDA(cudaMemcpyAsync(out_build, db->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
-                }
+                if (const uint64_t d = hj::probe_direct(pp))
+                    hj::copy_pairs(dp->as<uint32_t>(), db->as<uint32_t>(), out_probe, out_build, d, c->st);
                 hj::probe_write(t->t, pk, pp, ro, 2, c->st);
             }
         } catch (...) {

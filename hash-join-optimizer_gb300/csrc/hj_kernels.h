@@ -156,6 +156,8 @@ struct ProbePlan;  // opaque match list between the count and write passes
 uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, const RidOut* outs, int nout,
                      ProbePlan** pp, cudaStream_t st);
 uint64_t probe_direct(const ProbePlan* pp);
+// n words each of a and b to da and db (4-byte aligned), in one launch.
+void copy_pairs(const uint32_t* a, const uint32_t* b, uint32_t* da, uint32_t* db, uint64_t n, cudaStream_t st);
 // Write pass: emits the listed matches' row ids after the directly written
 // ones (all `nout` streams have probe_count() slots; the direct rows are there
 // already); the caller frees *pp with probe_free afterwards.
