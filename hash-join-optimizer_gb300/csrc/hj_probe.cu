@@ -85,6 +85,10 @@ struct Lists {
     // (the last up to the staged total); mask 0: the whole bucket sp matches,
     // kRowHit: build row sp, else the tuples sp + i for the set bits i of mask
     uint32_t *u_row, *u_sp, *u_off, *u_mask;
+    // entries of each list.  Past 2^32 staged matches (a result that is counted,
+    // but never written) the low word of counter 0 carries into the number of
+    // hits, and list slots up to one per carry lie behind the end: not stored
+    uint32_t cap;
     uint32_t *m_row, *m_s, *m_e, *m_cnt;    // mixed hits: tuples [s, e) compared with m_key
     int32_t*  m_key;
     // 0 staged hits << 32 | staged matches mod 2^32, 1 mixed hits, 2 staged
@@ -377,8 +381,7 @@ __global__ void __launch_bounds__(kPT, 4)
                         const uint32_t v = o.side == 0 ? qr[e] : qs[e];
                         o.dst[db + __popc(bd & lt)] = o.src ? __ldg(o.src + v) : v;
                     }
-                } else if (on) {
-                    const uint32_t h = li + __popc(bl & lt);
+                } else if (const uint32_t h = li + __popc(bl & lt); on && h < Ls.cap) {
                     Ls.u_row[h]  = qr[e];
                     Ls.u_sp[h]   = qs[e];
                     Ls.u_off[h]  = off + in - c;
@@ -472,10 +475,13 @@ __global__ void __launch_bounds__(kPT, 4)
                     if (hi > 0) {
                         const uint32_t           p = slot_of(T, k[u]), n = bucket_tuples(T, p);
                         const unsigned long long base = atomicAdd(Ls.ctr + 0, (1ull << 32) + n);
-                        Ls.u_row[base >> 32]  = row;
-                        Ls.u_sp[base >> 32]   = p;
-                        Ls.u_off[base >> 32]  = uint32_t(base);
-                        Ls.u_mask[base >> 32] = 0;
+                        const uint32_t           h    = uint32_t(base >> 32);
+                        if (h < Ls.cap) {
+                            Ls.u_row[h]  = row;
+                            Ls.u_sp[h]   = p;
+                            Ls.u_off[h]  = uint32_t(base);
+                            Ls.u_mask[h] = 0;
+                        }
                         listed += n;
                     } else {
                         list_mixed(T, Ls, row, k[u], uint32_t(hi));
@@ -1000,6 +1006,7 @@ uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, c
     L.m_e   = dalloc_n<uint32_t>(n, st);
     L.m_cnt = dalloc_n<uint32_t>(n, st);
     L.m_key = dalloc_n<int32_t>(n, st);
+    L.cap   = uint32_t(n);
     L.ctr   = reinterpret_cast<unsigned long long*>(prm.counters);
     Outs outs{};
     outs.n = nout;
@@ -1149,6 +1156,7 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
     L.m_e   = c.take<uint32_t>(n);
     L.m_cnt = c.take<uint32_t>(n);
     L.m_key = c.take<int32_t>(n);
+    L.cap   = uint32_t(n);
     m_off   = c.take<uint64_t>(n + 1);
     tmp     = c.take<uint64_t>(scan_tmp_words(n) + 1);
     // the scratch keeps the previous call's contents: the counters restart at zero
