@@ -1650,9 +1650,9 @@ int hj_table_probe(hj_context* c, const hj_hash_table* t, const int32_t* keys, c
             } else if (total > 0) {
                 if (!out_probe || !out_build) throw hj::Error(HJ_ERR_INVALID, "null output buffer");
                 const hj::RidOut ro[2] = {{0, nullptr, out_probe}, {1, nullptr, out_build}};
+                hj::probe_write(t->t, pk, pp, ro, 2, c->st);  // (refuses more than 2^32 rows, with nothing written)
                 if (const uint64_t d = hj::probe_direct(pp))
                     hj::copy_pairs(dp->as<uint32_t>(), db->as<uint32_t>(), out_probe, out_build, d, c->st);
-                hj::probe_write(t->t, pk, pp, ro, 2, c->st);
             }
         } catch (...) {
             hj::probe_free(pp, c->st);

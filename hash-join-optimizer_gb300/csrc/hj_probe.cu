@@ -767,6 +767,11 @@ __global__ void __launch_bounds__(512)
     }
 }
 
+// More rows than row ids can number are refused before any is written.
+void check_rows(uint64_t rows) {
+    if (rows > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
+}
+
 ProbeTab tab_of(const Table& t) { return ProbeTab{t.dir, t.summary, t.keys, t.rows, 1u << t.dir_bits}; }
 
 // How the count kernels read a probe column's keys.
@@ -960,7 +965,6 @@ void launch_uniform_g(const ProbeTab& T, const Lists& L, uint64_t n_u, const uin
 // The staged hits' matches (total of them, < 2^32) into the output streams.
 void launch_uniform(int G, const ProbeTab& T, const Lists& L, uint64_t n_u, const uint32_t* chunk_first,
                     uint64_t total, const Outs& outs, cudaStream_t st) {
-    if (total > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
     switch (G) {
     case 1: launch_uniform_g<1>(T, L, n_u, chunk_first, total, outs, st); break;
     case 2: launch_uniform_g<2>(T, L, n_u, chunk_first, total, outs, st); break;
@@ -1088,6 +1092,7 @@ void probe_write(const Table& t, const KeyCol& pk, ProbePlan* pp, const RidOut* 
     (void)pk;
     if (nout > kMaxRidOut) throw Error(HJ_ERR_INVALID, "too many output row-id streams");
     if (nout == 0) return;
+    check_rows(pp->tot_d + pp->tot_u);
     Outs outs{};
     outs.n = nout;
     for (int i = 0; i < nout; ++i) {
@@ -1171,6 +1176,7 @@ int probe_into_scratch(const Table& t, const KeyCol& pk, const ProbeParams& prm,
     *num_matches = total;
     if (total > capacity) return HJ_ERR_CAPACITY;
     if (total == 0) return HJ_OK;
+    check_rows(tot_u);
     Outs outs{};
     outs.n    = 2;
     outs.o[0] = RidOut{0, nullptr, out_probe};

@@ -36,3 +36,30 @@ def test_more_than_2_32_matches_are_counted(engine, hj, nb, fn):
         assert np.array_equal(np.sort(out[1].cpu().numpy()), np.arange(nb))
     finally:
         L.hj_table_free(t)
+
+
+def test_more_than_2_32_rows_are_not_written(engine, hj):
+    """Refused however the matches divide into single ones of their probe row and listed
+    ones (here just under 2^32 of these), with buffers that would hold them all."""
+    import torch
+    L = hj.lib()
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 60 GB of free device memory")
+    heavy, hits, singles = 1 << 16, (1 << 16) - 1, 1 << 17
+    keys = torch.full((heavy + 1,), 7, dtype=torch.int32, device="cuda")
+    keys[heavy] = 8
+    probe = torch.cat([torch.full((hits,), 7), torch.full((singles,), 8)]).int().cuda()
+    rows = heavy * hits + singles
+    assert heavy * hits < 1 << 32 < rows
+    out = [torch.empty(rows, dtype=torch.int32, device="cuda") for _ in range(2)]
+    for o in out:
+        o[:1000] = -1
+    torch.cuda.synchronize()
+    nm, t = C.c_uint64(), C.c_void_p()
+    assert L.hj_table_build(engine.handle, keys.data_ptr(), None, heavy + 1, -1, C.byref(t)) == 0
+    try:
+        assert L.hj_table_probe(engine.handle, t, probe.data_ptr(), None, probe.numel(), out[0].data_ptr(),
+                                out[1].data_ptr(), rows, C.byref(nm)) == hj.HJ_ERR_INVALID
+        assert nm.value == rows and all(int(o[:1000].max()) == -1 for o in out)
+    finally:
+        L.hj_table_free(t)
