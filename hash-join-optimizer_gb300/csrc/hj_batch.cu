@@ -31,6 +31,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "hj_batch_size.h"
 #include "hj_block.cuh"
 #include "hj_common.cuh"
 #include "hj_kernels.h"
@@ -633,7 +634,7 @@ __global__ void __launch_bounds__(kBuildT, 2)
         __syncthreads();
         // a piece of n rows from the table memory, emptied; counters cleared
         auto open = [&](uint32_t n, Piece* p, uint32_t d) {
-            const uint32_t nbk = min(nbmax, uint32_t((uint64_t(n) * T.slot_q16) >> 16) + 1);
+            const uint32_t nbk = min(nbmax, batch_piece_buckets(n, T.slot_q16));
             if (threadIdx.x == 0) {
                 g_first = atomicAdd(T.next, nbk);
                 *p      = Piece{g_first, nbk | d};
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(kBuildT, 2)
             __syncthreads();
             return nbk;
         };
-        // a row's slot in the open piece (its rows fit: a quarter of the slots or more stays free)
+        // a row's slot in the open piece (its rows fit: a fifth of the slots or more stays free)
         auto place = [&](uint32_t nbk, int32_t k, int32_t p) {
             uint32_t b = home_of(k, nbk), r;
             while ((r = (atomicAdd(fcnt + (b >> 1), 1u << (16 * (b & 1))) >> (16 * (b & 1))) & 0xffffu) >= 4)
@@ -1049,7 +1050,7 @@ namespace {
 struct Geometry {
     uint64_t T;
     uint32_t cap, max_bits, scap, load_q8, fcap;
-    double   buckets_per_row;
+    uint32_t slot_q16;  // buckets per row, in 65536ths
     size_t   build_smem;
 };
 
@@ -1062,8 +1063,8 @@ Geometry geometry(const BatchOptions& o) {
     g.load_q8  = std::max<uint32_t>(1, uint32_t(std::lround(o.load * 256.0)));
     const size_t tables = size_t(g.cap) * 8 + size_t(g.scap) * 4;
     if (tables > 200 * 1024) throw Error(HJ_ERR_INVALID, "batch: partition tables exceed shared memory");
-    g.buckets_per_row = 0.25 / std::min(0.8, std::max(0.25, o.load));
-    g.fcap = uint32_t(std::min<uint64_t>(uint64_t(double(g.cap) * g.buckets_per_row) + 1, (220 * 1024 - tables) / 2));
+    g.slot_q16 = batch_buckets_q16(o.load);
+    g.fcap     = uint32_t(std::min<uint64_t>(batch_piece_buckets(g.cap, g.slot_q16), (220 * 1024 - tables) / 2));
     g.build_smem = tables + size_t(g.fcap) * 2 + 4;
     return g;
 }
@@ -1090,8 +1091,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     };
     const uint64_t T   = G.T;
     const uint32_t cap = G.cap, scap = G.scap, fcap = G.fcap, max_bits = G.max_bits, load_q8 = G.load_q8;
-    const double   buckets_per_row = G.buckets_per_row;
-    const size_t   build_smem      = G.build_smem;
+    const size_t   build_smem = G.build_smem;
     std::vector<RelInst>  hr;
     std::vector<InstInfo> hi(n);
     uint64_t pbase = 0, ipbase = 0, items = 0, build_rows = 0;
@@ -1141,7 +1141,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
         items += (br.rows + irows - 1) / irows;
     }
     const uint32_t nr   = uint32_t(hr.size());
-    const uint64_t nbkt = uint64_t(double(build_rows) * buckets_per_row) + pbase + 2;
+    const uint64_t nbkt = batch_table_buckets(build_rows, pbase, G.slot_q16);
 
     std::vector<InstOut> ho(n);
     std::vector<void*>   owned;
@@ -1182,7 +1182,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     auto* side   = static_cast<uint32_t*>(take(nbkt * 4 * stride * 4));
     HJ_CUDA(cudaMemcpyAsync(d_R, hd.data(), hd.size(), cudaMemcpyHostToDevice, st));
 
-    Tables tb{tabs, side, reinterpret_cast<uint32_t*>(d_q + 2), stride, uint32_t(std::lround(buckets_per_row * 65536.0))};
+    Tables tb{tabs, side, reinterpret_cast<uint32_t*>(d_q + 2), stride, G.slot_q16};
 
     auto enqueue = [&]() {
         HJ_CUDA(cudaMemsetAsync(d_out, 0, zero_bytes, st));
@@ -1286,7 +1286,7 @@ std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const B
                 bad.push_back(i1);
                 continue;
             }
-            const uint64_t need = uint64_t(double(nb) * (G.buckets_per_row * (32 + 16 * (kMaxRel - 2)) + 8));
+            const uint64_t need = uint64_t(double(nb) * (G.slot_q16 / 65536.0 * (32 + 16 * (kMaxRel - 2)) + 8));
             if (i1 > i0 && bytes + need > kWaveBytes) break;
             bytes += need;
         }
