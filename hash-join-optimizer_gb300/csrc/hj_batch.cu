@@ -1069,24 +1069,25 @@ Geometry geometry(const BatchOptions& o) {
     return g;
 }
 
-// Build rows of an instance, all build relations together; 0 when one of them has none (no result rows).
+// Build rows of an instance, all build relations together; 0 when any relation has none (no result rows).
 uint64_t build_rows_of(const BatchInstance& b) {
     uint64_t nb = 0;
-    for (size_t j = 1; j < b.rels.size(); ++j) {
+    for (size_t j = 0; j < b.rels.size(); ++j) {
         if (!b.rels[j].rows) return 0;
-        nb += b.rels[j].rows;
+        if (j) nb += b.rels[j].rows;
     }
     return nb;
 }
 
-// Instances [i0, i1) of the batch; the ones in `plain` (left to the plain path) as if without rows.
-void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1, const std::vector<uint8_t>& plain,
+// Instances [i0, i1) of the batch; the ones in `idle` (without result rows, or
+// left to the plain path) as if without rows.
+void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1, const std::vector<uint8_t>& idle,
                 const BatchOptions& o, const Geometry& G, BatchGraph& graph, uint64_t* rows, uint64_t* sums,
                 std::vector<uint32_t>& bad, cudaStream_t st) {
     const uint32_t n = i1 - i0;
     auto           rel_of = [&](uint32_t i, uint32_t j) {
         BatchRelation r = all[i0 + i].rels[j];
-        if (plain[i0 + i]) r.rows = 0;
+        if (idle[i0 + i]) r.rows = 0;
         return r;
     };
     const uint64_t T   = G.T;
@@ -1269,12 +1270,13 @@ std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const B
         }
     }
     const Geometry        G = geometry(o);
-    std::vector<uint8_t>  plain(n, 0);
+    std::vector<uint8_t>  idle(n, 0);
     std::vector<uint32_t> bad;
     // Waves of instances whose tables stay within kWaveBytes, so that a large
     // batch takes no more memory than the inputs' own size and a slot's number
     // fits 32 bits.  An instance with more build rows than its partitions can
-    // hold goes to the plain path at once.
+    // hold goes to the plain path at once; one with an empty relation has no
+    // result rows, and its other relations take no memory.
     constexpr uint64_t kWaveBytes = 24ull << 30;
     for (uint32_t i0 = 0; i0 < n;) {
         uint64_t bytes = 0;
@@ -1282,15 +1284,16 @@ std::vector<uint32_t> batch_execute(const std::vector<BatchInstance>& B, const B
         for (; i1 < n; ++i1) {
             const uint64_t nb = build_rows_of(B[i1]);
             if (nb > (uint64_t(G.cap) << kMaxPartBits)) {
-                plain[i1] = 1;
                 bad.push_back(i1);
+                idle[i1] = 1;
                 continue;
             }
+            idle[i1] = nb == 0;
             const uint64_t need = uint64_t(double(nb) * (G.slot_q16 / 65536.0 * (32 + 16 * (kMaxRel - 2)) + 8));
             if (i1 > i0 && bytes + need > kWaveBytes) break;
             bytes += need;
         }
-        batch_wave(B, i0, i1, plain, o, G, graph, rows.data(), sums.data(), bad, st);
+        batch_wave(B, i0, i1, idle, o, G, graph, rows.data(), sums.data(), bad, st);
         i0 = i1;
     }
     return bad;

@@ -1,0 +1,44 @@
+"""Device memory that calls take beyond their inputs and results, each call in a
+process of its own, where the memory that is in use is known."""
+from __future__ import annotations
+
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
+HEAD = """
+import ctypes as C, sys
+sys.path.insert(0, {root!r})
+import numpy as np, torch
+from __graft_entry__ import load
+hj = load()
+E, L = hj.Engine(0), hj.lib()
+def free(): return torch.cuda.mem_get_info()[0]
+def ints(n, v): return torch.full((n,), v, dtype=torch.int32, device="cuda")
+"""
+
+
+def run(code: str):
+    out = subprocess.run([sys.executable, "-c", HEAD.format(root=str(ROOT)) + code], capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0, out.stdout + out.stderr
+
+
+def test_batch_instance_with_an_empty_relation():
+    """Its other relations, however large, are neither partitioned nor built on."""
+    run("""
+n = 50_000_000
+big, small, none = ints(n, 3), ints(100, 3), ints(1, 3)
+def rel(t, rows=None): return (t.data_ptr(), t.data_ptr(), t.numel() if rows is None else rows)
+inst = [[rel(small), rel(small)], [rel(small), rel(big), rel(none, 0)], [rel(none, 0), rel(big)], [rel(small), rel(none, 0)]]
+torch.cuda.synchronize()
+E.batch_execute([inst[0]])
+before = free()
+rows, sums, redo = E.batch_execute(inst)
+assert list(rows) == [100 * 100, 0, 0, 0] and sums[1] == sums[2] == sums[3] == 0 and redo == 0
+assert before - free() < 4 * n, before - free()
+""")
