@@ -108,7 +108,7 @@ __global__ void k_batch_generate(uint64_t seed, uint32_t inst, uint32_t rel, uin
 //      key is in all go to the partition's piece of table F, their
 //      partners' payloads beside the slot                           k_bt_build
 //   5. R0 rows looked up in F                                       k_bt_probe
-//   6. R0 rows of instances with duplicate keys in R2, R3, ...      k_bt_enum
+//   6. R0 rows whose key repeats: their results enumerated          k_bt_enum
 // Instance i gets p_i partition bits (about `part_rows` build rows per
 // partition summed over its build relations); a row belongs to partition
 // top_p_i(hash(key)).  A partition whose build rows exceed the shared-memory
@@ -138,6 +138,7 @@ struct RelInst {  // one relation of one instance
     uint32_t       inst;
     uint32_t       irows;  // R0s: rows per work item
     uint32_t       nrel;
+    uint32_t       fbase;  // R0s: first word of the instance's filter
 };
 
 // One work item of the probe, whole, so that a block waits for one load.
@@ -145,6 +146,7 @@ struct Item {
     const int32_t *k, *p;
     uint64_t       part_base;
     uint32_t       n, inst, pbits, nt;  // rows; instance; its partition bits and tables beside F
+    uint32_t       fbase;               // and the first word of its filter
 };
 
 struct InstInfo {
@@ -152,13 +154,14 @@ struct InstInfo {
     uint64_t ip_base;    // first instance partition (2^pbits of them)
     uint32_t nrel;
     uint32_t pbits;
+    uint32_t fbase;      // first word of its filter (2^(pbits + filter_log - 5) of them)
 };
 
 // Per-instance results and flags, cleared together.
 struct InstOut {
     unsigned long long rows, sum;
     uint32_t           ovf;   // a partition too large for shared memory, or a row equal to kFree
-    uint32_t           dups;  // R2, R3, ... hold a key of R1 more than once: partners are enumerated
+    uint32_t           lists;  // its partitions with listed keys (k_bt_enum)
 };
 
 // A table in buckets of four (key, payload) slots, 32 bytes (one L2 sector,
@@ -168,12 +171,32 @@ struct InstOut {
 // descending order, else ascending, so a lookup goes on only from those (5% of
 // the buckets at half load; 14% are full).
 // A piece is the part of a table that one instance partition's rows are in:
-// its first bucket, and its buckets | kDup when partners are enumerated from
-// the pieces of R2, R3, ....  Pieces without rows are bucket 0, which is free.
+// its first bucket, and its buckets.  Pieces without rows are bucket 0, which is
+// free.
+// Keys that R2, R3, ... hold more than once, and keys with so many rows in R1 that
+// they would fill runs of buckets which every lookup beside them walks, are not
+// in F.  Their partition has a piece of listed keys for each of its relations: a
+// slot a key, with the end of the key's list of payloads in place of a payload.
+// The lists take the place of the partitioned rows, the last row of each with
+// the list's length.  (A wave has fewer rows than 2^31, so an end is no kFree's.)
 struct Piece {
-    uint32_t first, nbk;
+    uint32_t first, nbk;  // nbk 0: no listed keys
 };
-constexpr uint32_t kDup = 1u << 31;
+// F is filled anew, without the keys of home buckets of more than kHeavy rows,
+// when linear probing takes more than kSteps steps a row.  64 chains of 8,000
+// build rows, 7,900 of one key, us: 410 (all of them in F: 10,044); of 16,000
+// Zipf(0.8) rows 512 (1,235), Zipf(1.1) 562 (5,361).  kSteps at 1 gives up keys of 8
+// rows each, which are as fast in F (497, 411); at 4 uniform keys of 16 rows stay
+// (614, 525).
+constexpr uint32_t kSteps = 2, kHeavy = 12;
+// A filter of an instance's listed keys, for those who look for rows of them: two
+// bits of a word a key, each partition with words of its own, at most as many as
+// fit a block's shared memory (2^17 bits).  Few rows of other keys pass it, and
+// what passes takes three dependent loads.
+constexpr uint32_t kFilterPart = 13, kFilterAll = 17;
+__host__ __device__ __forceinline__ uint32_t filter_log(uint32_t pbits) {
+    return kFilterAll - pbits < kFilterPart ? kFilterAll - pbits : kFilterPart;
+}
 
 // A free slot.  A build row that is this very pair cannot be stored: its
 // instance is left to the plain path.
@@ -240,6 +263,8 @@ struct Tables {
     uint64_t* tab;
     uint32_t* side;      // `stride` words per slot: the payloads of an F slot's partners
     uint32_t* next;      // buckets handed out, from 1 on
+    uint32_t* lists;     // zeroed; set when any partition has listed keys
+    uint32_t  buckets;   // of the memory
     uint32_t  stride;
     uint32_t  slot_q16;  // buckets per row, in 65536ths
 };
@@ -268,7 +293,7 @@ __global__ void k_item_rel(const RelInst* __restrict__ R, uint32_t nr, uint64_t 
         const RelInst& r  = R[ri];
         const uint64_t r0 = (t - r.item_base) * r.irows;
         imap[t - bitems]  = Item{r.keys + r0, r.pay + r0, r.part_base, uint32_t(min(r.rows - r0, uint64_t(r.irows))),
-                                r.inst, r.pbits, r.nrel - 2};
+                                r.inst, r.pbits, r.nrel - 2, r.fbase};
     }
 }
 
@@ -437,11 +462,17 @@ __device__ __forceinline__ Slots load_bucket(const uint64_t* tab, uint64_t b) {
 // partition's multiplicative hash will not do: keys in arithmetic progression
 // can fall into few of its buckets, and linear probing then runs through them
 // (64 chains of 1k .. 16k build rows: 148 us of probing, with this hash 41 us).
-__device__ __forceinline__ uint32_t home_of(int32_t k, uint32_t nbk) {
+__device__ __forceinline__ uint32_t mix_of(int32_t k) {
     uint32_t h = uint32_t(k);
     h = (h ^ (h >> 16)) * 0x85ebca6bu;
-    h = (h ^ (h >> 13)) * 0xc2b2ae35u;
-    return __umulhi(h, nbk);
+    return (h ^ (h >> 13)) * 0xc2b2ae35u;
+}
+__device__ __forceinline__ uint32_t home_of(int32_t k, uint32_t nbk) { return __umulhi(mix_of(k), nbk); }
+// A key's bits in a partition's 2^log bits of the filter, and the word that they are in.
+__device__ __forceinline__ uint32_t filter_bits(int32_t k, uint32_t log, uint32_t& word) {
+    const uint32_t h = mix_of(k);
+    word             = (h >> 10) & ((1u << (log - 5)) - 1);
+    return (1u << (h & 31)) | (1u << ((h >> 5) & 31));
 }
 __device__ __forceinline__ uint64_t slot_of(int32_t k, int32_t p) {
     return uint64_t(uint32_t(k)) | (uint64_t(uint32_t(p)) << 32);
@@ -450,38 +481,6 @@ __device__ __forceinline__ int32_t slot_key(uint64_t s) { return int32_t(uint32_
 __device__ __forceinline__ int32_t slot_pay(uint64_t s) { return int32_t(uint32_t(s >> 32)); }
 __device__ __forceinline__ bool goes_on(const Slots& s) { return s.s[2] >= s.s[3] && s.s[3] != kFree; }
 __device__ __forceinline__ uint32_t next_bucket(uint32_t b, uint32_t nbk) { return b + 1 == nbk ? 0u : b + 1; }
-
-// Walks the rows of key k in a table, in slot order.
-struct Walk {
-    const uint64_t* tab;
-    uint32_t        nbk, b, left;
-    int32_t         k;
-    Slots           s;
-    int             i;
-    Walk() = default;
-    __device__ __forceinline__ Walk(const uint64_t* tab_, uint32_t nbk_, int32_t k_)
-        : tab(tab_), nbk(nbk_), b(home_of(k_, nbk_)), left(nbk_), k(k_), i(0) {
-        s = load_bucket(tab, b);
-    }
-    // the next such row: its payload and slot in the piece; false at the end
-    __device__ __forceinline__ bool next(int32_t& pay, uint64_t& slot) {
-        for (;;) {
-            for (; i < 4; ++i) {
-                const uint64_t v = i == 0 ? s.s[0] : i == 1 ? s.s[1] : i == 2 ? s.s[2] : s.s[3];
-                if (slot_key(v) == k && v != kFree) {
-                    pay  = slot_pay(v);
-                    slot = uint64_t(b) * 4 + i++;
-                    return true;
-                }
-            }
-            if (!goes_on(s) || --left == 0) return false;
-            b = next_bucket(b, nbk);
-            s = load_bucket(tab, b);
-            i = 0;
-        }
-    }
-};
-
 
 __device__ __forceinline__ uint64_t part_rows(const uint64_t* off, uint64_t pid) { return off[pid + 1] - off[pid]; }
 
@@ -494,19 +493,22 @@ __device__ __forceinline__ uint64_t part_rows(const uint64_t* off, uint64_t pid)
 // R1's rows are looked up twice: counted, so that the piece is as large as its
 // rows need (tables of long chains shrink with every relation), then placed.
 // Bound by the latency of its phases: two blocks an SM, each at another one.
+// Listed keys take some 13 us more a block (8 chains of 1M rows, a hundredth
+// repeated in R2: 428 us, without 248): each relation's table is made by atomics
+// on its slots in L2, counts first, then the lists' starts, then the rows.
 constexpr int kBuildT = 512;
 __global__ void __launch_bounds__(kBuildT, 2)
     k_bt_build(const InstInfo* __restrict__ I, const uint32_t* __restrict__ pmap, uint64_t nip,
-               const uint64_t* __restrict__ off, const int2* __restrict__ kp, uint32_t cap, uint32_t scap,
-               uint32_t fcap, uint32_t max_bits, uint32_t load_q8,
-               Tables T, Piece* __restrict__ pieces, InstOut* __restrict__ out) {
+               const uint64_t* __restrict__ off, int2* kp, uint32_t cap, uint32_t scap, uint32_t fcap,
+               uint32_t max_bits, uint32_t load_q8, Tables T, Piece* __restrict__ pieces, Piece* __restrict__ listed,
+               uint32_t* __restrict__ filters, InstOut* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem[];
     int32_t*  skey = reinterpret_cast<int32_t*>(smem);
     int32_t*  spay = skey + cap;
     uint32_t* S    = reinterpret_cast<uint32_t*>(spay + cap);
     __shared__ uint32_t wsum[32];
-    __shared__ uint32_t g_tb[kMaxRel], g_tn[kMaxRel], g_ts[kMaxRel], g_to[kMaxRel + 1], g_words, g_skip, g_cnt, g_flags,
-        g_first;
+    __shared__ uint32_t g_tb[kMaxRel], g_tn[kMaxRel], g_ts[kMaxRel], g_to[kMaxRel + 1], g_words, g_skip, g_cnt, g_nl,
+        g_first, g_steps;
     __shared__ uint64_t g_src[kMaxRel];
     for (uint64_t e = blockIdx.x; e < nip; e += gridDim.x) {
         const uint32_t  ii  = pmap[e];
@@ -551,9 +553,9 @@ __global__ void __launch_bounds__(kBuildT, 2)
             const bool big = all > cap || words > scap;
             if (big && !empty) out[ii].ovf = 1;
             g_skip  = big || empty;
-            g_cnt   = 0;
-            g_flags = 0;
-            if (empty || big) pieces[pid] = Piece{0, 1};
+            g_cnt = g_nl = 0;
+            pieces[pid]  = Piece{0, 1};
+            listed[pid]  = Piece{0, 0};
         }
         __syncthreads();
         if (g_skip) continue;
@@ -612,89 +614,278 @@ __global__ void __launch_bounds__(kBuildT, 2)
                 }
             return c;
         };
-        // R1 rows that are in every table: how many, and whether any has several partners
-        uint32_t mine = nt == 0 && threadIdx.x == 0 ? n1 : 0u, dup = 0;
+        // R1 rows that are in every table, and the ones of them whose key a table
+        // holds more than once: bits of this thread's rows, and how many
         static_assert((2u << 13) / kBuildT <= 32, "a bit for each of a thread's rows");
-        uint32_t found = nt ? 0u : ~0u;  // this thread's rows that are
-        for (uint32_t r = threadIdx.x, i = 0; nt && r < n1; r += kBuildT, ++i) {
-            const int32_t k   = __ldg(r1 + r).x;
-            bool          all = true;
-            for (uint32_t j = 0; j < nt && all; ++j) {
-                uint32_t       y;
-                const uint32_t c = lookup(j, k, y);
-                all              = c > 0;
-                dup |= c > 1;
+        uint32_t in_f = 0, in_l = 0;
+        for (uint32_t r = threadIdx.x, i = 0; r < n1; r += kBuildT, ++i) {
+            bool all = true, many = false;
+            if (nt) {
+                const int32_t k = __ldg(r1 + r).x;
+                for (uint32_t j = 0; j < nt && all; ++j) {
+                    uint32_t       y;
+                    const uint32_t c = lookup(j, k, y);
+                    all              = c > 0;
+                    many |= c > 1;
+                }
             }
-            mine += all;
-            found |= uint32_t(all) << i;
+            in_f |= uint32_t(all && !many) << i;
+            in_l |= uint32_t(all && many) << i;
         }
-        mine = warp_sum(mine);
-        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&g_cnt, mine);
-        if (dup) g_flags = 1;
+        auto count_rows = [&](uint32_t bits, uint32_t* to) {
+            const uint32_t c = warp_sum(uint32_t(__popc(bits)));
+            if ((threadIdx.x & 31) == 0 && c) atomicAdd(to, c);
+        };
+        count_rows(in_f, &g_cnt);
+        count_rows(in_l, &g_nl);
         __syncthreads();
-        // a piece of n rows from the table memory, emptied; counters cleared
-        auto open = [&](uint32_t n, Piece* p, uint32_t d) {
-            const uint32_t nbk = min(nbmax, batch_piece_buckets(n, T.slot_q16));
+        // Buckets from the table memory, at g_first (it is sized for all of them; were
+        // it short, the instance would go to the plain path)
+        auto reserve = [&](uint32_t nbk) {
+            __syncthreads();
             if (threadIdx.x == 0) {
                 g_first = atomicAdd(T.next, nbk);
-                *p      = Piece{g_first, nbk | d};
+                if (g_first > T.buckets || nbk > T.buckets - g_first) out[ii].ovf = g_skip = 1;
             }
-            for (uint32_t b = threadIdx.x; b < (nbk + 1) / 2; b += kBuildT) fcnt[b] = 0;
             __syncthreads();
-            ulonglong2* to = reinterpret_cast<ulonglong2*>(T.tab + 4 * uint64_t(g_first));
+            return g_skip == 0;
+        };
+        // its slots emptied, and `words` counters beside it
+        auto empty = [&](uint32_t first, uint32_t nbk, uint32_t* cnt, uint32_t words) {
+            __syncthreads();
+            for (uint32_t w = threadIdx.x; w < words; w += kBuildT) cnt[w] = 0;
+            ulonglong2* to = reinterpret_cast<ulonglong2*>(T.tab + 4 * uint64_t(first));
             for (uint32_t b = threadIdx.x; b < 2 * nbk; b += kBuildT) to[b] = make_ulonglong2(kFree, kFree);
             __syncthreads();
-            return nbk;
         };
-        // a row's slot in the open piece (its rows fit: a fifth of the slots or more stays free)
-        auto place = [&](uint32_t nbk, int32_t k, int32_t p) {
-            uint32_t b = home_of(k, nbk), r;
-            while ((r = (atomicAdd(fcnt + (b >> 1), 1u << (16 * (b & 1))) >> (16 * (b & 1))) & 0xffffu) >= 4)
-                b = next_bucket(b, nbk);
-            const uint64_t slot = uint64_t(g_first + b) * 4 + r, v = slot_of(k, p);
-            T.tab[slot] = v;
-            if (v == kFree) out[ii].ovf = 1;
-            return slot;
+        auto buckets = [&](uint32_t n) { return min(nbmax, batch_piece_buckets(n, T.slot_q16)); };
+        // f(bit, row, key, payload) for R1's rows in `bits`
+        auto rows_of = [&](uint32_t bits, auto f) {
+            for (; bits; bits &= bits - 1) {
+                const uint32_t i = __ffs(bits) - 1, r = i * kBuildT + threadIdx.x;
+                const int2     kv = __ldg(r1 + r);
+                f(1u << i, r, kv.x, kv.y);
+            }
         };
-        // the order of each full bucket's last slots (and, in F, of their partners)
-        auto close = [&](uint32_t nbk, uint32_t words) {
+        auto add = [&](uint32_t b) {
+            return (atomicAdd(fcnt + (b >> 1), 1u << (16 * (b & 1))) >> (16 * (b & 1))) & 0xffffu;
+        };
+        uint32_t nf = g_cnt, nl = g_nl, nbk = 0;
+        if (nf + nl == 0) continue;
+        // F's piece and behind it R1's listed keys, however the rows divide
+        if (!reserve(batch_pair_buckets(nf + nl, T.slot_q16))) continue;
+        const uint32_t first = g_first;
+        // F: a slot a row (they fit: a fifth of the slots or more stays free)
+        for (uint32_t limit = kSteps * nf; nf; limit = ~0u) {
+            nbk = buckets(nf);
+            if (threadIdx.x == 0) g_steps = 0;
+            empty(first, nbk, fcnt, (nbk + 1) / 2);
+            uint32_t steps = 0;  // past full buckets; in g_steps 8 at a time
+            rows_of(in_f, [&](uint32_t, uint32_t, int32_t k, int32_t p) {
+                if (*const_cast<volatile uint32_t*>(&g_steps) > limit) return;
+                uint32_t b = home_of(k, nbk), r;
+                while ((r = add(b)) >= 4) {
+                    b = next_bucket(b, nbk);
+                    if ((++steps & 7) == 0 && atomicAdd(&g_steps, 8u) >= limit) return;
+                }
+                const uint64_t slot = uint64_t(first + b) * 4 + r, v = slot_of(k, p);
+                T.tab[slot] = v;
+                if (v == kFree) out[ii].ovf = 1;
+                for (uint32_t j = 0; j < nt; ++j) {
+                    uint32_t y = 0;
+                    lookup(j, k, y);
+                    T.side[slot * T.stride + j] = uint32_t(spay[y]);
+                }
+            });
+            steps = warp_sum(steps & 7);
+            if ((threadIdx.x & 31) == 0 && steps) atomicAdd(&g_steps, steps);
             __syncthreads();
+            if (limit == ~0u || g_steps <= limit) break;
+            // the keys of heavy home buckets are listed, and F takes the others
+            for (uint32_t b = threadIdx.x; b < (nbk + 1) / 2; b += kBuildT) fcnt[b] = 0;
+            __syncthreads();
+            rows_of(in_f, [&](uint32_t, uint32_t, int32_t k, int32_t) { add(home_of(k, nbk)); });
+            __syncthreads();
+            uint32_t heavy = 0;
+            rows_of(in_f, [&](uint32_t bit, uint32_t, int32_t k, int32_t) {
+                if (count(home_of(k, nbk)) > kHeavy) heavy |= bit;
+            });
+            in_f &= ~heavy;
+            in_l |= heavy;
+            count_rows(heavy, &g_nl);
+            __syncthreads();
+            nf -= g_nl - nl;
+            nl = g_nl;
+        }
+        if (nf) {
+            if (threadIdx.x == 0) pieces[pid] = Piece{first, nbk};
+            // the order of each full bucket's last slots, and of their partners
             for (uint32_t b = threadIdx.x; b < nbk; b += kBuildT) {
                 const uint32_t n = count(b);
                 if (n < 4) continue;
-                const uint64_t c = uint64_t(g_first + b) * 4 + 2;
+                const uint64_t c = uint64_t(first + b) * 4 + 2;
                 const uint64_t x = T.tab[c], y = T.tab[c + 1];
                 if ((n > 4) == (x >= y)) continue;
                 T.tab[c]     = y;
                 T.tab[c + 1] = x;
-                for (uint32_t j = 0; j < words; ++j) {
+                for (uint32_t j = 0; j < nt; ++j) {
                     const uint32_t w                  = T.side[c * T.stride + j];
                     T.side[c * T.stride + j]          = T.side[(c + 1) * T.stride + j];
                     T.side[(c + 1) * T.stride + j]    = w;
                 }
             }
-        };
-        const uint32_t fl  = g_flags ? kDup : 0u;
-        const uint32_t nbk = open(g_cnt, pieces + pid, fl);
-        for (uint32_t r = threadIdx.x; r < n1; r += kBuildT, found = nt ? found >> 1 : ~0u) {
-            if (!(found & 1u)) continue;
-            const int2     kv   = __ldg(r1 + r);
-            const uint64_t slot = place(nbk, kv.x, kv.y);
-            for (uint32_t j = 0; j < nt; ++j) {
-                uint32_t y = 0;
-                lookup(j, kv.x, y);
-                T.side[slot * T.stride + j] = uint32_t(spay[y]);
-            }
+        } else {
+            nbk = 0;
         }
-        close(nbk, nt);
-        // duplicates: R2, R3, ... as pieces too
-        if (fl) {
-            if (threadIdx.x == 0) out[ii].dups = 1;
-            for (uint32_t j = 0; j < nt; ++j) {
+        if (nl == 0) continue;
+        // The listed keys.  R1's rows of them come to the others' in shared memory,
+        // as the lists take the place of what has been read.
+        __syncthreads();
+        const uint32_t o1 = nt ? g_to[nt - 1] + g_tn[nt - 1] : 0u;
+        const uint32_t flog = filter_log(pb);
+        uint32_t*      filter = S + scap + (fcap + 1) / 2;
+        for (uint32_t w = threadIdx.x; w < 1u << (flog - 5); w += kBuildT) filter[w] = 0;
+        __syncthreads();
+        rows_of(in_l, [&](uint32_t, uint32_t r, int32_t k, int32_t p) {
+            skey[o1 + r]     = k;
+            spay[o1 + r]     = p;
+            uint32_t       w;
+            const uint32_t m = filter_bits(k, flog, w);
+            atomicOr(filter + w, m);
+        });
+        __syncthreads();
+        for (uint32_t w = threadIdx.x; w < 1u << (flog - 5); w += kBuildT)
+            filters[s.fbase + (uint32_t(l) << (flog - 5)) + w] = filter[w];
+        if (threadIdx.x == 0) {
+            atomicAdd(&out[ii].lists, 1u);
+            *T.lists = 1;
+        }
+        const uint32_t  behind_f = first + nbk;
+        uint32_t*       passed = S + scap;  // a bit a bucket: a key went past it
+        const uint64_t* keys   = nullptr;   // R1's piece
+        uint32_t        nbk1   = 0;
+        // (this block's atomics and stores of a moment ago: past the L1)
+        auto fresh = [&](const uint64_t* tab, uint32_t b) {
+            Slots q;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q.s[i] = *const_cast<const volatile uint64_t*>(tab + 4 * b + i);
+            return q;
+        };
+        auto slot_in = [&](const Slots& q, int32_t k) {
+            int at = -1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (q.s[i] != kFree && slot_key(q.s[i]) == k) at = i;
+            return at;
+        };
+        for (uint32_t j = 0; j <= nt; ++j) {
+            const uint32_t o = j ? g_to[j - 1] : o1;
+            const uint32_t dst = uint32_t(j ? g_src[j - 1] : off[pid]);
+            uint32_t       bits = in_l;
+            if (j) {  // the rows whose key is listed
+                bits = 0;
+                for (uint32_t r = threadIdx.x, i = 0; r < g_tn[j - 1]; r += kBuildT, ++i) {
+                    const int32_t  k = skey[o + r];
+                    uint32_t       w;
+                    const uint32_t m = filter_bits(k, flog, w);
+                    if ((filter[w] & m) != m) continue;
+                    for (uint32_t b = home_of(k, nbk1);; b = next_bucket(b, nbk1)) {
+                        const Slots q    = fresh(keys, b);
+                        const bool  here = slot_in(q, k) >= 0;
+                        bits |= uint32_t(here) << i;
+                        if (here || !goes_on(q)) break;
+                    }
+                }
+                if (threadIdx.x == 0) g_nl = 0;
                 __syncthreads();
-                const uint32_t tn = g_tn[j], nb = open(tn, pieces + pid + (j + 1) * np2, 0);
-                for (uint32_t r = threadIdx.x; r < tn; r += kBuildT) place(nb, skey[g_to[j] + r], spay[g_to[j] + r]);
-                close(nb, 0);
+                count_rows(bits, &g_nl);
+            }
+            auto each = [&](auto f) {
+                for (uint32_t m = bits; m; m &= m - 1) {
+                    const uint32_t r = o + (__ffs(m) - 1) * kBuildT + threadIdx.x;
+                    f(skey[r], spay[r]);
+                }
+            };
+            __syncthreads();
+            const uint32_t nbk = buckets(g_nl);
+            if (j && !reserve(nbk)) break;
+            const uint32_t lf = j ? g_first : behind_f;
+            if (threadIdx.x == 0) listed[pid + j * np2] = Piece{lf, nbk};
+            empty(lf, nbk, passed, (nbk + 31) / 32);
+            uint64_t* const tab = T.tab + 4 * uint64_t(lf);
+            auto word = [&](uint64_t slot) { return reinterpret_cast<uint32_t*>(tab + slot) + 1; };
+            // each key's slot, with the number of its rows
+            each([&](int32_t k, int32_t) {
+                for (uint32_t b = home_of(k, nbk);; b = next_bucket(b, nbk)) {
+                    const Slots q  = fresh(tab, b);
+                    int         at = -1;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (at >= 0) continue;
+                        uint64_t v = q.s[i];
+                        if (v == kFree) {
+                            v = atomicCAS(reinterpret_cast<unsigned long long*>(tab + 4 * b + i), kFree, slot_of(k, 0));
+                            if (v == kFree) v = slot_of(k, 0);
+                        }
+                        if (slot_key(v) == k) at = i;
+                    }
+                    if (at >= 0) {
+                        atomicAdd(word(4 * b + at), 1u);
+                        break;
+                    }
+                    atomicOr(passed + (b >> 5), 1u << (b & 31));
+                }
+            });
+            __syncthreads();
+            // the number becomes the list's start
+            uint32_t at = dst;
+            for (uint32_t b0 = 0; b0 < nbk; b0 += kBuildT) {
+                const uint32_t b = b0 + threadIdx.x;
+                uint32_t       c[4], sum = 0;
+                Slots          q;
+                if (b < nbk) q = fresh(tab, b);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    c[i] = b < nbk && q.s[i] != kFree ? uint32_t(slot_pay(q.s[i])) : 0u;
+                    sum += c[i];
+                }
+                const uint32_t inc = warp_inclusive_scan(sum);
+                if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = inc;
+                __syncthreads();
+                uint32_t x = at + inc - sum;
+                for (uint32_t w = 0; w < kBuildT / 32; ++w) {
+                    if (w < threadIdx.x >> 5) x += wsum[w];
+                    at += wsum[w];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!c[i]) continue;
+                    *word(4 * b + i) = x;
+                    x += c[i];
+                    kp[x - 1].y = int32_t(c[i]);
+                }
+                __syncthreads();
+            }
+            // and, with the rows' payloads in place, its end
+            each([&](int32_t k, int32_t p) {
+                for (uint32_t b = home_of(k, nbk);; b = next_bucket(b, nbk)) {
+                    const int at = slot_in(fresh(tab, b), k);
+                    if (at < 0) continue;
+                    kp[atomicAdd(word(4 * b + at), 1u)].x = p;
+                    break;
+                }
+            });
+            __syncthreads();
+            for (uint32_t b = threadIdx.x; b < nbk; b += kBuildT) {
+                const Slots q = fresh(tab, b);
+                if (q.s[3] == kFree || ((passed[b >> 5] >> (b & 31)) & 1u) == (q.s[2] >= q.s[3])) continue;
+                tab[4 * b + 2] = q.s[3];
+                tab[4 * b + 3] = q.s[2];
+            }
+            __syncthreads();
+            if (j == 0) {
+                keys = tab;
+                nbk1 = nbk;
             }
         }
     }
@@ -731,8 +922,8 @@ struct Sums {
 // together, and rows that have to go on to a next bucket (one in twenty at half
 // load, some in every warp) until 32 of them look together.  The instance's
 // pieces are kept in shared memory (reads of them through L1 would cost as
-// much as the buckets).  Each match of a key in F is a result row, unless R2,
-// R3, ... hold duplicates (k_bt_enum).
+// much as the buckets).  Each match of a key in F is a result row; listed keys are
+// not in it.
 constexpr uint32_t kQueue = 96;  // a step leaves at most 31 rows and adds at most 32 * kU
 static_assert(31 + 32 * kU <= int(kQueue), "a step's rows fit the queues");
 struct Queues {
@@ -835,7 +1026,7 @@ __global__ void __launch_bounds__(kBT, 4)
             go_on(0);
             fold(0);
             acc.at(it.inst, out);
-            skip = out[it.inst].ovf || out[it.inst].dups;
+            skip = out[it.inst].ovf;
             pb   = it.pbits;
             nt   = it.nt;
             __syncthreads();
@@ -885,92 +1076,187 @@ __global__ void __launch_bounds__(kBT, 4)
     acc.at(~0u, out);
 }
 
-// 6. The same for instances whose R2, R3, ... hold a key of R1 more than once:
-// each F row of the key with every combination of one partner per table (an
-// odometer).  Up to kKeep partners a table are kept in the thread; a table
-// with more is walked for every combination of the tables before it.
-__global__ void __launch_bounds__(kBT)
+// 6. The rows whose key is listed.  Their keys are looked for in the filter, kEU a
+// lane in flight and the next ones on their way; those that it holds wait in the
+// warp's queue until 32 of them are looked up in every relation, a lane each.  A
+// row's results are the combinations of one payload a list.  The warp shares out those
+// of its rows together: of a row with kMany of them by themselves, else by a
+// search of the running sums.
+// Bound by the scan of R0's keys where few are listed (360e9 rows/s, half of the
+// warps waiting for shared memory), so what a listed row needs is kept out of its
+// registers.  Results by the rows' own lanes instead: 64 chains of 16,000 rows, 16 a
+// key, half of R0's rows with a partner 1,836 us, so 1,080.
+constexpr int      kEU     = 8;
+constexpr uint32_t kMany   = 64;
+constexpr uint32_t kMaxTab = kMaxRel - 1;
+struct EnumRows {
+    int2     queue[32 * (kEU + 1)];  // key and row; a step leaves at most 31 and adds 32 * kEU
+    uint64_t fp[32];                 // of the 32 rows: key and R0's payload folded
+    uint32_t before[32];             // results of the rows before
+    uint32_t start[kMaxTab][32], len[kMaxTab][32];
+};
+// What the rows of an instance are looked up in.
+struct EnumOf {
+    const uint64_t* tabs;
+    const int2*     kp;
+    const Piece*    listed;  // of R1's partition 0
+    const int32_t*  pay;     // R0's payloads; the queue's rows count from here
+    uint32_t        pb, nt;
+};
+// The results of the queue's n rows from q on.  (Not inlined: its registers would
+// be the scan's.)
+__device__ __noinline__ void enum_rows(EnumRows& W, const EnumOf& I, uint32_t q, uint32_t n, Sums& acc) {
+    const unsigned lane = threadIdx.x & 31;
+    const uint32_t nt   = I.nt;
+    const int2*    kp   = I.kp;
+    uint64_t       total = 0, sum = 0;
+    uint32_t       done = 0;
+    // a result: row r's combination c
+    auto result = [&](uint32_t r, auto c) {
+        uint32_t at[kMaxTab];
+#pragma unroll
+        for (int j = kMaxTab - 1; j > 0; --j) {
+            if (j > int(nt)) continue;
+            const uint32_t l = W.len[j][r];
+            const auto     d = c / l;
+            at[j] = uint32_t(c - d * l);
+            c     = d;
+        }
+        at[0]       = uint32_t(c);
+        uint64_t fp = W.fp[r];
+#pragma unroll
+        for (int j = 0; j < int(kMaxTab); ++j)
+            if (j <= int(nt)) fp = fp_add(fp, __ldg(&kp[W.start[j][r] + at[j]].x));
+        ++done;
+        sum += fp_final(fp);
+    };
+    __syncwarp();
+    if (lane < n) {
+        const int2    r    = W.queue[q + lane];
+        const int32_t p    = __ldcs(I.pay + uint32_t(r.y));
+        const Piece*  part = I.listed + part_of(r.x, I.pb);
+        total              = 1;
+        for (uint32_t j = 0; j <= nt && total; ++j) {
+            const Piece x   = part[uint64_t(j) << I.pb];
+            uint32_t    end = 0, len = 0;
+            for (uint32_t b = home_of(r.x, x.nbk);; b = next_bucket(b, x.nbk)) {
+                const Slots s = load_bucket(I.tabs, uint64_t(x.first) + b);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (s.s[i] != kFree && slot_key(s.s[i]) == r.x) end = uint32_t(slot_pay(s.s[i]));
+                if (end || !goes_on(s)) break;
+            }
+            if (end) len = uint32_t(__ldg(&kp[end - 1].y));
+            W.start[j][lane] = end - len;
+            W.len[j][lane]   = len;
+            total *= len;
+        }
+        W.fp[lane] = fp_start(r.x, p);
+    }
+    const uint32_t few = total < kMany ? uint32_t(total) : 0u;
+    const uint32_t inc = warp_inclusive_scan(few), all = __shfl_sync(0xffffffffu, inc, 31);
+    W.before[lane]     = inc - few;
+    __syncwarp();
+    for (uint32_t i = lane; i < all; i += 32) {
+        uint32_t r = 0;  // the last row with at most i results before it (one without results shares the next one's number)
+#pragma unroll
+        for (uint32_t d = 16; d; d >>= 1)
+            if (W.before[r + d] <= i) r += d;
+        result(r, i - W.before[r]);
+    }
+    for (unsigned big = __ballot_sync(0xffffffffu, total >= kMany); big; big &= big - 1) {
+        const int      r = __ffs(big) - 1;
+        const uint64_t t = __shfl_sync(0xffffffffu, total, r);
+        if (nt == 0) {
+            const uint64_t fp = W.fp[r];
+            const int2*    l  = kp + W.start[0][r];
+            for (uint32_t c = lane; c < t; c += 32, ++done) sum += fp_final(fp_add(fp, __ldg(&l[c].x)));
+        } else if (t <= 0xffffffe0ull) {
+            for (uint32_t c = lane; c < t; c += 32) result(uint32_t(r), c);
+        } else {
+            for (uint64_t c = lane; c < t; c += 32) result(uint32_t(r), c);
+        }
+    }
+    acc.rows += done;
+    acc.sum += sum;
+    __syncwarp();
+}
+
+constexpr size_t kEnumSmem = sizeof(EnumRows) * (kBT / 32) + (size_t(1) << kFilterAll) / 8;
+__global__ void __launch_bounds__(kBT, 3)
     k_bt_enum(const Item* __restrict__ imap, uint64_t items, const uint64_t* __restrict__ tabs,
-              const uint32_t* __restrict__ side, uint32_t stride, const Piece* __restrict__ pieces,
-              InstOut* __restrict__ out) {
-    constexpr int kKeep = 8;
-    Sums          acc;
+              const int2* __restrict__ kp, const Piece* __restrict__ listed, const uint32_t* __restrict__ filters,
+              const uint32_t* __restrict__ any, InstOut* __restrict__ out) {
+    if (!*any) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    EnumRows&      W      = reinterpret_cast<EnumRows*>(smem)[threadIdx.x >> 5];
+    uint32_t*      filter = reinterpret_cast<uint32_t*>(smem + sizeof(EnumRows) * (kBT / 32));  // the instance's
+    const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1;
+    uint32_t       qn   = 0, pb = 0, flog = 0;
+    EnumOf         I{tabs, kp, listed, nullptr, 0, 0};
+    Sums           acc;
     for (uint64_t t = blockIdx.x; t < items; t += gridDim.x) {
         const Item it = imap[t];
-        if (out[it.inst].ovf || !out[it.inst].dups) continue;
-        const uint32_t nt = it.nt, pb = it.pbits;
-        // walk over key k's rows of relation j + 1
-        auto walk = [&](uint32_t j, int32_t k) {
-            const Piece x = pieces[it.part_base + (uint64_t(j) << pb) + part_of(k, pb)];
-            return Walk(tabs + 4 * uint64_t(x.first), x.nbk & ~kDup, k);
+        if (out[it.inst].ovf || !out[it.inst].lists) continue;
+        if (it.inst != acc.cur) {
+            if (qn) enum_rows(W, I, 0, qn, acc);
+            qn = 0;
+            acc.at(it.inst, out);
+            pb   = it.pbits;
+            flog = filter_log(pb);
+            I    = EnumOf{tabs, kp, listed + it.part_base, it.p, pb, it.nt};
+            __syncthreads();
+            const uint32_t words = 1u << (pb + flog - 5);
+            for (uint32_t w0 = threadIdx.x; w0 < words; w0 += 8 * kBT) {
+                uint32_t v[8], on[8];
+#pragma unroll
+                for (uint32_t u = 0; u < 8; ++u) {  // (words of a partition without listed keys hold anything)
+                    const uint32_t w = min(w0 + u * kBT, words - 1);
+                    v[u]             = __ldg(filters + it.fbase + w);
+                    on[u]            = __ldg(&I.listed[w >> (flog - 5)].nbk);
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 8; ++u)
+                    if (w0 + u * kBT < words) filter[w0 + u * kBT] = on[u] ? v[u] : 0u;
+            }
+            __syncthreads();
+        }
+        const uint32_t row = uint32_t(it.p - I.pay);
+        int32_t        nk[kEU];
+        uint32_t       x0    = threadIdx.x;
+        auto           fetch = [&]() {
+#pragma unroll
+            for (int u = 0; u < kEU; ++u) nk[u] = x0 + u * kBT < it.n ? __ldcs(it.k + x0 + u * kBT) : 0;
         };
-        acc.at(it.inst, out);
-        for (uint32_t x = threadIdx.x; x < it.n; x += kBT) {
-            const int32_t  k = __ldcs(it.k + x);
-            const uint64_t fp0 = fp_start(k, __ldcs(it.p + x));
-            int32_t        kept[kMaxRel - 2][kKeep], pay[kMaxRel - 2];  // pay: the combination's partners
-            uint32_t       cnt[kMaxRel - 2], at[kMaxRel - 2];
-            Walk           at_big[kMaxRel - 2];
-            uint64_t       fpl[kMaxRel - 1], slot;
-            int32_t        p;
-            Walk           f    = walk(0, k);
-            bool           some = f.next(p, slot);  // a key in F is in every table
-            if (!some) continue;
-            const Piece x1 = pieces[it.part_base + part_of(k, pb)];
-            if (!(x1.nbk & kDup)) {  // this partition has one partner per table
-                for (; some; some = f.next(p, slot)) {
-                    const uint32_t* w  = side + (uint64_t(x1.first) * 4 + slot) * stride;
-                    uint64_t        fp = fp_add(fp0, p);
-                    for (uint32_t j = 0; j < nt; ++j) fp = fp_add(fp, int32_t(w[j]));
-                    ++acc.rows;
-                    acc.sum += fp_final(fp);
-                }
-                continue;
+        fetch();
+        while (x0 - lane < it.n) {
+            int32_t        k[kEU];
+            const uint32_t at = x0;
+            uint32_t       on = 0;
+#pragma unroll
+            for (int u = 0; u < kEU; ++u) {
+                k[u]             = nk[u];
+                uint32_t       w;
+                const uint32_t m = filter_bits(k[u], flog, w);
+                const uint32_t f = filter[(part_of(k[u], pb) << (flog - 5)) + w];
+                on |= uint32_t(x0 + u * kBT < it.n && (f & m) == m) << u;
             }
-            for (uint32_t j = 0; j < nt; ++j) {
-                Walk           w = walk(j + 1, k);
-                uint32_t       c = 0;
-                int32_t        pj;
-                while (w.next(pj, slot)) {
-                    if (c < kKeep) kept[j][c] = pj;
-                    ++c;
-                }
-                cnt[j] = c;
-                at[j]  = 0;
-                pay[j] = kept[j][0];
-                if (c > kKeep) {
-                    at_big[j] = walk(j + 1, k);
-                    at_big[j].next(pj, slot);
-                }
+            x0 += kBT * kEU;
+            fetch();
+            if (!__any_sync(0xffffffffu, on != 0)) continue;
+#pragma unroll
+            for (int u = 0; u < kEU; ++u) {
+                const unsigned bal = __ballot_sync(0xffffffffu, (on >> u) & 1u);
+                if ((on >> u) & 1u) W.queue[qn + __popc(bal & lt)] = make_int2(k[u], int32_t(row + at + u * kBT));
+                qn += __popc(bal);
             }
-            // the next partner of table j; back at the first one, false
-            auto step = [&](uint32_t j) {
-                if (cnt[j] <= kKeep) {
-                    const bool more = ++at[j] < cnt[j];
-                    if (!more) at[j] = 0;
-                    pay[j] = kept[j][at[j]];
-                    return more;
-                }
-                uint64_t sl;
-                if (at_big[j].next(pay[j], sl)) return true;
-                at_big[j] = walk(j + 1, k);
-                at_big[j].next(pay[j], sl);
-                return false;
-            };
-            for (; some; some = f.next(p, slot)) {
-                fpl[0] = fp_add(fp0, p);
-                for (uint32_t z = 0;;) {
-                    for (; z < nt; ++z) fpl[z + 1] = fp_add(fpl[z], pay[z]);
-                    ++acc.rows;
-                    acc.sum += fp_final(fpl[nt]);
-                    int j = int(nt) - 1;
-                    while (j >= 0 && !step(uint32_t(j))) --j;
-                    if (j < 0) break;
-                    z = uint32_t(j);
-                }
+            while (qn >= 32) {
+                qn -= 32;
+                enum_rows(W, I, qn, 32, acc);
             }
         }
     }
+    if (qn) enum_rows(W, I, 0, qn, acc);
     acc.at(~0u, out);
 }
 
@@ -1065,7 +1351,7 @@ Geometry geometry(const BatchOptions& o) {
     if (tables > 200 * 1024) throw Error(HJ_ERR_INVALID, "batch: partition tables exceed shared memory");
     g.slot_q16 = batch_buckets_q16(o.load);
     g.fcap     = uint32_t(std::min<uint64_t>(batch_piece_buckets(g.cap, g.slot_q16), (220 * 1024 - tables) / 2));
-    g.build_smem = tables + size_t(g.fcap) * 2 + 4;
+    g.build_smem = tables + size_t(g.fcap) * 2 + 4 + (1u << kFilterPart) / 8;
     return g;
 }
 
@@ -1095,7 +1381,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     const size_t   build_smem = G.build_smem;
     std::vector<RelInst>  hr;
     std::vector<InstInfo> hi(n);
-    uint64_t pbase = 0, ipbase = 0, items = 0, build_rows = 0;
+    uint64_t pbase = 0, ipbase = 0, items = 0, build_rows = 0, fwords = 0;
     uint32_t pmax = 0, stride = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const uint32_t nrel = uint32_t(all[i0 + i].rels.size());
@@ -1108,10 +1394,12 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
         s.ip_base        = ipbase;
         s.nrel           = nrel;
         s.pbits          = p;
+        s.fbase          = uint32_t(fwords);
+        fwords += 1ull << (p + filter_log(p) - 5);
         stride           = std::max(stride, s.nrel - 2);
         for (uint32_t j = 1; j < s.nrel; ++j) {
             const BatchRelation br = rel_of(i, j);
-            hr.push_back({br.keys, br.payload, br.rows, items, pbase + (uint64_t(j - 1) << p), p, i, 0, 0});
+            hr.push_back({br.keys, br.payload, br.rows, items, pbase + (uint64_t(j - 1) << p), p, i, 0, 0, 0});
             items += (br.rows + kPartItem - 1) / kPartItem;
         }
         build_rows += nb;
@@ -1126,7 +1414,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     const int    g_scat    = resident_grid(k_bpart_scatter, kPT, scat_smem);
     const int    g_bld     = resident_grid(k_bt_build, kBuildT, build_smem);
     const int    g_prb     = resident_grid(k_bt_probe, kBT, prb_smem);
-    const int    g_enm     = resident_grid(k_bt_enum, kBT, 0);
+    const int    g_enm     = resident_grid(k_bt_enum, kBT, kEnumSmem);
     auto grid_for = [](int g, uint64_t work) { return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, work))); };
 
     // R0s: an item is what one block has of its instance's rows when the grid
@@ -1138,11 +1426,12 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
         const BatchRelation  br    = rel_of(i, 0);
         const uint64_t       steps = br.rows / (2 * uint64_t(g_prb) * kStepRows);
         const uint64_t       irows = std::min<uint64_t>(std::max<uint64_t>(steps, 16), 64) * kStepRows;
-        hr.push_back({br.keys, br.payload, br.rows, items, hi[i].part_base, hi[i].pbits, i, uint32_t(irows), hi[i].nrel});
+        hr.push_back({br.keys, br.payload, br.rows, items, hi[i].part_base, hi[i].pbits, i, uint32_t(irows), hi[i].nrel,
+                      hi[i].fbase});
         items += (br.rows + irows - 1) / irows;
     }
     const uint32_t nr   = uint32_t(hr.size());
-    const uint64_t nbkt = batch_table_buckets(build_rows, pbase, G.slot_q16);
+    const uint64_t nbkt = batch_table_buckets(build_rows, pbase + ipbase, G.slot_q16);
 
     std::vector<InstOut> ho(n);
     std::vector<void*>   owned;
@@ -1174,6 +1463,8 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     auto* d_I    = reinterpret_cast<InstInfo*>(d_R + nr);
     auto* off    = static_cast<uint64_t*>(take((pbase + 2) * 8));
     auto* pieces = static_cast<Piece*>(take((pbase + 1) * sizeof(Piece)));
+    auto* listed = static_cast<Piece*>(take((pbase + 1) * sizeof(Piece)));
+    auto* filters = static_cast<uint32_t*>(take(fwords * 4));
     auto* tmp    = static_cast<uint64_t*>(take((scan_tmp_words(pbase) + 1) * 8));
     auto* pkp    = static_cast<int2*>(take(build_rows * 8));  // (key, payload) in partition order
     auto* rmap   = static_cast<uint32_t*>(take(bitems * 4));
@@ -1183,7 +1474,8 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
     auto* side   = static_cast<uint32_t*>(take(nbkt * 4 * stride * 4));
     HJ_CUDA(cudaMemcpyAsync(d_R, hd.data(), hd.size(), cudaMemcpyHostToDevice, st));
 
-    Tables tb{tabs, side, reinterpret_cast<uint32_t*>(d_q + 2), stride, G.slot_q16};
+    Tables tb{tabs, side, reinterpret_cast<uint32_t*>(d_q + 2), reinterpret_cast<uint32_t*>(d_q + 3),
+              uint32_t(nbkt), stride, G.slot_q16};
 
     auto enqueue = [&]() {
         HJ_CUDA(cudaMemsetAsync(d_out, 0, zero_bytes, st));
@@ -1198,16 +1490,14 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
                                                                           pkp);
         HJ_LAUNCH_CHECK();
         k_bt_build<<<grid_for(g_bld, ipbase), kBuildT, build_smem, st>>>(d_I, pmap, ipbase, off, pkp, cap, scap, fcap,
-                                                                         max_bits, load_q8, tb, pieces, d_out);
+                                                                         max_bits, load_q8, tb, pieces, listed, filters, d_out);
         HJ_LAUNCH_CHECK();
         k_bt_probe<<<grid_for(g_prb, items - bitems), kBT, prb_smem, st>>>(imap, items - bitems, tabs, side, stride,
                                                                            pieces, d_out);
         HJ_LAUNCH_CHECK();
-        if (stride) {
-            k_bt_enum<<<grid_for(g_enm, items - bitems), kBT, 0, st>>>(imap, items - bitems, tabs, side, stride,
-                                                                       pieces, d_out);
-            HJ_LAUNCH_CHECK();
-        }
+        k_bt_enum<<<grid_for(g_enm, items - bitems), kBT, kEnumSmem, st>>>(imap, items - bitems, tabs, pkp, listed, filters,
+                                                                           tb.lists, d_out);
+        HJ_LAUNCH_CHECK();
     };
     if (o.graph) {
         cudaGraph_t g = nullptr;

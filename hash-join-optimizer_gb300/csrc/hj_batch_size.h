@@ -21,6 +21,9 @@ inline uint32_t batch_buckets_q16(double load) {
 // Buckets of a piece of n rows: a fifth of its slots or more stays free.
 HJ_BATCH_HD uint32_t batch_piece_buckets(uint32_t n, uint32_t q16) { return uint32_t((uint64_t(n) * q16) >> 16) + 1; }
 
+// Buckets for two pieces of n rows in all, however the rows divide between them.
+HJ_BATCH_HD uint32_t batch_pair_buckets(uint32_t n, uint32_t q16) { return batch_piece_buckets(n, q16) + 1; }
+
 // Buckets for `pieces` pieces of `rows` rows in all, and the free bucket 0: no
 // fewer than the pieces take however the rows divide among them.  In the
 // pieces' own fixed point: with the exact quotient, pieces whose size it
