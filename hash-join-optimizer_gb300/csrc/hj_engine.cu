@@ -967,7 +967,7 @@ struct Exec {
         try {
             // streams for one match a probe row and some slack for keys with
             // several, which the count pass fills as far as matches are single;
-            // a result beyond them gets larger ones (its direct rows copied)
+            // a result that does not fit gets others (its direct rows copied)
             const uint64_t      cap = pkc.n + std::min<uint64_t>(3 * pkc.n, 16u << 20);
             std::vector<RidOut> ro;
             std::vector<Buf>    dst;
@@ -981,13 +981,17 @@ struct Exec {
             phase("probe_write");
             if (total > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
             out.rows = total;
+            // the streams stay until the plan has read them: large ones that a
+            // selective join has left mostly empty are exchanged for such of its
+            // size too (below an eighth, the copy is little beside the probe)
+            const bool fits = total <= cap && (cap * 4 < kBig || total >= cap / 8);
             for (size_t i = 0; i < ro.size(); ++i) {
-                if (total > cap) {
-                    Buf            more = make_buf(total * 4, c->st);
-                    const uint64_t d    = probe_direct(pp);
-                    if (d) HJ_CUDA(cudaMemcpyAsync(more->p, dst[i]->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
-                    dst[i]    = more;
-                    ro[i].dst = more->as<uint32_t>();
+                if (!fits) {
+                    Buf            sized = make_buf(std::max<uint64_t>(total, 1) * 4, c->st);
+                    const uint64_t d     = probe_direct(pp);
+                    if (d) HJ_CUDA(cudaMemcpyAsync(sized->p, dst[i]->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
+                    dst[i]    = sized;
+                    ro[i].dst = sized->as<uint32_t>();
                 }
                 const auto [side, s] = need[i];
                 out.srcs.push_back(Source{(side == 1 ? B : P).srcs[s].table, dst[i]});

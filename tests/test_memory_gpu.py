@@ -42,3 +42,28 @@ rows, sums, redo = E.batch_execute(inst)
 assert list(rows) == [100 * 100, 0, 0, 0] and sums[1] == sums[2] == sums[3] == 0 and redo == 0
 assert before - free() < 4 * n, before - free()
 """)
+
+
+def test_selective_join_keeps_streams_of_its_result():
+    """Two joins over 40M probe rows, few of which match: the row ids of the first take
+    no more than its result while the second runs, so both together take a probe's lists
+    and output streams once."""
+    run("""
+n = 40_000_000
+a = np.zeros(n, np.int32); a[:1000] = np.arange(1, 1001)
+few = np.arange(1, 1001, dtype=np.int32)
+p = hj.Plan()
+for cols, rows in (([few], 1000), ([a, a], n)):
+    p.new_input(E.upload(hj.Table(rows, [hj.Column.int32(c) for c in cols])))
+I = hj.INT32
+def join():  # (few x big): big's two columns and few's
+    s, b = p.new_scan_node(0, [(0, I)]), p.new_scan_node(1, [(0, I), (1, I)])
+    return p.new_join_node(True, s, b, 0, 0, [(1, I), (2, I), (0, I)])
+p.root = p.new_join_node(True, join(), join(), 0, 0, [(0, I), (3, I)])
+first = free()
+r = E.execute_raw(p)
+assert E.stats(r)[2] == 3000
+# a probe's lists are 36 bytes a row, its streams here 2 x 4 bytes for n + 2^24 rows; the decoded
+# columns are read in place
+assert first - free() < 36 * n + 8 * (n + (1 << 24)) + (300 << 20), first - free()
+""")
