@@ -1626,21 +1626,30 @@ void plain_instance(const BatchInstance& b, const ProbeParams& prm, int dir_bits
                     dir_cap_bits);
         ProbePlan* pp    = nullptr;
         uint64_t   total = 0;
-        uint32_t * pr = nullptr, *bw = nullptr;
+        RidOut     ro[2] = {{0, nullptr, nullptr}, {1, nullptr, nullptr}};
         try {
-            pr = static_cast<uint32_t*>(take(np * 4));  // one match a row, or more: below
-            bw = static_cast<uint32_t*>(take(np * 4));
-            RidOut ro[2] = {{0, nullptr, pr}, {1, nullptr, bw}};
-            total        = probe_count(t, pk, prm, ro, 2, &pp, st);
-            if (total > np) {
+            // streams for one match a row, made before the count; others for more,
+            // and where there is no room for them
+            auto count = [&](bool ahead) {
+                for (RidOut& o : ro) o.dst = ahead ? static_cast<uint32_t*>(take(np * 4)) : nullptr;
+                total = probe_count(t, pk, prm, ro, ahead ? 2 : 0, &pp, st);
+                if (ahead && total <= np) return;
                 for (RidOut& o : ro) {
-                    uint32_t* more = static_cast<uint32_t*>(take(total * 4));
+                    uint32_t* sized = static_cast<uint32_t*>(take(total * 4));
                     if (const uint64_t d = probe_direct(pp))
-                        HJ_CUDA(cudaMemcpyAsync(more, o.dst, d * 4, cudaMemcpyDeviceToDevice, st));
-                    o.dst = more;
+                        HJ_CUDA(cudaMemcpyAsync(sized, o.dst, d * 4, cudaMemcpyDeviceToDevice, st));
+                    o.dst = sized;
                 }
-                pr = ro[0].dst;
-                bw = ro[1].dst;
+            };
+            const size_t before = owned.size();
+            try {
+                count(true);
+            } catch (const Error& e) {
+                if (e.status != HJ_ERR_NOMEM) throw;
+                probe_free(pp, st);
+                pp = nullptr;
+                for (; owned.size() > before; owned.pop_back()) dfree(owned.back(), st);
+                count(false);
             }
             if (total) probe_write(t, pk, pp, ro, 2, st);
         } catch (...) {
@@ -1654,7 +1663,7 @@ void plain_instance(const BatchInstance& b, const ProbeParams& prm, int dir_bits
         uint64_t* nf = last ? nullptr : static_cast<uint64_t*>(take(total * 8));
         if (total) {
             k_pairs_next<<<unsigned(std::min<uint64_t>(div_up(total, 256), uint64_t(num_sms()) * 8)), 256, 0, st>>>(
-                pr, bw, total, pkeys, pfp, ppay, br.payload, nk, nf, d_sum);
+                ro[0].dst, ro[1].dst, total, pkeys, pfp, ppay, br.payload, nk, nf, d_sum);
             HJ_LAUNCH_CHECK();
         }
         pkeys = nk;

@@ -910,15 +910,18 @@ struct Exec {
             pkc.n > 0 && pkc.n <= kReduceKeys && pkc.n <= bkc.n / 16) {
             std::vector<RidOut> ro;
             std::vector<Buf>    dst;
-            for (int s : ss) {
-                dst.push_back(make_buf(bkc.n * 4, c->st));
-                ro.push_back(RidOut{1, B.srcs[s].rid ? B.srcs[s].rid->as<uint32_t>() : nullptr,
-                                    dst.back()->as<uint32_t>()});
+            try {
+                for (int s : ss) {
+                    dst.push_back(make_buf(bkc.n * 4, c->st));
+                    ro.push_back(RidOut{1, B.srcs[s].rid ? B.srcs[s].rid->as<uint32_t>() : nullptr,
+                                        dst.back()->as<uint32_t>()});
+                }
+            } catch (const Error& e) {
+                if (e.status != HJ_ERR_NOMEM) throw;
+                dst.clear();  // no room for the cut
             }
-            ProbeParams rp;
-            rp.pinned        = c->pinned;
-            rp.counters      = c->counters;
-            const uint64_t m = reduce_build(bkc, pkc, rp, ro.data(), int(ro.size()), c->st);
+            const uint64_t m = dst.empty() ? bkc.n : reduce_build(bkc, pkc, context_probe_params(c), ro.data(),
+                                                                  int(ro.size()), c->st);
             // not worth it when most rows stay: the streams are dropped
             if (m <= bkc.n / 2) {
                 for (size_t i = 0; i < ss.size(); ++i) B.srcs[ss[i]].rid = dst[i];
@@ -962,40 +965,55 @@ struct Exec {
         phase("probe");
         ProbeParams prm = context_probe_params(c);
         prm.after_count = [this] { phase("probe_sync"); };
-        ProbePlan* pp = nullptr;
-        uint64_t total = 0;
-        try {
-            // streams for one match a probe row and some slack for keys with
-            // several, which the count pass fills as far as matches are single;
-            // a result that does not fit gets others (its direct rows copied)
-            const uint64_t      cap = pkc.n + std::min<uint64_t>(3 * pkc.n, 16u << 20);
-            std::vector<RidOut> ro;
-            std::vector<Buf>    dst;
+        ProbePlan*          pp    = nullptr;
+        uint64_t            total = 0;
+        std::vector<RidOut> ro;
+        std::vector<Buf>    dst;
+        // Counts the matches and makes the output streams.  `ahead`: streams for one
+        // match a probe row and some slack for keys with several, made before, which
+        // the count pass fills as far as matches are single; a result that does
+        // not fit gets others (its direct rows copied).
+        const uint64_t cap   = pkc.n + std::min<uint64_t>(3 * pkc.n, 16u << 20);
+        auto           count = [&](bool ahead) {
+            auto slots = [&](size_t i, uint64_t rows) {
+                dst[i]    = make_buf(std::max<uint64_t>(rows, 1) * 4, c->st);
+                ro[i].dst = dst[i]->as<uint32_t>();
+            };
+            dst.assign(need.size(), nullptr);
+            ro.clear();
             for (auto [side, s] : need) {
-                Inter& side_in = side == 1 ? B : P;
-                dst.push_back(make_buf(std::max<uint64_t>(cap, 1) * 4, c->st));
-                ro.push_back(RidOut{side, side_in.srcs[s].rid ? side_in.srcs[s].rid->as<uint32_t>() : nullptr,
-                                    dst.back()->as<uint32_t>()});
+                const Buf& rid = (side == 1 ? B : P).srcs[s].rid;
+                ro.push_back(RidOut{side, rid ? rid->as<uint32_t>() : nullptr, nullptr});
             }
-            total = probe_count(t, pkc, prm, ro.data(), int(ro.size()), &pp, c->st);
-            phase("probe_write");
+            for (size_t i = 0; i < ro.size() && ahead; ++i) slots(i, cap);
+            total = probe_count(t, pkc, prm, ro.data(), ahead ? int(ro.size()) : 0, &pp, c->st);
             if (total > 0xffffffffull) throw Error(HJ_ERR_INVALID, "join result exceeds 2^32 rows");
-            out.rows = total;
             // the streams stay until the plan has read them: large ones that a
             // selective join has left mostly empty are exchanged for such of its
             // size too (below an eighth, the copy is little beside the probe)
-            const bool fits = total <= cap && (cap * 4 < kBig || total >= cap / 8);
+            if (ahead && total <= cap && (cap * 4 < kBig || total >= cap / 8)) return;
             for (size_t i = 0; i < ro.size(); ++i) {
-                if (!fits) {
-                    Buf            sized = make_buf(std::max<uint64_t>(total, 1) * 4, c->st);
-                    const uint64_t d     = probe_direct(pp);
-                    if (d) HJ_CUDA(cudaMemcpyAsync(sized->p, dst[i]->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
-                    dst[i]    = sized;
-                    ro[i].dst = sized->as<uint32_t>();
-                }
-                const auto [side, s] = need[i];
-                out.srcs.push_back(Source{(side == 1 ? B : P).srcs[s].table, dst[i]});
+                const Buf      full = dst[i];
+                const uint64_t d    = probe_direct(pp);
+                slots(i, total);
+                if (d) HJ_CUDA(cudaMemcpyAsync(dst[i]->p, full->p, d * 4, cudaMemcpyDeviceToDevice, c->st));
             }
+        };
+        try {
+            try {
+                count(true);
+            } catch (const Error& e) {
+                if (e.status != HJ_ERR_NOMEM) throw;
+                // no room for that: every match listed, and streams for them alone
+                probe_free(pp, c->st);
+                pp = nullptr;
+                dst.clear();
+                count(false);
+            }
+            phase("probe_write");
+            out.rows = total;
+            for (size_t i = 0; i < ro.size(); ++i)
+                out.srcs.push_back(Source{(need[i].first == 1 ? B : P).srcs[need[i].second].table, dst[i]});
             if (total > 0) probe_write(t, pkc, pp, ro.data(), int(ro.size()), c->st);
         } catch (...) {
             probe_free(pp, c->st);
@@ -1658,19 +1676,30 @@ int hj_table_probe(hj_context* c, const hj_hash_table* t, const int32_t* keys, c
         const hj::ProbeParams prm = hj::context_probe_params(c);
         hj::ProbePlan*        pp  = nullptr;
         // nothing may be written before the matches are known to fit, so the
-        // directly written pairs go to buffers of the call's own
-        hj::Buf dp, db;
-        int     nout = 0;
-        if (out_probe && out_build && capacity && n) {
-            dp   = hj::make_buf(n * 4, c->st);
-            db   = hj::make_buf(n * 4, c->st);
-            nout = 2;
-        }
-        const hj::RidOut tmp[2] = {{0, nullptr, dp ? dp->as<uint32_t>() : nullptr},
-                                   {1, nullptr, db ? db->as<uint32_t>() : nullptr}};
+        // directly written pairs go to buffers of the call's own; without room for
+        // them every match is listed
+        hj::Buf  dp, db;
+        uint64_t total = 0;
+        auto     count = [&](bool ahead) {
+            if (ahead) {
+                dp = hj::make_buf(n * 4, c->st);
+                db = hj::make_buf(n * 4, c->st);
+            }
+            const hj::RidOut tmp[2] = {{0, nullptr, ahead ? dp->as<uint32_t>() : nullptr},
+                                       {1, nullptr, ahead ? db->as<uint32_t>() : nullptr}};
+            total = hj::probe_count(t->t, pk, prm, tmp, ahead ? 2 : 0, &pp, c->st);
+        };
         try {
-            const uint64_t total = hj::probe_count(t->t, pk, prm, tmp, nout, &pp, c->st);
-            *num_matches         = total;
+            try {
+                count(out_probe && out_build && capacity && n);
+            } catch (const hj::Error& e) {
+                if (e.status != HJ_ERR_NOMEM) throw;
+                hj::probe_free(pp, c->st);
+                pp = nullptr;
+                dp = db = nullptr;
+                count(false);
+            }
+            *num_matches = total;
             if (total > capacity) {
                 status = HJ_ERR_CAPACITY;
             } else if (total > 0) {

@@ -67,3 +67,43 @@ assert E.stats(r)[2] == 3000
 # columns are read in place
 assert first - free() < 36 * n + 8 * (n + (1 << 24)) + (300 << 20), first - free()
 """)
+
+
+@pytest.mark.parametrize("call", ["table_probe", "execute", "plain"])
+def test_probe_without_room_for_streams_ahead(call):
+    """With device memory for a probe's lists and its result, but not for output streams of
+    the probe side's length beside them, the result is the same."""
+    run("call = " + repr(call) + """
+n, nb = 1 << 25, 1000
+build, probe = ints(nb, 0), ints(n, -5)
+build.copy_(torch.arange(nb)); probe[:300] = torch.arange(300, dtype=torch.int32)
+torch.cuda.synchronize()
+lists = 9 * 4 * n
+def fill(room):
+    global hold
+    torch.cuda.synchronize()
+    hold = torch.empty(free() - room, dtype=torch.uint8, device="cuda")
+if call == "table_probe":
+    t, nm = C.c_void_p(), C.c_uint64()
+    assert L.hj_table_build(E.handle, build.data_ptr(), None, nb, -1, C.byref(t)) == 0
+    op, ob = ints(1000, -1), ints(1000, -1)
+    fill(lists + (230 << 20))  # (an array takes up to 16 MB more than its size; streams would take 256 MB)
+    assert L.hj_table_probe(E.handle, t, probe.data_ptr(), None, n, op.data_ptr(), ob.data_ptr(), 1000, C.byref(nm)) == 0
+    torch.cuda.synchronize()
+    assert nm.value == 300 and bool((op[:300] == ob[:300]).all()) and int(op[:300].sum()) == 300 * 299 // 2
+elif call == "execute":
+    p, I = hj.Plan(), hj.INT32
+    for t in (build, probe):
+        p.new_input(E.upload(hj.Table(t.numel(), [hj.Column.int32(t.cpu().numpy())])))
+    p.root = p.new_join_node(True, p.new_scan_node(0, [(0, I)]), p.new_scan_node(1, [(0, I)]), 0, 0, [(0, I), (1, I)])
+    fill(lists + (360 << 20))  # (streams would take 400 MB)
+    r = E.execute(p)
+    v, ok = hj.decode_int32(r.columns[0])
+    assert r.num_rows == 300 and sorted(v.tolist()) == list(range(300))
+else:
+    inst = [[(probe.data_ptr(), probe.data_ptr(), n), (build.data_ptr(), build.data_ptr(), nb)]]
+    want, sums, _ = E.batch_execute(inst)  # (persistent: takes little)
+    fill(lists + (230 << 20))
+    rows, s2, _ = E.batch_execute(inst, hj.BATCH_PLAIN)
+    assert rows[0] == want[0] == 300 and sums[0] == s2[0]
+""")
