@@ -900,14 +900,12 @@ struct Exec {
         // 1,984 325 / 106, 10M x 8,192 338 / 267; Zipf probe keys 1M x 1,984 117 /
         // 68; one key's 20M pairs 1M x 1,984 339 / 282.  It loses where one key
         // takes a quarter of the build rows, which then stay: 300,000 x 30 154 /
-        // 168, 1M x 400 338 / 368.  At 2^16 rows and less a build is one launch.  The
-        // table over the probe side instead was as fast for distinct keys, but a
+        // 168, 1M x 400 338 / 368.  The table over the probe side instead was as fast for distinct keys, but a
         // repeated one made its buckets heavy (Zipf, 1M x 31,250: 122 / 149).
         std::vector<int> ss{bk.src};  // the build side's sources that are read
         for (auto [side, s] : need)
             if (side == 1 && s != bk.src) ss.push_back(s);
-        if (!cacheable && ss.size() <= size_t(kMaxRidOut) && bkc.n > (1u << 16) && bkc.n <= 0xffffffffull &&
-            pkc.n > 0 && pkc.n <= kReduceKeys && pkc.n <= bkc.n / 16) {
+        if (!cacheable && ss.size() <= size_t(kMaxRidOut) && build_is_cut(bkc.n, pkc.n)) {
             std::vector<RidOut> ro;
             std::vector<Buf>    dst;
             try {
@@ -973,7 +971,7 @@ struct Exec {
         // match a probe row and some slack for keys with several, made before, which
         // the count pass fills as far as matches are single; a result that does
         // not fit gets others (its direct rows copied).
-        const uint64_t cap   = pkc.n + std::min<uint64_t>(3 * pkc.n, 16u << 20);
+        const uint64_t cap   = stream_slots(pkc.n);
         auto           count = [&](bool ahead) {
             auto slots = [&](size_t i, uint64_t rows) {
                 dst[i]    = make_buf(std::max<uint64_t>(rows, 1) * 4, c->st);

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <functional>
 #include <vector>
@@ -144,6 +145,15 @@ struct ProbeParams {
 // stream o.dst[k] = o.src ? o.src[row] : row (b.n slots each).  One host
 // synchronisation.  p.n <= kReduceKeys, b.n < 2^32.
 constexpr uint64_t kReduceKeys = 8192;
+// Is a build side of b rows cut down to what p probe rows can meet?  At 2^16 rows
+// and less a build is one launch; the figures stand at the join.
+inline bool build_is_cut(uint64_t b, uint64_t p) {
+    return b > kDirectKeys && b <= 0xffffffffull && p > 0 && p <= kReduceKeys && p <= b / 16;
+}
+// Slots of a join's output streams made before its p probe rows are counted: one
+// match a row, and some for keys with several.
+inline uint64_t stream_slots(uint64_t p) { return p + std::min<uint64_t>(3 * p, 16u << 20); }
+constexpr uint64_t kListBytes = 36;  // of the probe's lists, per probe row
 uint64_t reduce_build(const KeyCol& b, const KeyCol& p, const ProbeParams& prm, const RidOut* outs, int nout,
                       cudaStream_t st);
 

@@ -78,8 +78,9 @@ uint64_t next_pow2(uint64_t x) {
 
 // Working memory of a plan in HBM, from the row counts of its inputs: per
 // join its table (adjacency array, directory, partition temporaries), its
-// probe lists and the row ids of its result (estimated as the larger input),
-// plus the result pages.
+// probe lists, the row ids of its result (estimated as the larger input, or the
+// streams made before it is counted) and of a build side that is cut down, plus
+// the result pages.
 uint64_t estimate_bytes(const hj_context* c, const hj_plan_desc& p) {
     std::vector<uint64_t> rows(p.num_nodes, 0);
     std::vector<int>      state(p.num_nodes, 0);
@@ -100,8 +101,10 @@ uint64_t estimate_bytes(const hj_context* c, const hj_plan_desc& p) {
             const uint64_t b = n.build_left ? l : rr, q = n.build_left ? rr : l;
             r                = std::max(b, q);
             bytes += 8 * b + 8 * std::min<uint64_t>(next_pow2(b), 1ull << 22) + 24 * b;  // table + build temporaries
-            bytes += 32 * q;                                                           // probe lists, counts
-            bytes += 4 * r * std::max<uint32_t>(2, n.num_attrs);                       // result row ids
+            bytes += kListBytes * q;                                                   // probe lists, counts
+            const uint64_t streams = std::max<uint32_t>(2, n.num_attrs);               // of row ids, at most
+            bytes += 4 * std::max(r, stream_slots(q)) * streams;                       // the result's
+            if (build_is_cut(b, q)) bytes += 4 * b * std::min<uint64_t>(streams + 1, kMaxRidOut);  // and the cut's
         }
         rows[i]  = r;
         state[i] = 2;
