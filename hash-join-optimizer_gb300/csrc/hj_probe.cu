@@ -555,11 +555,12 @@ __device__ __forceinline__ uint64_t hit_of(const uint32_t* __restrict__ off, uin
     return lo;
 }
 
-// chunk_first[c] = the uniform hit holding output position c * chunk.
+// chunk_first[c] = the uniform hit holding the first output position of chunk c.
+// Chunk c is the positions from c * chunk - lead on, those below 0 absent.
 __global__ void k_chunk_first(const uint32_t* __restrict__ off, uint64_t n_u, uint64_t nchunks, uint32_t chunk,
-                              uint32_t* __restrict__ chunk_first) {
+                              uint32_t lead, uint32_t* __restrict__ chunk_first) {
     const uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (c < nchunks) chunk_first[c] = uint32_t(hit_of(off, n_u, c * chunk));
+    if (c < nchunks) chunk_first[c] = uint32_t(hit_of(off, n_u, c ? c * chunk - lead : 0));
 }
 
 // Outputs of one warp's chunk in k_write_uniform<G>, and the per-warp
@@ -594,7 +595,7 @@ __device__ __forceinline__ void store_run(uint32_t* dst, const uint32_t (&v)[G],
 template <int G>
 __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
     k_write_uniform(ProbeTab T, Lists Ls, uint64_t n_u, const uint32_t* __restrict__ chunk_first, uint64_t total,
-                    Outs outs) {
+                    uint32_t lead, Outs outs) {
     const uint32_t* __restrict__ off = Ls.u_off;
     constexpr uint32_t CH = warp_chunk(G);
     constexpr uint32_t NW = CH + 2;
@@ -605,16 +606,21 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
     uint32_t*      s_s    = s_pr + NW;                          // first tuple of each hit's bucket
     uint32_t*      s_orel = s_s + NW;                           // hit start - chunk start, mod 2^32
     uint32_t*      s_msk  = s_orel + NW;                        // match mask (0: every tuple)
-    // vector stores need every stream 16-byte aligned (engine buffers are)
+    // vector stores need every stream 16-byte aligned at a chunk's start: `lead` words
+    // before the first one's (the engine's streams start at the same word, behind
+    // the rows that the count pass wrote).  6M rows behind one of them: 75 us with
+    // single stores, 71 with vectors, and 72 behind none.
     bool vec = true;
-    for (int oi = 0; oi < outs.n; ++oi) vec &= (reinterpret_cast<uintptr_t>(outs.o[oi].dst) & 15) == 0;
-    const uint64_t nchunks = (total + CH - 1) / CH;
+    for (int oi = 0; oi < outs.n; ++oi)
+        vec &= ((reinterpret_cast<uintptr_t>(outs.o[oi].dst) - 4 * lead) & 15) == 0;
+    const uint64_t nchunks = (total + lead + CH - 1) / CH;
     const uint64_t nw      = (uint64_t(gridDim.x) * blockDim.x) >> 5;
     const uint64_t stream  = l2_evict_first();  // row ids are written once, read later in order
     for (uint64_t c = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += nw) {
-        const uint64_t o0  = c * CH;
-        const uint32_t len = uint32_t(umin64(CH, total - o0));
-        const uint64_t h0  = chunk_first ? __ldg(chunk_first + c) : hit_of(off, n_u, o0);
+        const int64_t  o0  = int64_t(c * CH) - lead;
+        const uint32_t len = uint32_t(umin64(CH, uint64_t(int64_t(total) - o0)));
+        const uint32_t q_lo = c ? 0 : lead;  // the chunk's outputs are [q_lo, len)
+        const uint64_t h0  = chunk_first ? __ldg(chunk_first + c) : hit_of(off, n_u, c ? o0 : 0);
         const uint64_t h1  = c + 1 < nchunks ? (chunk_first ? __ldg(chunk_first + c + 1) : hit_of(off, n_u, o0 + CH))
                                              : n_u - 1;
         const uint32_t nh  = uint32_t(h1 - h0) + 1;  // hits h0 .. h0 + nh - 1 cover the chunk
@@ -623,7 +629,7 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
             // key): lane 0 reads the hit, every lane takes consecutive matches
             uint32_t orel = 0, m = 0, t0 = 0, prow = 0;
             if (lane == 0) {
-                orel           = uint32_t(uint64_t(__ldg(off + h0)) - o0);  // mod 2^32: the hit may start earlier
+                orel           = uint32_t(int64_t(__ldg(off + h0)) - o0);  // mod 2^32: the hit may start earlier
                 m              = __ldg(Ls.u_mask + h0);
                 const uint32_t sp = __ldg(Ls.u_sp + h0);
                 prow           = __ldg(Ls.u_row + h0);
@@ -639,10 +645,10 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
 #pragma unroll
                 for (int i = 0; i < G; ++i) {
                     const uint32_t idx = q0 + i - orel;  // match number within the hit
-                    brow[i]            = q0 + i >= len ? 0u
+                    brow[i]            = q0 + i >= len || q0 + i < q_lo ? 0u
                                        : m == kRowHit ? t0 : __ldg(T.rows + t0 + (m ? nth_bit(m, idx) : idx));
                 }
-                const bool full = q0 + G <= len;
+                const bool full = q0 >= q_lo && q0 + G <= len;
                 for (int oi = 0; oi < outs.n; ++oi) {
                     const RidOut o = outs.o[oi];
                     uint32_t     v[G];
@@ -650,13 +656,13 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
 #pragma unroll
                     for (int i = 0; i < G; ++i)
                         v[i] = o.side == 0 ? pv : ((o.src && q0 + i < len) ? __ldg(o.src + brow[i]) : brow[i]);
-                    uint32_t* dst = o.dst + o0 + q0;
+                    uint32_t* dst = o.dst + (o0 + int64_t(q0));
                     if (full) {
                         store_run<G>(dst, v, vec, stream);
                     } else {
 #pragma unroll
                         for (int i = 0; i < G; ++i)
-                            if (q0 + i < len) dst[i] = v[i];
+                            if (q0 + i >= q_lo && q0 + i < len) dst[i] = v[i];
                     }
                 }
             }
@@ -664,8 +670,8 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
         }
         for (uint32_t q = lane; q <= nh; q += 32) {
             const uint64_t hq  = h0 + q;
-            const uint64_t o   = hq < n_u ? uint64_t(__ldg(off + hq)) : total;
-            const uint64_t rel = o > o0 ? o - o0 : 0;
+            const int64_t  o   = hq < n_u ? int64_t(__ldg(off + hq)) : int64_t(total);
+            const uint64_t rel = o > o0 ? uint64_t(o - o0) : 0;
             s_rel[q]           = uint32_t(umin64(rel, len));
             if (q < nh) {
                 const uint32_t m  = __ldg(Ls.u_mask + hq);
@@ -692,7 +698,7 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
             for (int i = 0; i < G; ++i) {
                 const uint32_t q = q0 + i;
                 prow[i] = brow[i] = 0;
-                if (q < len) {
+                if (q >= q_lo && q < len) {
                     while (s_rel[k + 1] <= q) ++k;
                     const uint32_t idx = q - s_orel[k];  // match number within the hit
                     const uint32_t m   = s_msk[k];
@@ -700,7 +706,7 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
                     brow[i]            = m == kRowHit ? s_s[k] : __ldg(T.rows + s_s[k] + (m ? nth_bit(m, idx) : idx));
                 }
             }
-            const bool full = q0 + G <= len;
+            const bool full = q0 >= q_lo && q0 + G <= len;
             for (int oi = 0; oi < outs.n; ++oi) {
                 const RidOut o = outs.o[oi];
                 uint32_t     v[G];
@@ -709,13 +715,13 @@ __global__ void __launch_bounds__(256, G <= 4 ? 6 : (G <= 8 ? 4 : 2))
                     const uint32_t x = o.side == 0 ? prow[i] : brow[i];
                     v[i]             = (o.src && q0 + i < len) ? __ldg(o.src + x) : x;
                 }
-                uint32_t* dst = o.dst + o0 + q0;
+                uint32_t* dst = o.dst + (o0 + int64_t(q0));
                 if (full) {
                     store_run<G>(dst, v, vec, stream);
                 } else {
 #pragma unroll
                     for (int i = 0; i < G; ++i)
-                        if (q0 + i < len) dst[i] = v[i];
+                        if (q0 + i >= q_lo && q0 + i < len) dst[i] = v[i];
                 }
             }
         }
@@ -943,6 +949,9 @@ __global__ void __launch_bounds__(kRT, 2)
     ctr[6]      = 0;
 }
 
+// Words between the 16-byte boundary before the first stream's start and that start.
+uint32_t stream_lead(const Outs& outs) { return uint32_t(reinterpret_cast<uintptr_t>(outs.o[0].dst) >> 2) & 3; }
+
 template <int G>
 void launch_uniform_g(const ProbeTab& T, const Lists& L, uint64_t n_u, const uint32_t* chunk_first, uint64_t total,
                       const Outs& outs, cudaStream_t st) {
@@ -956,9 +965,10 @@ void launch_uniform_g(const ProbeTab& T, const Lists& L, uint64_t n_u, const uin
         resident.store(n);
     });
     const int per_sm = resident.load();
-    const uint64_t nchunks = (total + warp_chunk(G) - 1) / warp_chunk(G);
+    const uint32_t lead    = stream_lead(outs);
+    const uint64_t nchunks = (total + lead + warp_chunk(G) - 1) / warp_chunk(G);
     const uint64_t grid    = std::max<uint64_t>(1, std::min<uint64_t>((nchunks + 7) / 8, uint64_t(num_sms()) * std::max(1, per_sm)));
-    k_write_uniform<G><<<unsigned(grid), 256, smem, st>>>(T, L, n_u, chunk_first, total, outs);
+    k_write_uniform<G><<<unsigned(grid), 256, smem, st>>>(T, L, n_u, chunk_first, total, lead, outs);
     HJ_LAUNCH_CHECK();
 }
 
@@ -1104,9 +1114,10 @@ void probe_write(const Table& t, const KeyCol& pk, ProbePlan* pp, const RidOut* 
     if (pp->n_u) {
         const int      G       = writer_items(pp->group);
         const uint64_t chunk   = warp_chunk(G);
-        const uint64_t nchunks = (pp->tot_u + chunk - 1) / chunk;
+        const uint32_t lead    = stream_lead(outs);
+        const uint64_t nchunks = (pp->tot_u + lead + chunk - 1) / chunk;
         uint32_t*      cfirst  = dalloc_n<uint32_t>(nchunks + 1, st);
-        k_chunk_first<<<div_up(nchunks, 256), 256, 0, st>>>(L.u_off, pp->n_u, nchunks, uint32_t(chunk), cfirst);
+        k_chunk_first<<<div_up(nchunks, 256), 256, 0, st>>>(L.u_off, pp->n_u, nchunks, uint32_t(chunk), lead, cfirst);
         HJ_LAUNCH_CHECK();
         launch_uniform(G, T, L, pp->n_u, cfirst, pp->tot_u, outs, st);
         dfree(cfirst, st);
