@@ -138,7 +138,7 @@ struct RelInst {  // one relation of one instance
     uint32_t       inst;
     uint32_t       irows;  // R0s: rows per work item
     uint32_t       nrel;
-    uint32_t       fbase;  // R0s: first word of the instance's filter
+    uint32_t       fbase, flog;  // R0s: first word of the instance's filter; log2 of a partition's bits
 };
 
 // One work item of the probe, whole, so that a block waits for one load.
@@ -146,7 +146,7 @@ struct Item {
     const int32_t *k, *p;
     uint64_t       part_base;
     uint32_t       n, inst, pbits, nt;  // rows; instance; its partition bits and tables beside F
-    uint32_t       fbase;               // and the first word of its filter
+    uint32_t       fbase, flog;         // and its filter
 };
 
 struct InstInfo {
@@ -154,7 +154,8 @@ struct InstInfo {
     uint64_t ip_base;    // first instance partition (2^pbits of them)
     uint32_t nrel;
     uint32_t pbits;
-    uint32_t fbase;      // first word of its filter (2^(pbits + filter_log - 5) of them)
+    uint32_t fbase;      // first word of its filter (2^(pbits + flog - 5) of them)
+    uint32_t flog;       // log2 of a partition's bits there
 };
 
 // Per-instance results and flags, cleared together.
@@ -191,12 +192,9 @@ struct Piece {
 constexpr uint32_t kSteps = 2, kHeavy = 12;
 // A filter of an instance's listed keys, for those who look for rows of them: two
 // bits of a word a key, each partition with words of its own, at most as many as
-// fit a block's shared memory (2^17 bits).  Few rows of other keys pass it, and
-// what passes takes three dependent loads.
+// fit a block's shared memory (2^17 bits), and 8 to 16 bits a build row.  Few rows
+// of other keys pass it, and what passes takes three dependent loads.
 constexpr uint32_t kFilterPart = 13, kFilterAll = 17;
-__host__ __device__ __forceinline__ uint32_t filter_log(uint32_t pbits) {
-    return kFilterAll - pbits < kFilterPart ? kFilterAll - pbits : kFilterPart;
-}
 
 // A free slot.  A build row that is this very pair cannot be stored: its
 // instance is left to the plain path.
@@ -293,7 +291,7 @@ __global__ void k_item_rel(const RelInst* __restrict__ R, uint32_t nr, uint64_t 
         const RelInst& r  = R[ri];
         const uint64_t r0 = (t - r.item_base) * r.irows;
         imap[t - bitems]  = Item{r.keys + r0, r.pay + r0, r.part_base, uint32_t(min(r.rows - r0, uint64_t(r.irows))),
-                                r.inst, r.pbits, r.nrel - 2, r.fbase};
+                                r.inst, r.pbits, r.nrel - 2, r.fbase, r.flog};
     }
 }
 
@@ -742,7 +740,7 @@ __global__ void __launch_bounds__(kBuildT, 2)
         // as the lists take the place of what has been read.
         __syncthreads();
         const uint32_t o1 = nt ? g_to[nt - 1] + g_tn[nt - 1] : 0u;
-        const uint32_t flog = filter_log(pb);
+        const uint32_t flog   = s.flog;
         uint32_t*      filter = S + scap + (fcap + 1) / 2;
         for (uint32_t w = threadIdx.x; w < 1u << (flog - 5); w += kBuildT) filter[w] = 0;
         __syncthreads();
@@ -1203,7 +1201,7 @@ __global__ void __launch_bounds__(kBT, 3)
             qn = 0;
             acc.at(it.inst, out);
             pb   = it.pbits;
-            flog = filter_log(pb);
+            flog = it.flog;
             I    = EnumOf{tabs, kp, listed + it.part_base, it.p, pb, it.nt};
             __syncthreads();
             const uint32_t words = 1u << (pb + flog - 5);
@@ -1395,7 +1393,8 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
         s.nrel           = nrel;
         s.pbits          = p;
         s.fbase          = uint32_t(fwords);
-        fwords += 1ull << (p + filter_log(p) - 5);
+        s.flog           = std::min({kFilterPart, kFilterAll - p, std::max(5u, ceil_log2u(8 * std::max<uint64_t>(nb, 1)))});
+        fwords += 1ull << (p + s.flog - 5);
         stride           = std::max(stride, s.nrel - 2);
         for (uint32_t j = 1; j < s.nrel; ++j) {
             const BatchRelation br = rel_of(i, j);
@@ -1427,7 +1426,7 @@ void batch_wave(const std::vector<BatchInstance>& all, uint32_t i0, uint32_t i1,
         const uint64_t       steps = br.rows / (2 * uint64_t(g_prb) * kStepRows);
         const uint64_t       irows = std::min<uint64_t>(std::max<uint64_t>(steps, 16), 64) * kStepRows;
         hr.push_back({br.keys, br.payload, br.rows, items, hi[i].part_base, hi[i].pbits, i, uint32_t(irows), hi[i].nrel,
-                      hi[i].fbase});
+                      hi[i].fbase, hi[i].flog});
         items += (br.rows + irows - 1) / irows;
     }
     const uint32_t nr   = uint32_t(hr.size());

@@ -107,3 +107,20 @@ else:
     rows, s2, _ = E.batch_execute(inst, hj.BATCH_PLAIN)
     assert rows[0] == want[0] == 300 and sums[0] == s2[0]
 """)
+
+
+def test_batch_of_many_small_instances():
+    """What an instance takes beside its rows does not grow past them: 200,000 instances of
+    10 build rows, each with a key that repeats."""
+    run("""
+n = 200_000
+k = torch.arange(10, dtype=torch.int32, device="cuda")
+k[9] = 3
+one = [(k.data_ptr(), k.data_ptr(), 10)] * 3
+torch.cuda.synchronize()
+E.batch_execute([one])
+before = free()
+rows, sums, redo = E.batch_execute([one] * n)
+assert set(rows) == {8 + 2 * 2 * 2} and len(set(sums)) == 1 and redo == 0
+assert before - free() < n * 1600, before - free()
+""")
