@@ -116,8 +116,8 @@ __global__ void k_batch_generate(uint64_t seed, uint32_t inst, uint32_t rel, uin
 // the plain path.
 //
 // F is read in place of a partitioned R0: random 32-byte reads of tables up to
-// 64 MB run at 292e9/s on a GB300 (one L2 sector per SM and cycle; 84e9/s at
-// 256 MB, past the L2), and at 273e9 rows/s together with the stream of R0,
+// 64 MB (4M build rows) run at 292e9/s on a GB300 (one L2 sector per SM and cycle;
+// 84e9/s at 256 MB, past the L2), and at 273e9 rows/s together with the stream of R0,
 // where a partition of R0 beside the build relations (28 bytes a row in three
 // passes) took 17 ps a row.  64 instances of 1k .. 4M build rows (364M R0
 // rows): 5.5 ms with R0 partitioned, 3.5 ms so.  Tables built in place by
@@ -914,11 +914,13 @@ struct Sums {
 // 5. R0 rows against F.  kU rows a thread: keys and payloads of the next rows
 // are on their way while the buckets of these are looked at.  Bound by its
 // instructions and the L1's lines (about 155 a row of 32, 56% issue active, the
-// L1 77% busy: 142e9 rows/s on 1M-row tables), so the bucket reads allocate no
-// L1 lines, two rows a thread fit 64 registers without spills, and what only
-// some rows need is put off until a whole warp needs it: matches wait in the warp's queue until 32 of them are folded
-// together, and rows that have to go on to a next bucket (one in twenty at half
-// load, some in every warp) until 32 of them look together.  The instance's
+// L1 77% busy), not by where the table lies: 80M rows against a table of 1, 4, 16 or
+// 64 MB 331, 337, 342, 361 us without a match, 477, 484, 482, 512 with one for half
+// of the rows, 579, 586, 584, 595 with one each.  So the bucket reads allocate no
+// L1 lines, two rows a thread fit 64 registers without spills, and what only some
+// rows need is put off until a whole warp needs it: matches wait in the warp's queue
+// until 32 of them are folded together, and rows that have to go on to a next bucket
+// (one in twenty at half load, some in every warp) until 32 of them look together.  The instance's
 // pieces are kept in shared memory (reads of them through L1 would cost as
 // much as the buckets).  Each match of a key in F is a result row; listed keys are
 // not in it.
@@ -1080,9 +1082,9 @@ __global__ void __launch_bounds__(kBT, 4)
 // row's results are the combinations of one payload a list.  The warp shares out those
 // of its rows together: of a row with kMany of them by themselves, else by a
 // search of the running sums.
-// Bound by the scan of R0's keys where few are listed (360e9 rows/s, half of the
-// warps waiting for shared memory), so what a listed row needs is kept out of its
-// registers.  Results by the rows' own lanes instead: 64 chains of 16,000 rows, 16 a
+// Bound by the scan of R0's keys where few are listed (500e9 rows/s, 57% issue
+// active), so what a listed row needs is kept out of its registers (within them
+// 360e9).  Results by the rows' own lanes instead: 64 chains of 16,000 rows, 16 a
 // key, half of R0's rows with a partner 1,836 us, so 1,080.
 constexpr int      kEU     = 8;
 constexpr uint32_t kMany   = 64;

@@ -898,9 +898,11 @@ struct Exec {
         // matches, and their order in the tile, are as before).  A join without
         // and with it, us: 66,000 x 1,984 rows 98 / 70, 1M x 1,984 116 / 72, 10M x
         // 1,984 325 / 106, 10M x 8,192 338 / 267; Zipf probe keys 1M x 1,984 117 /
-        // 68; one key's 20M pairs 1M x 1,984 339 / 282.  It loses where one key
-        // takes a quarter of the build rows, which then stay: 300,000 x 30 154 /
-        // 168, 1M x 400 338 / 368.  The table over the probe side instead was as fast for distinct keys, but a
+        // 68; one key's 0.45M pairs 300,000 x 30 148 / 142, 8M pairs 1M x 1,984 250 /
+        // 183.  It loses where one key's rows stay and little else is saved: 1M x 400,
+        // a quarter of the rows and 20M pairs 325 / 331, a twentieth 166 / 171; where
+        // at most an eighth or a thirty-second may stay, 339 and 340, 170 and 177.
+        // The table over the probe side instead was as fast for distinct keys, but a
         // repeated one made its buckets heavy (Zipf, 1M x 31,250: 122 / 149).
         std::vector<int> ss{bk.src};  // the build side's sources that are read
         for (auto [side, s] : need)

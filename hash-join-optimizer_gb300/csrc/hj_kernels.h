@@ -133,8 +133,8 @@ struct RidOut {
 constexpr int kMaxRidOut = 16;
 
 struct ProbeParams {
-    int       light_max = 32;       // larger buckets are not scanned by one thread
-    int       group     = 8;        // threads per probe key in the write pass (1, 4, 8, 32)
+    int       light_max = 32;       // larger buckets of several keys (at most 31 tuples) are not scanned by one thread
+    int       group     = 8;        // output rows per thread of the match writer (1, 2, 4, 8, 16; 32 as 16)
     uint64_t* pinned    = nullptr;  // >= 8 words of pinned host memory for count readback
     uint64_t* counters  = nullptr;  // 8 zeroed device words; zero again after each probe (probe_free)
     std::function<void()> after_count;  // called once the count kernels are enqueued
@@ -160,9 +160,9 @@ uint64_t reduce_build(const KeyCol& b, const KeyCol& p, const ProbeParams& prm, 
 struct ProbePlan;  // opaque match list between the count and write passes
 
 // Count pass: returns the number of matches; keeps the hit list in *pp.  With
-// outputs (streams of pk.n slots each), tiles of rows with at most one match
-// each are written at once: probe_direct() rows, the first of the result; the
-// list holds the others.
+// outputs (streams of pk.n slots each), a match that is the only one of its probe
+// row is written at once (for one tile of rows, when all are such):
+// probe_direct() rows, the first of the result; the list holds the others.
 uint64_t probe_count(const Table& t, const KeyCol& pk, const ProbeParams& prm, const RidOut* outs, int nout,
                      ProbePlan** pp, cudaStream_t st);
 uint64_t probe_direct(const ProbePlan* pp);

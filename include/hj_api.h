@@ -152,8 +152,8 @@ void* hj_context_stream(hj_context* ctx);
  * build, 0..12), "probe_group" (output rows per thread of the match writer,
  * so a probe key's matches spread over count / probe_group threads: 1, 2, 4,
  * 8, 16 or 32; default 4), "light_max" (a bucket of several keys with at most
- * this many tuples is compared by the probing thread itself; larger ones by a
- * warp or block per hit), "timing" (1: record per-phase device times of
+ * this many tuples, and at most 31, is compared by the probing thread itself;
+ * larger ones by a warp or block per hit), "timing" (1: record per-phase device times of
  * each hj_execute, read with hj_result_phase_ms), "host_access" (1, default:
  * where the GPU can read and write pageable host memory, it moves input and
  * result pages itself; 0: host threads stage them through pinned memory),
@@ -220,8 +220,9 @@ int  hj_result_phase_ms(const hj_result* res, const char* phase, double* ms);
 /* Counters of the hj_execute that made `res`, summed over its joins (no
  * counterpart in the reference; they size the roofline of a run):
  * "dir_words" (directory words of the built tables, 2^b + 1 each),
- * "table_tuples" (tuples inserted, i.e. non-NULL build keys), "joins",
- * "launches" (kernels launched).  HJ_ERR_INVALID for another name. */
+ * "table_tuples" (tuples inserted, i.e. non-NULL build keys; of a build side
+ * that a short probe side cuts down, those it can meet), "joins", "launches"
+ * (kernels launched).  HJ_ERR_INVALID for another name. */
 int  hj_result_counter(const hj_result* res, const char* name, uint64_t* value);
 void hj_result_free(hj_result* res);
 
