@@ -1160,8 +1160,9 @@ int set_err(hj_context* c, const Error& e) {
 
 // A copy by the host comes after the work on the stream, as a copy on the stream
 // does: a program that has taken the stream may have put reads of its buffer
-// there.  (The engine's own calls wait for their work.  A query takes 2 us a
-// column: with one always, a point query of four columns 91 us instead of 84.)
+// there.  (The engine's own calls wait for their work.  A query takes 1.6 us, a
+// point query of four columns 91 us with them instead of 84; whether the program
+// has put anything there since the last one is known to the driver alone.)
 void wait_for_program(const hj_context* c) {
     if (!c->st_taken.load(std::memory_order_acquire)) return;
     const cudaError_t e = cudaStreamQuery(c->st);

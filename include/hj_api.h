@@ -194,7 +194,8 @@ int hj_execute(hj_context* ctx, const hj_plan_desc* plan, hj_result** out);
 int hj_result_shape(const hj_result* res, uint64_t* num_rows, uint32_t* num_columns);
 int hj_result_column(const hj_result* res, uint32_t col, int32_t* type, uint64_t* num_pages);
 /* Copies the pages of column `col` to host memory: page i goes to dst_pages[i]
- * (8192 bytes each; no alignment needed). */
+ * (8192 bytes each; no alignment needed).  Ordered after the work on the context
+ * stream, the program's own included; complete on return. */
 int hj_result_copy_pages(hj_context* ctx, const hj_result* res, uint32_t col,
                          void* const* dst_pages);
 /* Same, into one contiguous host buffer of num_pages * 8192 bytes. */
